@@ -33,13 +33,259 @@ __global__ void grid_vis_kernel(const float2* __restrict__ vis, int n_fv, long l
   out[idx] = make_float2(re, im);
 }
 
-// out[d, t, cell] = sum_{src in cell} vis_joined[t + shift[s(src), d], src]
-// where vis_joined = concat(prev[0:n_prev], cur) along time.
-__global__ void dedisp_vis_kernel(const float2* __restrict__ prev, const float2* __restrict__ cur,
-                                  int n_prev, long long nsrc, int ceff,
-                                  const int* __restrict__ off, const int* __restrict__ src,
-                                  const int* __restrict__ shifts, int n_dm, int n_filled,
-                                  int t_dedisp, float2* __restrict__ out) {
+// Stage 1 on visibilities: out[d, t, cell] = sum_{src in cell}
+// vis_joined[t + shift[s(src), d], src], vis_joined = concat(prev[0:n_prev],
+// cur) along time.
+//
+// What bounds it: every visibility is needed once per coarse DM, at a
+// different time for each, so the adds read n_dm x the input.  Read straight
+// from global memory (one thread per output) those were 8-byte gathers a row
+// of sources apart, a sector each: 23.9 ms for 32 DMs of a native page (512
+// tiles, 4656 baselines x 24 subbands, 0.46 GB).  So a CTA takes 4 adjacent
+// cells, 64 output times and up to 32 DMs, and stages each source's time
+// window (the 64 times plus the spread of its subband's shifts over the DMs)
+// in shared memory by 8-byte asynchronous copies, one batch of sources ahead:
+// lanes run over the sources of a row, which are consecutive in memory where
+// a baseline's subbands share a cell.  A warp then owns DPW DMs and its lanes
+// the times, so that the adds read consecutive 8-byte words (no bank
+// conflicts); the shared-memory pipe is what is left to bound it: 1.32 ms for
+// the same page.  Each cell's sources are added in CSR order, as before.
+constexpr int DV_TT = 64;        // output times per CTA
+constexpr int DV_CELLS = 4;      // cells per CTA (32 bytes of an output row)
+constexpr int DV_THREADS = 256;
+constexpr int DV_SLOTS = 6144;   // float2 slots of one window buffer (offsets fit 16 bits)
+constexpr int DV_MAXB = 96;      // sources per batch
+constexpr int DV_MAX_C = 512;    // subbands whose shift tables fit
+
+// dynamic shared memory: two window buffers, two offset tables [source][DM],
+// the subbands' shifts relative to their smallest [subband][DM] and their
+// smallest and largest shift
+__host__ __device__ inline size_t dv_smem_bytes(int ceff, int dg) {
+  return (size_t)2 * DV_SLOTS * 8 + (size_t)2 * DV_MAXB * dg * 2 + (size_t)ceff * dg * 2 +
+         (size_t)ceff * 8 + 16;
+}
+
+DSB_DEV void cp_async8(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src)
+               : "memory");
+}
+DSB_DEV void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+DSB_DEV void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+template <int DPW>
+__global__ void __launch_bounds__(DV_THREADS, 2)
+    dedisp_vis_kernel(const float2* __restrict__ prev, const float2* __restrict__ cur, int n_prev,
+                      long long nsrc, int ceff, const int* __restrict__ off,
+                      const int* __restrict__ src, const int* __restrict__ shifts, int n_dm,
+                      int n_filled, int t_dedisp, int n_tiles, float2* __restrict__ out) {
+  constexpr int DG = DPW * (DV_THREADS / 32);  // DMs per CTA
+  constexpr int TPL = DV_TT / 32;              // times per lane
+  extern __shared__ __align__(16) uint8_t dv_smem[];
+  __shared__ int s_w;                          // window pitch of a source
+  float2* win = reinterpret_cast<float2*>(dv_smem);                    // [2][DV_SLOTS]
+  uint16_t* boff = reinterpret_cast<uint16_t*>(win + 2 * DV_SLOTS);    // [2][DV_MAXB][DG]
+  uint16_t* rel = boff + 2 * DV_MAXB * DG;                             // [ceff][DG]
+  int* s_lo = reinterpret_cast<int*>(rel + (size_t)ceff * DG);         // [ceff]
+  int* s_hi = s_lo + ceff;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int t0 = (int)(blockIdx.x % n_tiles) * DV_TT;
+  const int cell0 = (int)(blockIdx.x / n_tiles) * DV_CELLS;
+  const int nt = min(DV_TT, t_dedisp - t0);
+  const int nc = min(DV_CELLS, n_filled - cell0);
+  const int d0 = blockIdx.y * DG;
+  const int nd = min(DG, n_dm - d0);
+
+  // each subband's shift range over this CTA's DMs, and the window pitch:
+  // the longest window, made odd so that lanes on consecutive sources write
+  // different banks
+  if (tid == 0) s_w = 0;
+  __syncthreads();
+  int w_max = 0;
+  for (int sb = tid; sb < ceff; sb += DV_THREADS) {
+    const int* sh = shifts + (long long)sb * n_dm + d0;
+    int lo = sh[0], hi = sh[0];
+    for (int d = 1; d < nd; ++d) {
+      lo = min(lo, sh[d]);
+      hi = max(hi, sh[d]);
+    }
+    s_lo[sb] = lo;
+    s_hi[sb] = hi;
+    // a spread too wide for the buffers (or for 16 bits) sends the CTA to
+    // the direct path; clamped so that the sum stays an int
+    w_max = max(w_max, (int)min((long long)hi - lo, (long long)DV_SLOTS));
+  }
+  atomicMax(&s_w, w_max);
+  __syncthreads();
+  const int W = (s_w + DV_TT) | 1;
+  const int NB = min(DV_SLOTS / W, DV_MAXB);   // sources per batch; 0: the direct path
+  const int c_end = cell0 + nc;
+  float2 acc[DPW][TPL], res[DV_CELLS][DPW][TPL];
+#pragma unroll
+  for (int k = 0; k < DPW; ++k)
+#pragma unroll
+    for (int h = 0; h < TPL; ++h) acc[k][h] = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int c = 0; c < DV_CELLS; ++c)
+#pragma unroll
+    for (int k = 0; k < DPW; ++k)
+#pragma unroll
+      for (int h = 0; h < TPL; ++h) res[c][k][h] = make_float2(0.f, 0.f);
+  auto finish = [&](int c) {
+#pragma unroll
+    for (int k = 0; k < DPW; ++k)
+#pragma unroll
+      for (int h = 0; h < TPL; ++h) {
+        res[c - cell0][k][h] = acc[k][h];
+        acc[k][h] = make_float2(0.f, 0.f);
+      }
+  };
+  auto row_of = [&](long long r) {
+    return r < n_prev ? prev + r * nsrc : cur + (r - n_prev) * nsrc;
+  };
+
+  if (NB > 0) {
+    for (int i = tid; i < ceff * DG; i += DV_THREADS) {
+      const int sb = i / DG, d = i % DG;
+      rel[i] = (uint16_t)(d < nd ? shifts[(long long)sb * n_dm + d0 + d] - s_lo[sb] : 0);
+    }
+    __syncthreads();
+    // batch (c, j): sources j .. j + NB - 1 of cell c (fewer at its end)
+    auto load = [&](int buf, int c, int j) {
+      const int nb = min(NB, off[c + 1] - j);
+      float2* wb = win + buf * DV_SLOTS;
+      int lo = 0x7fffffff, hi = -0x7fffffff;
+      for (int i = lane; i < nb; i += 32) {
+        const int sb = src[j + i] % ceff;
+        lo = min(lo, s_lo[sb]);
+        hi = max(hi, s_hi[sb]);
+      }
+      lo = __reduce_min_sync(0xffffffffu, lo);
+      hi = __reduce_max_sync(0xffffffffu, hi);
+      for (int i = tid & 15; i < nb; i += 16) {
+        const int sj = src[j + i], sb = sj % ceff;
+        const int l = s_lo[sb], n = s_hi[sb] - l + nt;   // rows t0 + l .. t0 + l + n - 1
+        for (int r = lo + (tid >> 4); r < hi + nt; r += DV_THREADS / 16) {
+          const int k = r - l;
+          if (k >= 0 && k < n) cp_async8(wb + i * W + k, row_of((long long)t0 + r) + sj);
+        }
+      }
+      uint16_t* bo = boff + buf * DV_MAXB * DG;
+      for (int x = tid; x < nb * DG; x += DV_THREADS) {
+        const int i = x / DG;
+        bo[x] = (uint16_t)(i * W + rel[(src[j + i] % ceff) * DG + x % DG]);
+      }
+      cp_async_commit();
+    };
+    auto advance = [&](int& c, int& j) {   // to the next batch; c == c_end at the end
+      j += NB;
+      while (c < c_end && j >= off[c + 1]) {
+        ++c;
+        if (c < c_end) j = off[c];
+      }
+    };
+    int c = cell0, j = off[cell0] - NB;
+    advance(c, j);
+    int buf = 0;
+    if (c < c_end) load(0, c, j);
+    while (c < c_end) {
+      int cn = c, jn = j;
+      advance(cn, jn);
+      if (cn < c_end) {
+        load(buf ^ 1, cn, jn);
+        cp_async_wait<1>();
+      } else {
+        cp_async_wait<0>();
+      }
+      __syncthreads();
+      if (warp * DPW < nd) {
+        const int nb = min(NB, off[c + 1] - j);
+        const float2* wb = win + buf * DV_SLOTS + lane;
+        const uint16_t* bo = boff + buf * DV_MAXB * DG + warp * DPW;
+#pragma unroll 2
+        for (int i = 0; i < nb; ++i) {
+          uint16_t o[DPW];
+          if constexpr (DPW == 4) {
+            const uint2 w = *reinterpret_cast<const uint2*>(bo + i * DG);
+            o[0] = (uint16_t)w.x; o[1] = (uint16_t)(w.x >> 16);
+            o[2] = (uint16_t)w.y; o[3] = (uint16_t)(w.y >> 16);
+          } else {
+#pragma unroll
+            for (int k = 0; k < DPW; ++k) o[k] = bo[i * DG + k];
+          }
+#pragma unroll
+          for (int k = 0; k < DPW; ++k)
+#pragma unroll
+            for (int h = 0; h < TPL; ++h) acc[k][h] = f2_add(acc[k][h], wb[o[k] + 32 * h]);
+        }
+      }
+      if (cn != c) finish(c);
+      c = cn;
+      j = jn;
+      buf ^= 1;
+      __syncthreads();   // the buffer just read is the next batch's target
+    }
+  } else {
+    for (int c = cell0; c < c_end; ++c) {
+      for (int j = off[c]; j < off[c + 1]; ++j) {
+        const int sj = src[j];
+        const int* sh = shifts + (long long)(sj % ceff) * n_dm + d0;
+#pragma unroll
+        for (int k = 0; k < DPW; ++k)
+#pragma unroll
+          for (int h = 0; h < TPL; ++h)
+            if (warp * DPW + k < nd && lane + 32 * h < nt)
+              acc[k][h] = f2_add(acc[k][h], row_of((long long)t0 + lane + 32 * h +
+                                                   sh[warp * DPW + k])[sj]);
+      }
+      finish(c);
+    }
+  }
+  // four lanes exchange (cell, time) so that they write the 4 cells of one
+  // time together (one sector instead of four)
+  const int q = lane & 3;
+#pragma unroll
+  for (int k = 0; k < DPW; ++k)
+#pragma unroll
+    for (int h = 0; h < TPL; ++h) {
+      float2 a[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) a[c] = res[c][k][h];
+      // lane q's a[c] (cell c, time 4 (lane / 4) + q) -> lane c's a[q]
+#pragma unroll
+      for (int m = 1; m <= 2; m *= 2)
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          if (!(c & m)) {
+            const bool up = q & m;
+            const float2 give = up ? a[c] : a[c | m];
+            float2 got;
+            got.x = __shfl_xor_sync(0xffffffffu, give.x, m);
+            got.y = __shfl_xor_sync(0xffffffffu, give.y, m);
+            if (up) a[c] = got;
+            else a[c | m] = got;
+          }
+      const int d = warp * DPW + k;
+      if (d < nd && q < nc) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const int t = 32 * h + (lane & ~3) + c;
+          if (t < nt)
+            out[((long long)(d0 + d) * t_dedisp + t0 + t) * n_filled + cell0 + q] = a[c];
+        }
+      }
+    }
+}
+
+// More subbands than the shift tables hold: one thread per output.
+__global__ void dedisp_vis_wide_kernel(const float2* __restrict__ prev,
+                                       const float2* __restrict__ cur, int n_prev,
+                                       long long nsrc, int ceff, const int* __restrict__ off,
+                                       const int* __restrict__ src,
+                                       const int* __restrict__ shifts, int n_dm, int n_filled,
+                                       int t_dedisp, float2* __restrict__ out) {
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long per_d = (long long)t_dedisp * n_filled;
   if (idx >= per_d * n_dm) return;
@@ -55,6 +301,25 @@ __global__ void dedisp_vis_kernel(const float2* __restrict__ prev, const float2*
     im += x.y;
   }
   out[idx] = make_float2(re, im);
+}
+
+template <int DPW>
+int launch_dedisp_vis(const float2* prev, const float2* cur, int n_prev, long long nsrc, int ceff,
+                      const int* off, const int* src, const int* shifts, int n_dm, int n_filled,
+                      int t_dedisp, float2* out, cudaStream_t stream) {
+  constexpr int DG = DPW * (DV_THREADS / 32);
+  const size_t smem = dv_smem_bytes(ceff, DG);
+  if (cudaFuncSetAttribute(dedisp_vis_kernel<DPW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)smem) != cudaSuccess)
+    return DSB_E_CUDA;
+  const int n_tiles = (t_dedisp + DV_TT - 1) / DV_TT;
+  const long long blocks = (long long)n_tiles * ((n_filled + DV_CELLS - 1) / DV_CELLS);
+  // times fastest: CTAs that run together share a cell group's input rows and
+  // complete the output rows' sectors in L2
+  const dim3 grid((unsigned)blocks, (n_dm + DG - 1) / DG);
+  dedisp_vis_kernel<DPW><<<grid, DV_THREADS, smem, stream>>>(
+      prev, cur, n_prev, nsrc, ceff, off, src, shifts, n_dm, n_filled, t_dedisp, n_tiles, out);
+  return cudaGetLastError() == cudaSuccess ? DSB_OK : DSB_E_CUDA;
 }
 
 // Static-sky mean (per cell): mean of the past `count` block means held in
@@ -366,9 +631,24 @@ int dsb_dedisp_vis(const void* prev, const void* cur, int n_prev, long long nsrc
   if (n_prev > 0 && !prev) return DSB_E_ARG;
   const long long n = (long long)n_dm * t_dedisp * n_filled;
   if (n <= 0) return DSB_OK;
-  dedisp_vis_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(
-      (const float2*)prev, (const float2*)cur, n_prev, nsrc, ceff, cell_off, cell_src, shifts,
-      n_dm, n_filled, t_dedisp, (float2*)out);
+  const auto* p = (const float2*)prev;
+  const auto* v = (const float2*)cur;
+  auto* o = (float2*)out;
+  // the windowed kernel while the subbands' shift tables fit beside the
+  // window buffers; DMs per warp as few as cover the DMs of the call, so that
+  // no warp of a short list idles
+  if (ceff <= DV_MAX_C && (n_dm + 31) / 32 <= 65535) {
+    if (n_dm <= 8)
+      return launch_dedisp_vis<1>(p, v, n_prev, nsrc, ceff, cell_off, cell_src, shifts, n_dm,
+                                  n_filled, t_dedisp, o, stream);
+    if (n_dm <= 16)
+      return launch_dedisp_vis<2>(p, v, n_prev, nsrc, ceff, cell_off, cell_src, shifts, n_dm,
+                                  n_filled, t_dedisp, o, stream);
+    return launch_dedisp_vis<4>(p, v, n_prev, nsrc, ceff, cell_off, cell_src, shifts, n_dm,
+                                n_filled, t_dedisp, o, stream);
+  }
+  dedisp_vis_wide_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(
+      p, v, n_prev, nsrc, ceff, cell_off, cell_src, shifts, n_dm, n_filled, t_dedisp, o);
   return launch_status();
 }
 
