@@ -577,15 +577,16 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 }
 
 // ===========================================================================
-// tensor-core correlator on split (GEMM-layout) voltages: tcgen05 kind::f16
-// (int8 codes and float16 voltages, exact conversion to f16) or kind::tf32
-// (float32 voltages, rounded to tf32 as a float32 tensor-core product does),
-// float32 accumulators in TMEM.
+// tensor-core correlators on split (GEMM-layout) voltages, float32
+// accumulators in TMEM: tcgen05 kind::f16 for int8 codes (exact conversion)
+// and float16 voltages (corr_split_mn_kernel), kind::tf32 for float32
+// voltages, rounded to tf32 as a float32 tensor-core product does
+// (corr_split_tc_kernel).
 // ===========================================================================
 struct SplitTcArgs {
-  const void* re;
-  const void* im;
-  int dtype;                 // DSB_DT_INT8 / DSB_DT_F16 / DSB_DT_F32
+  const void* re;            // int8, float16: rounded down to 4 bytes, the
+  const void* im;            //   first element off_re / off_im elements on
+  int off_re, off_im;
   int nchan, npkt, nant, nant_p, ppfv, fuse, csf, ceff;
   int n_fv, n_units, kprime, n_chunks, rows, nstage, stage_bytes;
   float2* out;
@@ -610,31 +611,23 @@ DSB_DEV void split_unit(const SplitTcArgs& A, int u, int& fv, int& ch0, int& pol
   }
 }
 
-template <int ELEM>
-DSB_DEV uint32_t split_load_bits(const SplitTcArgs& A, const void* p, size_t o) {
-  if constexpr (ELEM == 2) {
-    if (A.dtype == DSB_DT_INT8)
-      return (uint32_t)__half_as_ushort(__int2half_rn((int)static_cast<const int8_t*>(p)[o]));
-    return (uint32_t)__half_as_ushort(static_cast<const __half*>(p)[o]);
-  } else {
-    // round the float32 to tf32 (10 mantissa bits), nearest with ties away
-    // from zero: add half of the dropped range to the magnitude bits (a
-    // carry moves into the exponent correctly), clear the dropped bits;
-    // infinities and NaNs pass unchanged
-    const uint32_t u = __float_as_uint(static_cast<const float*>(p)[o]);
-    if ((u & 0x7F800000u) == 0x7F800000u) return u;
-    return (u + 0x1000u) & 0xFFFFE000u;
-  }
+// Element o rounded to tf32 (10 mantissa bits), nearest with ties away from
+// zero: add half of the dropped range to the magnitude bits (a carry moves
+// into the exponent correctly), clear the dropped bits; infinities and NaNs
+// pass unchanged.
+DSB_DEV uint32_t split_load_bits(const void* p, size_t o) {
+  const uint32_t u = __float_as_uint(static_cast<const float*>(p)[o]);
+  if ((u & 0x7F800000u) == 0x7F800000u) return u;
+  return (u + 0x1000u) & 0xFFFFE000u;
 }
 
 // One K chunk (KC complex samples) of unit u into an operand stage:
 // rows [0, nant_p) = [R | I], rows [nant_p, 2 nant_p) = [I | -R] (K-major,
 // SW128, one 128-byte row per operand row); samples past the unit's K and
 // antennas past nant are zero.
-template <int ELEM>
 DSB_DEV void split_fill(const SplitTcArgs& A, uint8_t* st, int u, int q) {
-  constexpr int KC = 64 / ELEM;    // complex samples per chunk
-  constexpr int G = 16 / ELEM;     // samples per 16-byte group
+  constexpr int KC = 16;           // complex samples per chunk
+  constexpr int G = 4;             // samples per 16-byte group
   constexpr int NG = KC / G;       // groups per half row (4)
   int fv, ch0, pol0, npol_u;
   split_unit(A, u, fv, ch0, pol0, npol_u);
@@ -656,24 +649,14 @@ DSB_DEV void split_fill(const SplitTcArgs& A, uint8_t* st, int u, int q) {
         const int ch = ch0 + k / npol_u;
         const size_t o = (((size_t)ch * 2 + t) * 2 + pol) * plane +
                          (size_t)(fv * A.ppfv + p) * A.nant + a;
-        r[i] = split_load_bits<ELEM>(A, A.re, o);
-        m[i] = split_load_bits<ELEM>(A, A.im, o);
+        r[i] = split_load_bits(A.re, o);
+        m[i] = split_load_bits(A.im, o);
       }
     }
-    uint4 R, I, N;
-    if constexpr (ELEM == 2) {
-      R = make_uint4(r[0] | (r[1] << 16), r[2] | (r[3] << 16), r[4] | (r[5] << 16),
-                     r[6] | (r[7] << 16));
-      I = make_uint4(m[0] | (m[1] << 16), m[2] | (m[3] << 16), m[4] | (m[5] << 16),
-                     m[6] | (m[7] << 16));
-      N = make_uint4(R.x ^ 0x80008000u, R.y ^ 0x80008000u, R.z ^ 0x80008000u,
-                     R.w ^ 0x80008000u);
-    } else {
-      R = make_uint4(r[0], r[1], r[2], r[3]);
-      I = make_uint4(m[0], m[1], m[2], m[3]);
-      N = make_uint4(r[0] ^ 0x80000000u, r[1] ^ 0x80000000u, r[2] ^ 0x80000000u,
-                     r[3] ^ 0x80000000u);
-    }
+    const uint4 R = make_uint4(r[0], r[1], r[2], r[3]);
+    const uint4 I = make_uint4(m[0], m[1], m[2], m[3]);
+    const uint4 N = make_uint4(r[0] ^ 0x80000000u, r[1] ^ 0x80000000u, r[2] ^ 0x80000000u,
+                               r[3] ^ 0x80000000u);
     const uint32_t kr = (uint32_t)j * 16u, ki = 64u + (uint32_t)j * 16u;
     const uint32_t ra = (uint32_t)a, rb = (uint32_t)(A.nant_p + a);
     *reinterpret_cast<uint4*>(st + sw128_offset(ra, kr)) = R;
@@ -716,7 +699,6 @@ DSB_DEV void split_epilogue(const SplitTcArgs& A, uint32_t tmem_base, int buf, i
   }
 }
 
-template <int ELEM>
 __global__ void __launch_bounds__(TC_THREADS, 1) corr_split_tc_kernel(const SplitTcArgs A) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* stages = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -745,8 +727,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) corr_split_tc_kernel(const Spli
   const int u_begin = (int)blockIdx.x * per_cta;
   const int my_units = max(0, min(per_cta, A.n_units - u_begin));
   const int n_items = my_units * A.n_chunks;
-  // c_format F32; a/b format F16 (0) or TF32 (2); K-major; N = 2 nant_p; M = 128
-  constexpr uint32_t fmt = ELEM == 2 ? 0u : 2u;
+  // c_format F32; a/b format TF32 (2); K-major; N = 2 nant_p; M = 128
+  constexpr uint32_t fmt = 2u;
   const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) |
                          (((uint32_t)(2 * A.nant_p) >> 3) << 17) | ((128u >> 4) << 24);
   bool ok = true;
@@ -757,7 +739,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) corr_split_tc_kernel(const Spli
     if (it >= A.nstage) w_ok = mbar_wait(&bar_mma[slot], (uint32_t)((it / A.nstage - 1) & 1));
     if (!__syncthreads_and(w_ok)) { ok = false; break; }
     uint8_t* st = stages + (size_t)slot * A.stage_bytes;
-    split_fill<ELEM>(A, st, u_begin + lu, q);
+    split_fill(A, st, u_begin + lu, q);
     fence_proxy_async_smem();
     __syncthreads();
     if (tid == 0) {
@@ -767,8 +749,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) corr_split_tc_kernel(const Spli
 #pragma unroll
       for (int m = 0; m < 4; ++m) {   // 4 MMAs of 32 bytes of K each
         const uint64_t desc = sdesc_k_sw128(sbase + (uint32_t)m * 32u);
-        if constexpr (ELEM == 2) umma_f16_ss(d, desc, desc, idesc, (q > 0 || m > 0) ? 1u : 0u);
-        else umma_tf32_ss(d, desc, desc, idesc, (q > 0 || m > 0) ? 1u : 0u);
+        umma_tf32_ss(d, desc, desc, idesc, (q > 0 || m > 0) ? 1u : 0u);
       }
       umma_commit(&bar_mma[slot]);
       if (q == A.n_chunks - 1) umma_commit(&bar_acc[lu & 1]);
@@ -798,6 +779,283 @@ __global__ void __launch_bounds__(TC_THREADS, 1) corr_split_tc_kernel(const Spli
     umma_commit(bar_drain);
     mbar_wait(bar_drain, 0u);
   }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, TC_TMEM_COLS);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// The same correlator for int8 and float16 voltages, operands antenna-major.
+//
+// What bounds it: the voltages are read once (1.2 GB for a native float16
+// page), the products (four real 128 x nant x K ones per unit) need half of
+// that time on the tensor cores.  The K-major form above transposes every
+// element through 2-byte loads: 7.55 ms for that page (2048 packets, 96
+// antennas, 384 channels, 16 channels summed).  Here the operands stay as
+// they lie in memory, rows of antennas: tcgen05 reads A and B "MN-major" (128-byte
+// swizzle: atoms of 64 antennas x 8 samples, LBO between the two antenna
+// atoms, SBO between sample groups of 8), so that staging is a copy of 16-byte
+// chunks.  Re and Im get their own accumulators and four products per 16
+// samples, R_b R_a + I_b I_a and R_b I_a - I_b R_a, the sign by the
+// descriptor's negate-A bit, which drops the second [I | -R] operand copy.
+// Roles: warps 0-3 write the finished unit, warps 4-11 stage samples (rows of
+// a multiple of 8 float16 antennas by 16-byte asynchronous copies
+// MN_LAG stages ahead; other rows through registers, words funnel-shifted
+// to the row's offset), one thread of warp 12 issues the products: 0.57 ms for the same
+// page, exact sums unchanged.
+// ---------------------------------------------------------------------------
+constexpr int MN_EPI = 128, MN_LOAD = 256, MN_THREADS = MN_EPI + MN_LOAD + 32;
+constexpr int MN_KC = 64;                        // samples per stage
+constexpr int MN_PART = 2 * MN_KC * 128;         // bytes of one part (two antenna atoms)
+constexpr int MN_STAGE = 2 * MN_PART;            // real and imaginary parts
+constexpr int MN_NST = 6;
+constexpr int MN_LAG = 4;                        // copy stages in flight per loader thread
+constexpr int MN_SMEM = MN_NST * MN_STAGE + 1024 + (2 * MN_NST + 5) * 8 + 16;
+static_assert(MN_LAG < MN_NST && MN_SMEM <= 227 * 1024, "stages of one CTA per SM");
+
+// Shared-memory descriptor of an MN-major operand in the 128-byte swizzle:
+// atoms of 64 elements x 8 rows of K (1024 bytes), LBO = distance of the next
+// 64 elements, SBO = distance of the next 8 rows of K.
+DSB_DEV uint64_t sdesc_mn_sw128(uint32_t smem_addr, uint32_t lbo, uint32_t sbo) {
+  uint64_t d = 0;
+  d |= (uint64_t)((smem_addr >> 4) & 0x3FFFu);
+  d |= (uint64_t)((lbo >> 4) & 0x3FFFu) << 16;
+  d |= (uint64_t)((sbo >> 4) & 0x3FFFu) << 32;
+  d |= (uint64_t)1u << 46;
+  d |= (uint64_t)2u << 61;
+  return d;
+}
+
+DSB_DEV void cp_async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+
+// Four int8 codes (one word) as four float16 values: 0x6400 | (x + 128) is
+// the half 1024 + x + 128, exactly.
+DSB_DEV uint2 s8x4_to_h4(uint32_t w) {
+  const uint32_t b = w ^ 0x80808080u;
+  const __half2 off = __halves2half2(__ushort_as_half((unsigned short)0x6480),
+                                     __ushort_as_half((unsigned short)0x6480));  // 1152
+  uint32_t lo = __byte_perm(b, 0x64646464u, 0x4140);
+  uint32_t hi = __byte_perm(b, 0x64646464u, 0x4342);
+  const __half2 l = __hsub2(*reinterpret_cast<__half2*>(&lo), off);
+  const __half2 h = __hsub2(*reinterpret_cast<__half2*>(&hi), off);
+  return make_uint2(*reinterpret_cast<const uint32_t*>(&l), *reinterpret_cast<const uint32_t*>(&h));
+}
+
+// Eight elements (ESZ bytes each) from element o on, as 16 bytes of float16:
+// the aligned words that hold them, shifted to o.  Words past n_words, the
+// tensor's last, read as zero.
+template <int ESZ>
+DSB_DEV void mn_words(const void* p, size_t o, size_t n_words, uint32_t (&w)[2 * ESZ + 1]) {
+  const uint32_t* q = static_cast<const uint32_t*>(p);
+  const size_t w0 = o * ESZ / 4;
+#pragma unroll
+  for (int i = 0; i < 2 * ESZ + 1; ++i) w[i] = w0 + i < n_words ? __ldg(q + w0 + i) : 0u;
+}
+template <int ESZ>
+DSB_DEV uint4 mn_shift(size_t o, const uint32_t (&w)[2 * ESZ + 1]) {
+  const unsigned sh = (unsigned)(o * ESZ % 4) * 8u;
+  uint32_t v[2 * ESZ];
+#pragma unroll
+  for (int i = 0; i < 2 * ESZ; ++i) v[i] = __funnelshift_r(w[i], w[i + 1], sh);
+  if constexpr (ESZ == 2) return make_uint4(v[0], v[1], v[2], v[3]);
+  const uint2 a = s8x4_to_h4(v[0]), b = s8x4_to_h4(v[1]);
+  return make_uint4(a.x, a.y, b.x, b.y);
+}
+
+// ESZ: bytes of a voltage part (1 int8, 2 float16); COPY: float16 rows in
+// whole 16-byte chunks, staged by asynchronous copies.
+template <int ESZ, bool COPY>
+__global__ void __launch_bounds__(MN_THREADS, 1) corr_split_mn_kernel(const SplitTcArgs A) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* stages = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint64_t* bar_full = reinterpret_cast<uint64_t*>(stages + (size_t)MN_NST * MN_STAGE);
+  uint64_t* bar_free = bar_full + MN_NST;
+  uint64_t* bar_acc = bar_free + MN_NST;     // [2] accumulator finished
+  uint64_t* bar_out = bar_acc + 2;           // [2] accumulator written out
+  uint64_t* bar_drain = bar_out + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_drain + 1);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (warp == 0) {
+    tmem_alloc(tmem_slot, TC_TMEM_COLS);
+    tmem_relinquish();
+  }
+  if (tid == 0) {
+    for (int i = 0; i < MN_NST; ++i) {
+      mbar_init(&bar_full[i], MN_LOAD);
+      mbar_init(&bar_free[i], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&bar_acc[i], 1);
+      mbar_init(&bar_out[i], MN_EPI);
+    }
+    mbar_init(bar_drain, 1);
+    fence_mbar_init();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  const int per_cta = (A.n_units + (int)gridDim.x - 1) / (int)gridDim.x;
+  const int u_begin = (int)blockIdx.x * per_cta;
+  const int my_units = max(0, min(per_cta, A.n_units - u_begin));
+  const int n_items = my_units * A.n_chunks;
+  bool ok = true;
+
+  if (warp < MN_EPI / 32) {
+    // ---- write finished units: accumulator lane b, columns a (Re), 128 + a
+    //      (Im); the upper triangle b <= a goes to bls(a, b) ----
+    const int nant = A.nant, nbase = nant * (nant + 1) / 2;
+    const int b = warp * 32 + lane;
+    for (int lu = 0; ok && lu < my_units; ++lu) {
+      const int buf = lu & 1;
+      ok = __all_sync(0xffffffffu, mbar_wait(&bar_acc[buf], (uint32_t)((lu >> 1) & 1)));
+      if (!ok) break;
+      tc_fence_after();
+      int fv, ch0, pol0, npol_u;
+      split_unit(A, u_begin + lu, fv, ch0, pol0, npol_u);
+      const size_t step = A.fuse ? (size_t)A.ceff : (size_t)A.nchan * 2;
+      float2* o = A.out + (A.fuse ? (size_t)fv * nbase * A.ceff + ch0 / A.csf
+                                  : ((size_t)fv * nbase * A.nchan + ch0) * 2 + pol0);
+      const uint32_t lane_base = tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)(buf * 256);
+      for (int c0 = warp * 32; c0 < nant; c0 += 16) {   // columns a >= this warp's rows
+        __syncwarp();
+        uint32_t vr[16], vi[16];
+        tmem_ld16(lane_base + (uint32_t)c0, vr);
+        tmem_ld16(lane_base + 128u + (uint32_t)c0, vi);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          const int a = c0 + j;
+          if (a < b || a >= nant) continue;
+          o[(size_t)upper_bls(a, b) * step] =
+              make_float2(__uint_as_float(vr[j]), __uint_as_float(vi[j]));
+        }
+      }
+      tc_fence_before();
+      mbar_arrive(&bar_out[buf]);
+    }
+  } else if (warp < (MN_EPI + MN_LOAD) / 32) {
+    // ---- stage samples: thread (j, r) copies antennas 8j .. 8j + 7 of rows
+    //      r, r + 16, ... of the stage ----
+    const int lt = tid - MN_EPI;
+    const int j = lt & 15, r0 = lt >> 4;
+    const bool mine = 8 * j < A.nant;
+    const size_t plane = (size_t)A.npkt * A.nant;
+    // 4-byte words that hold the tensors (the last one may hold more)
+    const size_t n_el = plane * A.nchan * 4;
+    const size_t nw_re = ((n_el + A.off_re) * ESZ + 3) / 4, nw_im = ((n_el + A.off_im) * ESZ + 3) / 4;
+    const uint32_t jo = (uint32_t)(j >> 3) * (MN_KC * 128);
+    const int lag = COPY ? MN_LAG : 0;
+    for (int it = 0; it < n_items + lag; ++it) {
+      if (it < n_items) {
+        const int slot = it % MN_NST;
+        if (it >= MN_NST)
+          ok = __all_sync(0xffffffffu,
+                          mbar_wait(&bar_free[slot], (uint32_t)((it / MN_NST - 1) & 1)));
+        if (!ok) break;
+        const int q = it % A.n_chunks;
+        int fv, ch0, pol0, npol_u;
+        split_unit(A, u_begin + it / A.n_chunks, fv, ch0, pol0, npol_u);
+        // row k of the unit: plane k / ppfv (Stokes-I: consecutive (ch, t,
+        // pol); 2-pol: the unit's pol of t = 0, 1), packet k % ppfv
+        const int pl_step = A.fuse ? 1 : 2;
+        const size_t base = ((size_t)ch0 * 4 + pol0) * plane + (size_t)fv * A.ppfv * A.nant + 8 * j;
+        uint8_t* st = stages + (size_t)slot * MN_STAGE;
+        const int rows = (min(MN_KC, A.kprime - q * MN_KC) + 15) & ~15;  // whole products
+        if (mine) {
+          size_t o[MN_KC / 16];
+          bool in[MN_KC / 16];
+          uint32_t so[MN_KC / 16];
+#pragma unroll
+          for (int i = 0; i < MN_KC / 16; ++i) {
+            const int r = r0 + 16 * i, k = q * MN_KC + r;
+            const int pl = k / A.ppfv, pk = k - pl * A.ppfv;
+            in[i] = k < A.kprime;
+            o[i] = in[i] ? base + (size_t)(pl * pl_step) * plane + (size_t)pk * A.nant : 0;
+            so[i] = jo + (uint32_t)r * 128u + (uint32_t)(((j ^ r) & 7) << 4);
+          }
+          if constexpr (COPY) {
+#pragma unroll
+            for (int i = 0; i < MN_KC / 16; ++i) {
+              if (r0 + 16 * i >= rows) continue;
+              if (in[i]) {
+                cp_async16(smem_u32(st + so[i]), static_cast<const __half*>(A.re) + o[i]);
+                cp_async16(smem_u32(st + MN_PART + so[i]), static_cast<const __half*>(A.im) + o[i]);
+              } else {
+                *reinterpret_cast<uint4*>(st + so[i]) = make_uint4(0u, 0u, 0u, 0u);
+                *reinterpret_cast<uint4*>(st + MN_PART + so[i]) = make_uint4(0u, 0u, 0u, 0u);
+              }
+            }
+          } else {
+            uint32_t wr[MN_KC / 16][2 * ESZ + 1], wi[MN_KC / 16][2 * ESZ + 1];
+#pragma unroll
+            for (int i = 0; i < MN_KC / 16; ++i)
+              if (in[i]) {
+                mn_words<ESZ>(A.re, o[i] + A.off_re, nw_re, wr[i]);
+                mn_words<ESZ>(A.im, o[i] + A.off_im, nw_im, wi[i]);
+              }
+#pragma unroll
+            for (int i = 0; i < MN_KC / 16; ++i) {
+              if (r0 + 16 * i >= rows) continue;
+              const uint4 z = make_uint4(0u, 0u, 0u, 0u);
+              *reinterpret_cast<uint4*>(st + so[i]) = in[i] ? mn_shift<ESZ>(o[i] + A.off_re, wr[i]) : z;
+              *reinterpret_cast<uint4*>(st + MN_PART + so[i]) =
+                  in[i] ? mn_shift<ESZ>(o[i] + A.off_im, wi[i]) : z;
+            }
+          }
+        }
+      }
+      if constexpr (COPY) {
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (it >= lag) asm volatile("cp.async.wait_group %0;" ::"n"(MN_LAG) : "memory");
+      }
+      if (it >= lag) {
+        fence_proxy_async_smem();
+        mbar_arrive(&bar_full[(it - lag) % MN_NST]);
+      }
+    }
+    if constexpr (COPY) asm volatile("cp.async.wait_group 0;" ::: "memory");
+  } else if (lane == 0) {
+    // ---- issue the products ----
+    // c_format F32, a/b format F16, both MN-major; N = nant in 16s; M = 128
+    const uint32_t n_b = (uint32_t)((A.nant + 15) & ~15);
+    const uint32_t idesc = (1u << 4) | (1u << 15) | (1u << 16) | ((n_b >> 3) << 17) |
+                           ((128u >> 4) << 24);
+    constexpr uint32_t NEG_A = 1u << 13;
+    for (int it = 0; ok && it < n_items; ++it) {
+      const int lu = it / A.n_chunks, q = it % A.n_chunks;
+      const int slot = it % MN_NST, buf = lu & 1;
+      if (q == 0 && lu >= 2) ok = mbar_wait(&bar_out[buf], (uint32_t)(((lu >> 1) - 1) & 1));
+      ok = ok && mbar_wait(&bar_full[slot], (uint32_t)((it / MN_NST) & 1));
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t dr = tmem_base + (uint32_t)(buf * 256), di = dr + 128u;
+      const uint32_t sr = smem_u32(stages + (size_t)slot * MN_STAGE);
+      const int n16 = (min(MN_KC, A.kprime - q * MN_KC) + 15) >> 4;
+      for (int m = 0; m < n16; ++m) {
+        const uint64_t R = sdesc_mn_sw128(sr + (uint32_t)m * 2048u, MN_KC * 128, 1024);
+        const uint64_t I = sdesc_mn_sw128(sr + MN_PART + (uint32_t)m * 2048u, MN_KC * 128, 1024);
+        const uint32_t acc = (q > 0 || m > 0) ? 1u : 0u;
+        umma_f16_ss(dr, R, R, idesc, acc);
+        umma_f16_ss(dr, I, I, idesc, 1u);
+        umma_f16_ss(di, R, I, idesc, acc);
+        umma_f16_ss(di, I, R, idesc | NEG_A, 1u);
+      }
+      umma_commit(&bar_free[slot]);
+      if (q == A.n_chunks - 1) umma_commit(&bar_acc[buf]);
+    }
+    // a wait that ran out anywhere: every product issued here has to end
+    // before tensor memory and the stages are given back
+    umma_commit(bar_drain);
+    mbar_wait(bar_drain, 0u);
+  }
+  if (!ok && lane == 0) dsb_flag(A.status, DSB_E_TIMEOUT);
+  __syncwarp();
   tc_fence_before();
   __syncthreads();
   if (warp == 0) {
@@ -980,7 +1238,7 @@ int dsb_corr_split(const void* re, const void* im, int in_dtype, int nchan, int 
   if (in_dtype != DSB_DT_INT8 && in_dtype != DSB_DT_F16 && in_dtype != DSB_DT_F32)
     return DSB_E_ARG;
   SplitTcArgs A{};
-  A.re = re; A.im = im; A.dtype = in_dtype;
+  A.re = re; A.im = im;
   A.nchan = nchan; A.npkt = npkt; A.nant = nant;
   A.nant_p = (nant + 7) & ~7;
   A.ppfv = t_int / 2;
@@ -998,25 +1256,36 @@ int dsb_corr_split(const void* re, const void* im, int in_dtype, int nchan, int 
     A.n_units = A.n_fv * nchan * 2;
     A.kprime = t_int;               // (t-sub, packet)
   }
-  const int kc = in_dtype == DSB_DT_F32 ? 16 : 32;
+  const int kc = in_dtype == DSB_DT_F32 ? 16 : MN_KC;
   A.n_chunks = (A.kprime + kc - 1) / kc;
-  A.rows = std::max(128, 2 * A.nant_p);
-  A.stage_bytes = A.rows * 128;
-  A.nstage = 4;
   A.out = static_cast<float2*>(out);
   A.status = status;
-  const int smem = A.nstage * A.stage_bytes + 1024 + (A.nstage + 3) * 8 + 16;
   const int grid = std::min(A.n_units, num_sms());
   if (in_dtype == DSB_DT_F32) {
-    cudaFuncSetAttribute(corr_split_tc_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         smem);
-    corr_split_tc_kernel<4><<<grid, TC_THREADS, smem, stream>>>(A);
-  } else {
-    cudaFuncSetAttribute(corr_split_tc_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         smem);
-    corr_split_tc_kernel<2><<<grid, TC_THREADS, smem, stream>>>(A);
+    A.rows = std::max(128, 2 * A.nant_p);
+    A.stage_bytes = A.rows * 128;
+    A.nstage = 4;
+    const int smem = A.nstage * A.stage_bytes + 1024 + (A.nstage + 3) * 8 + 16;
+    cudaFuncSetAttribute(corr_split_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    corr_split_tc_kernel<<<grid, TC_THREADS, smem, stream>>>(A);
+    return launch_status();
   }
-  return launch_status();
+  const uintptr_t at_re = reinterpret_cast<uintptr_t>(re), at_im = reinterpret_cast<uintptr_t>(im);
+  const bool copy = in_dtype == DSB_DT_F16 && nant % 8 == 0 && (at_re | at_im) % 16 == 0;
+  const int esz = in_dtype == DSB_DT_INT8 ? 1 : 2;
+  if ((at_re | at_im) % esz) return DSB_E_ARG;
+  A.off_re = (int)(at_re % 4) / esz;
+  A.off_im = (int)(at_im % 4) / esz;
+  A.re = reinterpret_cast<const void*>(at_re & ~(uintptr_t)3);
+  A.im = reinterpret_cast<const void*>(at_im & ~(uintptr_t)3);
+  auto go = [&](auto kern) {
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MN_SMEM);
+    kern<<<grid, MN_THREADS, MN_SMEM, stream>>>(A);
+    return launch_status();
+  };
+  if (in_dtype == DSB_DT_INT8) return go(corr_split_mn_kernel<1, false>);
+  if (copy) return go(corr_split_mn_kernel<2, true>);
+  return go(corr_split_mn_kernel<2, false>);
 }
 
 int dsb_corr_tc(const void* raw, long long raw_g_stride, int n_chgroup, int npkt, int nant,
