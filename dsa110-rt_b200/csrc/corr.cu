@@ -68,6 +68,86 @@ __global__ void unpack_kernel(const uint32_t* __restrict__ raw, int rows, int nc
   }
 }
 
+// Four nibbles (code XOR 8, so 0..15) -> four values code * scale, each the
+// float32 product rounded once more to T, packed in row order.  2^23 + n is
+// exact, so subtracting 2^23 + 8 gives the code without an integer
+// conversion (a quarter-rate instruction).
+template <typename T>
+DSB_DEV void four_codes(const uint32_t (&n)[4], float scale, T* dst);
+DSB_DEV float nib_value(uint32_t n, float scale) {
+  return (__uint_as_float(0x4B000000u | n) - 8388616.0f) * scale;
+}
+template <>
+DSB_DEV void four_codes<int8_t>(const uint32_t (&n)[4], float, int8_t* dst) {
+  const uint32_t w = n[0] | (n[1] << 8) | (n[2] << 16) | (n[3] << 24);
+  // code = n - 8 per byte: set a guard bit, subtract, restore the sign bits
+  *reinterpret_cast<uint32_t*>(dst) = ((w | 0x80808080u) - 0x08080808u) ^ 0x80808080u;
+}
+template <>
+DSB_DEV void four_codes<__half>(const uint32_t (&n)[4], float scale, __half* dst) {
+  const __half2 a = __floats2half2_rn(nib_value(n[0], scale), nib_value(n[1], scale));
+  const __half2 b = __floats2half2_rn(nib_value(n[2], scale), nib_value(n[3], scale));
+  *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<const uint32_t*>(&a),
+                                              *reinterpret_cast<const uint32_t*>(&b));
+}
+template <>
+DSB_DEV void four_codes<float>(const uint32_t (&n)[4], float scale, float* dst) {
+  *reinterpret_cast<float4*>(dst) = make_float4(nib_value(n[0], scale), nib_value(n[1], scale),
+                                                nib_value(n[2], scale), nib_value(n[3], scale));
+}
+
+// Tile: 128 rows x 32 channels, four rows per thread and access.  The kernel
+// is bound by memory (1 byte read, 2 parts written per sample); the 32 x 32
+// tile above writes 64 bytes of a float16 plane at a time, here it is 256.  A
+// thread loads four rows of one channel (a warp one 128-byte line per row)
+// and stores them as one 16-byte word at column (row / 4) ^ channel, so that
+// neither the stores (lanes along channels) nor the loads (lanes along rows)
+// of a quarter warp meet in a bank.  A native float16 page (0.3 GB to 1.2 GB):
+// 476 -> 265 us (5.7 TB/s).
+template <typename T>
+__global__ void __launch_bounds__(256) unpack4_kernel(const uint32_t* __restrict__ raw, int rows,
+                                                      int nchan, float scale,
+                                                      T* __restrict__ ore, T* __restrict__ oim) {
+  __shared__ uint4 tile[32][32];
+  const int r0 = blockIdx.x * 128, c0 = blockIdx.y * 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t w[4][4];
+  const int c = c0 + lane;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int r = r0 + 4 * (warp + 8 * i) + k;
+      w[i][k] = (r < rows && c < nchan) ? __ldg(raw + (size_t)r * nchan + c) : 0u;
+    }
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    tile[lane][(warp + 8 * i) ^ lane] = make_uint4(w[i][0], w[i][1], w[i][2], w[i][3]);
+  __syncthreads();
+  const int r = r0 + 4 * lane;
+  if (r >= rows) return;   // rows is a multiple of 4
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int cl = warp + 8 * i;
+    if (c0 + cl >= nchan) break;
+    const uint4 q = tile[cl][lane ^ cl];
+    const uint32_t x[4] = {q.x ^ 0x88888888u, q.y ^ 0x88888888u, q.z ^ 0x88888888u,
+                           q.w ^ 0x88888888u};
+#pragma unroll
+    for (int tp = 0; tp < 4; ++tp) {  // byte tp = (t, pol): low nibble re, high im
+      uint32_t re[4], im[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        re[k] = (x[k] >> (8 * tp)) & 15u;
+        im[k] = (x[k] >> (8 * tp + 4)) & 15u;
+      }
+      const size_t o = ((size_t)(c0 + cl) * 4 + tp) * rows + r;
+      four_codes<T>(re, scale, ore + o);
+      four_codes<T>(im, scale, oim + o);
+    }
+  }
+}
+
 // ===========================================================================
 // tensor-core correlator (tcgen05, kind::i8)
 // ===========================================================================
@@ -1208,25 +1288,27 @@ const char* dsb_strerror(int code) {
 int dsb_unpack_int4(const void* raw, int npkt, int nant, int nchan, int out_dtype, float scale,
                     void* out_re, void* out_im, cudaStream_t stream) {
   if (!raw || !out_re || !out_im || npkt <= 0 || nant <= 0 || nchan <= 0) return DSB_E_ARG;
+  if (out_dtype != DSB_DT_INT8 && out_dtype != DSB_DT_F16 && out_dtype != DSB_DT_F32)
+    return DSB_E_ARG;
   const int rows = npkt * nant;
-  dim3 grid((rows + 31) / 32, (nchan + 31) / 32), block(32, 8);
   const uint32_t* r = static_cast<const uint32_t*>(raw);
-  switch (out_dtype) {
-    case DSB_DT_INT8:
-      unpack_kernel<int8_t><<<grid, block, 0, stream>>>(r, rows, nchan, scale, (int8_t*)out_re,
-                                                        (int8_t*)out_im);
-      break;
-    case DSB_DT_F16:
-      unpack_kernel<__half><<<grid, block, 0, stream>>>(r, rows, nchan, scale, (__half*)out_re,
-                                                        (__half*)out_im);
-      break;
-    case DSB_DT_F32:
-      unpack_kernel<float><<<grid, block, 0, stream>>>(r, rows, nchan, scale, (float*)out_re,
-                                                       (float*)out_im);
-      break;
-    default: return DSB_E_ARG;
-  }
-  return launch_status();
+  // four rows per store where every plane of rows starts on that boundary
+  const size_t esz = out_dtype == DSB_DT_INT8 ? 1 : out_dtype == DSB_DT_F16 ? 2 : 4;
+  const bool four = rows % 4 == 0 && (((uintptr_t)out_re | (uintptr_t)out_im) % (4 * esz)) == 0;
+  auto go = [&](auto t) {
+    using T = decltype(t);
+    T *re = static_cast<T*>(out_re), *im = static_cast<T*>(out_im);
+    if (four)
+      unpack4_kernel<T><<<dim3((rows + 127) / 128, (nchan + 31) / 32), 256, 0, stream>>>(
+          r, rows, nchan, scale, re, im);
+    else
+      unpack_kernel<T><<<dim3((rows + 31) / 32, (nchan + 31) / 32), dim3(32, 8), 0, stream>>>(
+          r, rows, nchan, scale, re, im);
+    return launch_status();
+  };
+  if (out_dtype == DSB_DT_INT8) return go(int8_t{});
+  if (out_dtype == DSB_DT_F16) return go(__half{});
+  return go(float{});
 }
 
 int dsb_corr_split(const void* re, const void* im, int in_dtype, int nchan, int npkt, int nant,
