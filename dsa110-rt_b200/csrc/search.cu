@@ -206,6 +206,141 @@ __global__ void combine_dense_kernel(const int8_t* __restrict__ streams,
     reinterpret_cast<float2*>(out)[o] = make_float2(o_re, o_im);
 }
 
+// The half-spectrum combine on row pairs: CTA (u, t, f) sums full rows u and
+// N - u of every chgroup at time t - shift[f][g], four cells per 4-byte load,
+// then forms the half cells of both rows from shared memory: every stream
+// byte is loaded once (the kernel above loads each one twice, byte by byte,
+// for 318 us per fine DM of 64 times at N = 256, 16 chgroups).  Bound by the
+// stream reads (n_f x the streams' bytes through L2: fine DMs are the fastest
+// grid index, so those that share a time run together): 138 us.
+// Integers: sums of 4 bytes in two words of 16-bit lanes, the bytes offset to
+// unsigned, spilled to 32 bits every 256 chgroups.  Calibrated: each cell's
+// float chain over g is the one of the kernel above, bit for bit.
+constexpr int CP_MAX_THREADS = 512;
+template <bool CALIB, bool OUT_F16, bool PER_T>
+__global__ void __launch_bounds__(CP_MAX_THREADS) combine_pair_kernel(
+    const int8_t* __restrict__ streams, const int* __restrict__ shifts,
+    const float* __restrict__ scales, const float* __restrict__ off_re,
+    const float* __restrict__ off_im, void* __restrict__ out, int G, int t_stream, int N, int n_f,
+    int n_t, int t_lo, int fftshift, float prescale) {
+  extern __shared__ __align__(16) uint8_t cp_smem[];
+  int* acc_s = reinterpret_cast<int*>(cp_smem);   // [row u, row N - u][re, im][N], int or float
+  const int f = blockIdx.x % n_f, u = blockIdx.x / n_f;   // u in [0, N/2]
+  const int um = (N - u) % N;
+  const int t = blockIdx.y, ta = t + t_lo;
+  const int nw4 = N / 4, nh = N / 2 + 1;
+  const int n_rows = um == u ? 1 : 2;
+  const size_t nsq = (size_t)N * N;
+  const int* sh = shifts + (size_t)f * G;
+  for (int task = threadIdx.x; task < n_rows * 2 * nw4; task += blockDim.x) {
+    const int w4 = task % nw4, part = (task / nw4) & 1, row = task / (2 * nw4);
+    const int8_t* src = streams + (size_t)part * nsq + (size_t)(row ? um : u) * N + 4 * w4;
+    int* dst = acc_s + (size_t)(row * 2 + part) * N + 4 * w4;
+    if constexpr (!CALIB) {
+      int s0 = 0, s1 = 0, s2 = 0, s3 = 0;
+      for (int gb = 0; gb < G; gb += 256) {
+        uint32_t lo = 0u, hi = 0u;
+        int cnt = 0;
+        const int ge = min(G, gb + 256);
+#pragma unroll 8
+        for (int g = gb; g < ge; ++g) {
+          const int ts = ta - __ldg(sh + g);
+          if (ts >= 0 && ts < t_stream) {
+            const uint32_t b = __ldg(reinterpret_cast<const uint32_t*>(
+                                   src + ((size_t)g * t_stream + ts) * 2 * nsq)) ^ 0x80808080u;
+            lo += b & 0x00ff00ffu;
+            hi += (b >> 8) & 0x00ff00ffu;
+            ++cnt;
+          }
+        }
+        s0 += (int)(lo & 0xffffu) - 128 * cnt;
+        s1 += (int)(hi & 0xffffu) - 128 * cnt;
+        s2 += (int)(lo >> 16) - 128 * cnt;
+        s3 += (int)(hi >> 16) - 128 * cnt;
+      }
+      *reinterpret_cast<int4*>(dst) = make_int4(s0, s1, s2, s3);
+    } else {
+      float a[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+      for (int g = 0; g < G; ++g) {
+        const int ts = ta - __ldg(sh + g);
+        if (ts >= 0 && ts < t_stream) {
+          const size_t gt = PER_T ? (size_t)g * t_stream + ts : (size_t)g;
+          const float sc = __ldg(scales + gt), of = __ldg((part ? off_im : off_re) + gt);
+          const uint32_t b = __ldg(reinterpret_cast<const uint32_t*>(
+              src + ((size_t)g * t_stream + ts) * 2 * nsq));
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            a[k] = fmaf(sc, (float)(int8_t)(uint8_t)(b >> (8 * k)), a[k]) + of;
+        }
+      }
+      *reinterpret_cast<float4*>(dst) = make_float4(a[0], a[1], a[2], a[3]);
+    }
+  }
+  __syncthreads();
+  const size_t o0 = ((size_t)f * n_t + t) * N * nh;
+  for (int i = threadIdx.x; i < n_rows * nh; i += blockDim.x) {
+    const int row = i / nh, w = i % nh;
+    const int ur = row ? um : u, wm = w ? N - w : 0;
+    const int* d = acc_s + (size_t)(row * 2) * N;                        // this row
+    const int* m = acc_s + (size_t)((n_rows == 1 ? 0 : 1 - row) * 2) * N;  // its mirror
+    float o_re, o_im;
+    if constexpr (!CALIB) {
+      o_re = 0.5f * (float)(d[w] + m[wm]);
+      o_im = 0.5f * (float)(d[N + w] - m[N + wm]);
+    } else {
+      o_re = 0.5f * (__int_as_float(d[w]) + __int_as_float(m[wm]));
+      o_im = 0.5f * (__int_as_float(d[N + w]) - __int_as_float(m[N + wm]));
+    }
+    if (fftshift && ((ur + w) & 1)) {
+      o_re = -o_re;
+      o_im = -o_im;
+    }
+    o_re *= prescale;
+    o_im *= prescale;
+    const size_t o = o0 + (size_t)ur * nh + w;
+    if (OUT_F16)
+      reinterpret_cast<__half2*>(out)[o] = __floats2half2_rn(o_re, o_im);
+    else
+      reinterpret_cast<float2*>(out)[o] = make_float2(o_re, o_im);
+  }
+}
+
+// Whether combine_pair_kernel takes the streams: whole 4-byte words of cells
+// in every row (other shapes run one cell per thread above).
+bool combine_pair_ok(const void* streams, int N, int n_t) {
+  return N % 4 == 0 && N <= 8192 && n_t <= 65535 &&
+         (reinterpret_cast<uintptr_t>(streams) & 3) == 0;
+}
+
+int launch_combine_pair(const int8_t* streams, const int* shifts, const float* scales,
+                        const float* off_re, const float* off_im, int per_t, void* out,
+                        int out_f16, int G, int t_stream, int N, int n_f, int n_t, int t_lo,
+                        int fftshift, float prescale, cudaStream_t stream) {
+  const long long bx = (long long)(N / 2 + 1) * n_f;
+  if (bx > 0x7fffffffLL || n_t > 65535) return DSB_E_ARG;
+  const int threads = std::min(CP_MAX_THREADS, (N + 31) / 32 * 32);
+  const size_t smem = (size_t)4 * N * 4;
+  auto go = [&](auto kern) {
+    if (smem > 48 * 1024 &&
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+            cudaSuccess)
+      return DSB_E_CUDA;
+    kern<<<dim3((unsigned)bx, n_t), threads, smem, stream>>>(
+        streams, shifts, scales, off_re, off_im, out, G, t_stream, N, n_f, n_t, t_lo, fftshift,
+        prescale);
+    return cudaGetLastError() == cudaSuccess ? DSB_OK : DSB_E_CUDA;
+  };
+  if (!scales)
+    return out_f16 ? go(combine_pair_kernel<false, true, false>)
+                   : go(combine_pair_kernel<false, false, false>);
+  if (per_t)
+    return out_f16 ? go(combine_pair_kernel<true, true, true>)
+                   : go(combine_pair_kernel<true, false, true>);
+  return out_f16 ? go(combine_pair_kernel<true, true, false>)
+                 : go(combine_pair_kernel<true, false, false>);
+}
+
 // ===========================================================================
 // image mask / normalise into the detector cube layout
 //   cube[t, f, h, w] = img[f, t, h, w] * mask_f[f, h, w]
@@ -341,42 +476,120 @@ __global__ void padded_cumsum_kernel(const T* __restrict__ x, int n, long long i
   for (int r = 0; r < pr; ++r) cs[(long long)(1 + pl + n + r) * inner + e] = last;
 }
 
+// A CTA walks BA_T consecutive outputs of V x 128 adjacent cells, V cells per
+// thread and access: the prefix rows of one output are the next ones' too, so
+// all but the first touch of a row come from L1, and what bounds the kernel
+// is the L1 rate of its 2 K loads per output (then memory: every prefix read
+// and 6 to 8 bytes written once).  One output per thread, with two 64-bit
+// divisions and 2 K 4-byte loads from L2 each, took 309 us for 128 outputs of
+// 4 x 256^2 cells at boxcars 1..16; this takes 107 us.
+//
 // CHECK: every prefix row read must lie in [0, cs_rows); an output whose
 // widths / offsets would read outside gets S/N NaN and winner -1 instead
 // (the rows outside belong to no call's data: the shared scratch array of
 // dsb_boxcar_argmax_noalloc).
-template <bool OUT_F16, bool CHECK = false>
-__global__ void multi_boxcar_argmax_kernel(const float* __restrict__ cs, long long inner,
-                                           const int* __restrict__ widths,
-                                           const int* __restrict__ offsets,
-                                           const float* __restrict__ sinv, int K, int n_out,
-                                           int t_base, void* __restrict__ out_max,
-                                           int16_t* __restrict__ out_win, long long cs_rows = 0) {
-  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (long long)n_out * inner) return;
-  const int t = (int)(idx / inner);
-  const long long e = idx % inner;
-  const int ta = t + t_base;
-  float best = 0.f;
-  int win = 0;
-  for (int k = 0; k < K; ++k) {
-    const long long lo = (long long)ta + offsets[k], hi = lo + widths[k];
-    if (CHECK && (lo < 0 || hi < 0 || lo >= cs_rows || hi >= cs_rows)) {
-      best = __int_as_float(0x7fc00000);
-      win = -1;
-      break;
+constexpr int BA_THREADS = 128, BA_T = 16, BA_MAX_K = 32;
+
+template <int V, bool OUT_F16, bool CHECK>
+__global__ void __launch_bounds__(BA_THREADS) multi_boxcar_argmax_kernel(
+    const float* __restrict__ cs, long long inner, const int* __restrict__ widths,
+    const int* __restrict__ offsets, const float* __restrict__ sinv, int K, int n_out, int t_base,
+    void* __restrict__ out_max, int16_t* __restrict__ out_win, long long cs_rows, int n_tt) {
+  __shared__ int s_lo[BA_MAX_K], s_w[BA_MAX_K];
+  __shared__ float s_si[BA_MAX_K];
+  const bool tab = K <= BA_MAX_K;   // longer lists are read in place
+  if (tab && (int)threadIdx.x < K) {
+    s_lo[threadIdx.x] = offsets[threadIdx.x];
+    s_w[threadIdx.x] = widths[threadIdx.x];
+    s_si[threadIdx.x] = sinv[threadIdx.x];
+  }
+  __syncthreads();
+  const int* lo_p = tab ? s_lo : offsets;
+  const int* w_p = tab ? s_w : widths;
+  const float* si_p = tab ? s_si : sinv;
+  // time tiles fastest: the CTAs that run together share rows in L2
+  const long long e = ((long long)(blockIdx.x / n_tt) * BA_THREADS + threadIdx.x) * V;
+  const int t0 = (int)(blockIdx.x % n_tt) * BA_T, t1 = min(n_out, t0 + BA_T);
+  if (e >= inner) return;
+  using VT = typename std::conditional<V == 4, float4, float>::type;
+  for (int t = t0; t < t1; ++t) {
+    const long long ta = (long long)t + t_base;
+    float best[V];
+    int win[V];
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+      best[v] = 0.f;
+      win[v] = 0;
     }
-    const float s = (cs[hi * inner + e] - cs[lo * inner + e]) * sinv[k];
-    if (k == 0 || s > best) {
-      best = s;
-      win = k;
+#pragma unroll 4
+    for (int k = 0; k < K; ++k) {
+      const long long lo = ta + lo_p[k], hi = lo + w_p[k];
+      if (CHECK && (lo < 0 || hi < 0 || lo >= cs_rows || hi >= cs_rows)) {
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+          best[v] = __int_as_float(0x7fc00000);
+          win[v] = -1;
+        }
+        break;
+      }
+      const VT h4 = *reinterpret_cast<const VT*>(cs + hi * inner + e);
+      const VT l4 = *reinterpret_cast<const VT*>(cs + lo * inner + e);
+      const float* h = reinterpret_cast<const float*>(&h4);
+      const float* l = reinterpret_cast<const float*>(&l4);
+      const float si = si_p[k];
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        const float s = (h[v] - l[v]) * si;
+        if (k == 0 || s > best[v]) {
+          best[v] = s;
+          win[v] = k;
+        }
+      }
+    }
+    const long long o = (long long)t * inner + e;
+    if constexpr (V == 4) {
+      if (OUT_F16) {
+        __half2 a = __floats2half2_rn(best[0], best[1]), b = __floats2half2_rn(best[2], best[3]);
+        *reinterpret_cast<uint2*>(static_cast<__half*>(out_max) + o) =
+            make_uint2(*reinterpret_cast<uint32_t*>(&a), *reinterpret_cast<uint32_t*>(&b));
+      } else {
+        *reinterpret_cast<float4*>(static_cast<float*>(out_max) + o) =
+            make_float4(best[0], best[1], best[2], best[3]);
+      }
+      *reinterpret_cast<short4*>(out_win + o) =
+          make_short4((short)win[0], (short)win[1], (short)win[2], (short)win[3]);
+    } else {
+      if (OUT_F16)
+        static_cast<__half*>(out_max)[o] = __float2half_rn(best[0]);
+      else
+        static_cast<float*>(out_max)[o] = best[0];
+      out_win[o] = (int16_t)win[0];
     }
   }
-  if (OUT_F16)
-    reinterpret_cast<__half*>(out_max)[idx] = __float2half_rn(best);
-  else
-    reinterpret_cast<float*>(out_max)[idx] = best;
-  out_win[idx] = (int16_t)win;
+}
+
+// Launch on any shape: four cells per access where the rows of every array
+// start on that boundary.
+template <bool CHECK>
+int launch_argmax(const float* cs, long long inner, const int* widths, const int* offsets,
+                  const float* sinv, int K, int n_out, int t_base, void* out_max, int out_f16,
+                  int16_t* out_win, long long cs_rows, cudaStream_t stream) {
+  const bool four = inner % 4 == 0 && (reinterpret_cast<uintptr_t>(cs) % 16) == 0 &&
+                    (reinterpret_cast<uintptr_t>(out_max) % (out_f16 ? 8 : 16)) == 0 &&
+                    (reinterpret_cast<uintptr_t>(out_win) % 8) == 0;
+  const int n_tt = (n_out + BA_T - 1) / BA_T;
+  const long long per = (long long)BA_THREADS * (four ? 4 : 1);
+  const long long blocks = (inner + per - 1) / per * n_tt;
+  if (blocks > 0x7fffffffLL) return DSB_E_ARG;
+  auto go = [&](auto kern) {
+    kern<<<(unsigned)blocks, BA_THREADS, 0, stream>>>(cs, inner, widths, offsets, sinv, K, n_out,
+                                                      t_base, out_max, out_win, cs_rows, n_tt);
+    return cudaGetLastError() == cudaSuccess ? DSB_OK : DSB_E_CUDA;
+  };
+  if (four) return out_f16 ? go(multi_boxcar_argmax_kernel<4, true, CHECK>)
+                           : go(multi_boxcar_argmax_kernel<4, false, CHECK>);
+  return out_f16 ? go(multi_boxcar_argmax_kernel<1, true, CHECK>)
+                 : go(multi_boxcar_argmax_kernel<1, false, CHECK>);
 }
 
 __global__ void boxcar_from_cs_kernel(const float* __restrict__ cs, long long inner, int width,
@@ -1212,6 +1425,10 @@ int dsb_combine_dense(const void* streams, const int* shifts, const float* scale
   if (half && (N & 1)) return DSB_E_ARG;
   const bool calib = scales != nullptr;
   if (calib && (!off_re || !off_im)) return DSB_E_ARG;
+  if (half && combine_pair_ok(streams, N, t_det - t_lo))
+    return launch_combine_pair(static_cast<const int8_t*>(streams), shifts, scales, off_re, off_im,
+                               per_t, out, out_f16, G, t_stream, N, 1, t_det - t_lo, t_lo,
+                               fftshift, 1.f, stream);
   const int nw = half ? N / 2 + 1 : N;
   dim3 block(32, 4, 8);
   dim3 grid((nw + 31) / 32, (N + 3) / 4, (t_det - t_lo + 7) / 8);
@@ -1265,15 +1482,8 @@ int dsb_multi_boxcar_argmax(const float* cs, long long inner, const int* widths,
                             cudaStream_t stream) {
   if (!cs || !widths || !offsets || !sigma_inv || !out_max || !out_win || K < 1 || n_out <= 0)
     return DSB_E_ARG;
-  const long long total = (long long)n_out * inner;
-  const unsigned grid = (unsigned)((total + 255) / 256);
-  if (out_f16)
-    multi_boxcar_argmax_kernel<true><<<grid, 256, 0, stream>>>(
-        cs, inner, widths, offsets, sigma_inv, K, n_out, t_base, out_max, (int16_t*)out_win);
-  else
-    multi_boxcar_argmax_kernel<false><<<grid, 256, 0, stream>>>(
-        cs, inner, widths, offsets, sigma_inv, K, n_out, t_base, out_max, (int16_t*)out_win);
-  return launch_status();
+  return launch_argmax<false>(cs, inner, widths, offsets, sigma_inv, K, n_out, t_base, out_max,
+                              out_f16, static_cast<int16_t*>(out_win), 0, stream);
 }
 
 int dsb_boxcar_from_cs(const float* cs, long long inner, int width, int start, int n_out,
@@ -1504,15 +1714,6 @@ extern "C" int dsb_boxcar_argmax_noalloc(const void* x, int x_f16, int n, long l
   // against those (n + max_w) rows.
   const int rc = dsb_padded_cumsum(x, x_f16, n, inner, max_w, cs, stream);
   if (rc != DSB_OK) return rc;
-  const long long total = (long long)n_out * inner;
-  const unsigned grid = (unsigned)((total + 255) / 256);
-  if (out_f16)
-    multi_boxcar_argmax_kernel<true, true><<<grid, 256, 0, stream>>>(
-        cs, inner, widths, offsets, sigma_inv, K, n_out, t_base, out_max, (int16_t*)out_win,
-        rows);
-  else
-    multi_boxcar_argmax_kernel<false, true><<<grid, 256, 0, stream>>>(
-        cs, inner, widths, offsets, sigma_inv, K, n_out, t_base, out_max, (int16_t*)out_win,
-        rows);
-  return launch_status();
+  return launch_argmax<true>(cs, inner, widths, offsets, sigma_inv, K, n_out, t_base, out_max,
+                             out_f16, static_cast<int16_t*>(out_win), rows, stream);
 }
