@@ -212,11 +212,13 @@ __global__ void combine_dense_kernel(const int8_t* __restrict__ streams,
 // byte is loaded once (the kernel above loads each one twice, byte by byte,
 // for 318 us per fine DM of 64 times at N = 256, 16 chgroups).  Bound by the
 // stream reads (n_f x the streams' bytes through L2: fine DMs are the fastest
-// grid index, so those that share a time run together): 138 us.
+// grid index, so those that share a time run together): 40 us with 8 fine
+// DMs in one launch (dsb_combine_dense_fdm).
 // Integers: sums of 4 bytes in two words of 16-bit lanes, the bytes offset to
 // unsigned, spilled to 32 bits every 256 chgroups.  Calibrated: each cell's
 // float chain over g is the one of the kernel above, bit for bit.
 constexpr int CP_MAX_THREADS = 512;
+constexpr int CP_G = 256;   // chgroups per staged list (16-bit lanes hold 257)
 template <bool CALIB, bool OUT_F16, bool PER_T>
 __global__ void __launch_bounds__(CP_MAX_THREADS) combine_pair_kernel(
     const int8_t* __restrict__ streams, const int* __restrict__ shifts,
@@ -224,6 +226,9 @@ __global__ void __launch_bounds__(CP_MAX_THREADS) combine_pair_kernel(
     const float* __restrict__ off_im, void* __restrict__ out, int G, int t_stream, int N, int n_f,
     int n_t, int t_lo, int fftshift, float prescale) {
   extern __shared__ __align__(16) uint8_t cp_smem[];
+  __shared__ size_t s_off[CP_G];
+  __shared__ float s_cal[3][CALIB ? CP_G : 1];
+  __shared__ int s_n;
   int* acc_s = reinterpret_cast<int*>(cp_smem);   // [row u, row N - u][re, im][N], int or float
   const int f = blockIdx.x % n_f, u = blockIdx.x / n_f;   // u in [0, N/2]
   const int um = (N - u) % N;
@@ -232,49 +237,68 @@ __global__ void __launch_bounds__(CP_MAX_THREADS) combine_pair_kernel(
   const int n_rows = um == u ? 1 : 2;
   const size_t nsq = (size_t)N * N;
   const int* sh = shifts + (size_t)f * G;
-  for (int task = threadIdx.x; task < n_rows * 2 * nw4; task += blockDim.x) {
-    const int w4 = task % nw4, part = (task / nw4) & 1, row = task / (2 * nw4);
-    const int8_t* src = streams + (size_t)part * nsq + (size_t)(row ? um : u) * N + 4 * w4;
-    int* dst = acc_s + (size_t)(row * 2 + part) * N + 4 * w4;
-    if constexpr (!CALIB) {
-      int s0 = 0, s1 = 0, s2 = 0, s3 = 0;
-      for (int gb = 0; gb < G; gb += 256) {
-        uint32_t lo = 0u, hi = 0u;
-        int cnt = 0;
-        const int ge = min(G, gb + 256);
-#pragma unroll 8
-        for (int g = gb; g < ge; ++g) {
-          const int ts = ta - __ldg(sh + g);
-          if (ts >= 0 && ts < t_stream) {
-            const uint32_t b = __ldg(reinterpret_cast<const uint32_t*>(
-                                   src + ((size_t)g * t_stream + ts) * 2 * nsq)) ^ 0x80808080u;
-            lo += b & 0x00ff00ffu;
-            hi += (b >> 8) & 0x00ff00ffu;
-            ++cnt;
+  for (int gb = 0; gb < G; gb += CP_G) {
+    // the chgroups that have this time, in order, with their planes' offsets
+    // (warp 0), so that the loop below has only independent loads
+    if (gb) __syncthreads();
+    if (threadIdx.x < 32) {
+      int n = 0;
+      for (int g0 = gb; g0 < min(G, gb + CP_G); g0 += 32) {
+        const int g = g0 + (int)threadIdx.x;
+        const int ts = g < min(G, gb + CP_G) ? ta - __ldg(sh + g) : -1;
+        const bool in = ts >= 0 && ts < t_stream;
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        if (in) {
+          const int i = n + __popc(m & ((1u << threadIdx.x) - 1u));
+          s_off[i] = ((size_t)g * t_stream + ts) * 2 * nsq;
+          if constexpr (CALIB) {
+            const size_t gt = PER_T ? (size_t)g * t_stream + ts : (size_t)g;
+            s_cal[0][i] = __ldg(scales + gt);
+            s_cal[1][i] = __ldg(off_re + gt);
+            s_cal[2][i] = __ldg(off_im + gt);
           }
         }
-        s0 += (int)(lo & 0xffffu) - 128 * cnt;
-        s1 += (int)(hi & 0xffffu) - 128 * cnt;
-        s2 += (int)(lo >> 16) - 128 * cnt;
-        s3 += (int)(hi >> 16) - 128 * cnt;
+        n += __popc(m);
       }
-      *reinterpret_cast<int4*>(dst) = make_int4(s0, s1, s2, s3);
-    } else {
-      float a[4] = {0.f, 0.f, 0.f, 0.f};
+      if (threadIdx.x == 0) s_n = n;
+    }
+    __syncthreads();
+    const int n = s_n;
+    for (int task = threadIdx.x; task < n_rows * 2 * nw4; task += blockDim.x) {
+      const int w4 = task % nw4, part = (task / nw4) & 1, row = task / (2 * nw4);
+      const int8_t* src = streams + (size_t)part * nsq + (size_t)(row ? um : u) * N + 4 * w4;
+      int* dst = acc_s + (size_t)(row * 2 + part) * N + 4 * w4;
+      if constexpr (!CALIB) {
+        uint32_t lo = 0u, hi = 0u;
+#pragma unroll 8
+        for (int i = 0; i < n; ++i) {
+          const uint32_t b = __ldg(reinterpret_cast<const uint32_t*>(src + s_off[i])) ^ 0x80808080u;
+          lo += b & 0x00ff00ffu;
+          hi += (b >> 8) & 0x00ff00ffu;
+        }
+        int4 q = make_int4((int)(lo & 0xffffu) - 128 * n, (int)(hi & 0xffffu) - 128 * n,
+                           (int)(lo >> 16) - 128 * n, (int)(hi >> 16) - 128 * n);
+        if (gb) {
+          const int4 o = *reinterpret_cast<const int4*>(dst);
+          q = make_int4(q.x + o.x, q.y + o.y, q.z + o.z, q.w + o.w);
+        }
+        *reinterpret_cast<int4*>(dst) = q;
+      } else {
+        float a[4] = {0.f, 0.f, 0.f, 0.f};
+        if (gb) {
+          const float4 o = *reinterpret_cast<const float4*>(dst);
+          a[0] = o.x; a[1] = o.y; a[2] = o.z; a[3] = o.w;
+        }
 #pragma unroll 4
-      for (int g = 0; g < G; ++g) {
-        const int ts = ta - __ldg(sh + g);
-        if (ts >= 0 && ts < t_stream) {
-          const size_t gt = PER_T ? (size_t)g * t_stream + ts : (size_t)g;
-          const float sc = __ldg(scales + gt), of = __ldg((part ? off_im : off_re) + gt);
-          const uint32_t b = __ldg(reinterpret_cast<const uint32_t*>(
-              src + ((size_t)g * t_stream + ts) * 2 * nsq));
+        for (int i = 0; i < n; ++i) {
+          const uint32_t b = __ldg(reinterpret_cast<const uint32_t*>(src + s_off[i]));
+          const float sc = s_cal[0][i], of = s_cal[1 + part][i];
 #pragma unroll
           for (int k = 0; k < 4; ++k)
             a[k] = fmaf(sc, (float)(int8_t)(uint8_t)(b >> (8 * k)), a[k]) + of;
         }
+        *reinterpret_cast<float4*>(dst) = make_float4(a[0], a[1], a[2], a[3]);
       }
-      *reinterpret_cast<float4*>(dst) = make_float4(a[0], a[1], a[2], a[3]);
     }
   }
   __syncthreads();
@@ -1448,6 +1472,19 @@ int dsb_combine_dense(const void* streams, const int* shifts, const float* scale
   };
   half ? by_c(T{}) : by_c(F{});
   return launch_status();
+}
+
+int dsb_combine_dense_fdm(const void* streams, const int* shifts, int n_f, const float* scales,
+                          const float* off_re, const float* off_im, int per_t, void* out, int G,
+                          int t_stream, int N, int n_t, int t_lo, int fftshift, float prescale,
+                          cudaStream_t stream) {
+  if (!streams || !shifts || !out || n_f <= 0 || G <= 0 || N <= 0 || (N & 1) || n_t <= 0 ||
+      t_lo < 0 || t_stream <= 0 || (scales && (!off_re || !off_im)))
+    return DSB_E_ARG;
+  if (!combine_pair_ok(streams, N, n_t)) return DSB_E_UNSUPPORTED;
+  return launch_combine_pair(static_cast<const int8_t*>(streams), shifts, scales, off_re, off_im,
+                             per_t, out, 0, G, t_stream, N, n_f, n_t, t_lo, fftshift, prescale,
+                             stream);
 }
 
 int dsb_mask_to_cube(const float* img, const float* mask, int mask_per_f, int n_f, int n_t,

@@ -51,6 +51,10 @@ _SIGNATURES = {
     "dsb_graph_abort": [_vp],
     "dsb_graph_destroy": [_vp],
     "dsb_irfft2": [_vp, _c_int, _c_int, _vp, _vp, _vp],
+    "dsb_irfft2_cube": [_vp, _c_ll, _c_int, _c_int, _c_int, _vp, _vp, _c_int, _vp, _c_int,
+                        _c_int, _c_int, _vp],
+    "dsb_combine_dense_fdm": [_vp, _vp, _c_int, _vp, _vp, _vp, _c_int, _vp, _c_int, _c_int,
+                              _c_int, _c_int, _c_int, _c_int, _c_float, _vp],
     "dsb_image_fft": [_vp, _c_int, _vp, _vp, _vp, _vp, _vp, _vp, _c_int, _c_int, _c_int, _vp, _vp, _vp, _c_int, _vp, _vp, _vp, _c_int,
                       _c_int, _vp,
                       _vp, _c_int, _vp, _c_int, _vp, _vp, _vp, _vp, _vp, _c_int, _c_int, _c_int,

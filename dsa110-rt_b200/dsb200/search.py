@@ -24,26 +24,21 @@ from . import _lib
 # ---------------------------------------------------------------------------
 
 
-def _combine_dense(streams_cint8, shifts, output, *, half, scales, offsets_re, offsets_im,
-                   t_lo, fftshift):
-    for t, nm in ((streams_cint8, "streams_cint8"), (shifts, "shifts"), (output, "output")):
-        _lib.require_cuda(t, nm)
+def _stream_shape(streams_cint8):
     if streams_cint8.dtype != torch.int8 or streams_cint8.ndim != 5 or streams_cint8.shape[2] != 2:
         raise RuntimeError(f"streams_cint8 must be int8 [G, T, 2, N, N]; got "
                            f"{streams_cint8.dtype} {tuple(streams_cint8.shape)}")
     G, T, _, N, N2 = streams_cint8.shape
     if N != N2:
         raise RuntimeError("streams_cint8 grid must be square")
-    if shifts.dtype != torch.int32 or shifts.shape != (G,):
-        raise RuntimeError(f"shifts must be int32 ({G},)")
-    nw = N // 2 + 1 if half else N
-    if output.ndim != 3 or output.shape[1:] != (N, nw):
-        raise RuntimeError(f"output must be [T_det - t_lo, {N}, {nw}]; got {tuple(output.shape)}")
-    if output.dtype not in (torch.complex32, torch.complex64):
-        raise RuntimeError(f"output dtype {output.dtype} not in (complex32, complex64)")
+    return G, T, N
+
+
+def _stream_calibration(G, T, scales, offsets_re, offsets_im):
+    """(calibrated, per source time): per-(chgroup, source time) scales [G, T]
+    (the wire's per-tile scales) when all three are 2-D, as
+    fused_combine_cuda.py:1299-1330 decides."""
     calib = scales is not None
-    # per-(chgroup, source time) scales [G, T] (the wire's per-tile scales) when
-    # all three are 2-D, as fused_combine_cuda.py:1299-1330 decides
     per_t = calib and all(t is not None and t.dim() == 2
                           for t in (scales, offsets_re, offsets_im))
     if calib:
@@ -54,6 +49,22 @@ def _combine_dense(streams_cint8, shifts, output, *, half, scales, offsets_re, o
             _lib.require_cuda(t, nm)
             if not t.is_contiguous():
                 raise RuntimeError(f"{nm} must be contiguous")
+    return calib, per_t
+
+
+def _combine_dense(streams_cint8, shifts, output, *, half, scales, offsets_re, offsets_im,
+                   t_lo, fftshift):
+    for t, nm in ((streams_cint8, "streams_cint8"), (shifts, "shifts"), (output, "output")):
+        _lib.require_cuda(t, nm)
+    G, T, N = _stream_shape(streams_cint8)
+    if shifts.dtype != torch.int32 or shifts.shape != (G,):
+        raise RuntimeError(f"shifts must be int32 ({G},)")
+    nw = N // 2 + 1 if half else N
+    if output.ndim != 3 or output.shape[1:] != (N, nw):
+        raise RuntimeError(f"output must be [T_det - t_lo, {N}, {nw}]; got {tuple(output.shape)}")
+    if output.dtype not in (torch.complex32, torch.complex64):
+        raise RuntimeError(f"output dtype {output.dtype} not in (complex32, complex64)")
+    calib, per_t = _stream_calibration(G, T, scales, offsets_re, offsets_im)
     t_det = int(t_lo) + int(output.shape[0])
     _lib.check(_lib.lib().dsb_combine_dense(
         _lib.ptr(streams_cint8), _lib.ptr(shifts), _lib.ptr(scales if calib else None),
@@ -165,6 +176,17 @@ def combine_sparse_v4(dense: torch.Tensor, csr: SparseCellCsr, shifts: torch.Ten
     also, complex64) at rows ``out_row0 ..``: the caller zeroes the rest.
     ``threads`` and the shift bounds are accepted for the reference's
     signature; this kernel needs neither."""
+    st = _lib.status_word(out.device)
+    _combine_sparse(dense, csr, shifts, t_rows=t_rows, t_out_len=t_out_len, t_lo=t_lo,
+                    fftshift=fftshift, out=out, out_row0=out_row0, status=st)
+    _lib.check_status(st, "dsb_combine_sparse")
+    return out
+
+
+def _combine_sparse(dense, csr, shifts, *, t_rows, t_out_len, t_lo, fftshift, out, out_row0,
+                    status) -> None:
+    """combine_sparse_v4's checks and launch; the device status is the
+    caller's to read."""
     n_sb, nfm, t_pad, two = dense.shape
     if two != 2 or n_sb != csr.n_sb:
         raise ValueError(f"dense {tuple(dense.shape)} does not match csr n_sb={csr.n_sb}")
@@ -195,15 +217,12 @@ def combine_sparse_v4(dense: torch.Tensor, csr: SparseCellCsr, shifts: torch.Ten
     for x, nm in ((dense, "dense"), (shifts, "shifts"), (out, "out")):
         _lib.require_cuda(x, nm)
     sh = shifts.to(torch.int32).contiguous()
-    st = _lib.status_word(out.device)
     _lib.check(_lib.lib().dsb_combine_sparse(
         _lib.ptr(dense), _lib.ptr(csr.cell_uw), _lib.ptr(csr.cell_ptr), _lib.ptr(csr.ent_g),
         _lib.ptr(csr.ent_k), _lib.ptr(csr.ent_km), csr.n_cells, _lib.ptr(sh), _lib.ptr(out),
         f16, n_sb, int(t_rows), int(t_pad), int(nfm), N, n_fdm, int(t_out_len), int(t_lo),
-        int(bool(fftshift)), out_rows, int(out_row0), _lib.ptr(st),
+        int(bool(fftshift)), out_rows, int(out_row0), _lib.ptr(status),
         _lib.stream_of(out.device)), "dsb_combine_sparse")
-    _lib.check_status(st, "dsb_combine_sparse")
-    return out
 
 
 # ---------------------------------------------------------------------------
@@ -356,16 +375,10 @@ class GpuImager:
         shape = (config.t_det, config.n_fdm, N, N)
         out = torch.empty(shape, dtype=config.cube_dtype, device=dev)
         out_alt = torch.empty(shape, dtype=config.cube_dtype, device=dev)
-        uv = torch.empty((config.t_det, N, N // 2 + 1), dtype=torch.complex64, device=dev)
+        # half spectra: a chunk of process_cube, at least one fine DM's times
+        n_uv = max(config.t_det, min(config.t_det * config.n_fdm, cls._chunk_images(N)))
+        uv = torch.empty((n_uv, N, N // 2 + 1), dtype=torch.complex64, device=dev)
         return cls(config, dev, edge_t, out, out_alt, uv)
-
-    def _img_buffer(self, n_t: int) -> torch.Tensor:
-        N = self.config.n_grid
-        buf = getattr(self, "_img", None)
-        if buf is None or buf.shape[0] < n_t:
-            buf = self._img = torch.empty((self.config.t_det, N, N), dtype=torch.float32,
-                                          device=self.device)
-        return buf[:n_t]
 
     def set_edge_mask_per_fdm(self, sigma_inv: Optional[torch.Tensor]) -> None:
         """``edge_mask * sigma_inv[f]`` per fine DM (the Layer-1 divide fused
@@ -398,7 +411,8 @@ class GpuImager:
                              f"({cfg.n_fdm}, {streams_cint8.shape[0]})")
         N = cfg.n_grid
         n_t = cfg.t_det - t_lo
-        uv = self.uv_slab[:n_t]
+        if t_lo < 0 or n_t <= 0:
+            raise ValueError(f"t_lo={t_lo} outside [0, t_det={cfg.t_det})")
         cube = self.output_cube_alt if self._flip else self.output_cube
         self._flip = not self._flip
         shifts = time_shifts_gpu.to(torch.int32).contiguous()
@@ -406,26 +420,85 @@ class GpuImager:
             return self._process_compact(streams_cint8, shifts, compact_inv_lut,
                                          int(compact_t_stream), t_lo, cube,
                                          (chgroup_scales, chgroup_offsets_re, chgroup_offsets_im))
-        for f in range(cfg.n_fdm):
-            fused_dequant_combine_per_fdm_half(streams_cint8, shifts[f], uv,
-                                               scales=chgroup_scales,
-                                               offsets_re=chgroup_offsets_re,
-                                               offsets_im=chgroup_offsets_im, t_lo=t_lo,
-                                               fftshift=True)
-            if cfg.imager_uv_prescale != 1.0:
-                uv.mul_(cfg.imager_uv_prescale)
-            img = irfft2_image(uv, N, out=self._img_buffer(n_t))[None]   # (1, n_t, N, N)
-            mask = (self.edge_mask_real if self.edge_mask_per_fdm is None
-                    else self.edge_mask_per_fdm[f:f + 1])
-            mask_into_cube(img.contiguous(), mask, cube[t_lo:] if t_lo else cube, f)
+        _lib.require_cuda(streams_cint8, "streams_cint8")
+        _lib.require_cuda(shifts, "shifts")
+        G, T, N2 = _stream_shape(streams_cint8)
+        if N2 != N:
+            raise RuntimeError(f"streams_cint8 grid {N2} != n_grid {N}")
+        calib, per_t = _stream_calibration(G, T, chgroup_scales, chgroup_offsets_re,
+                                           chgroup_offsets_im)
+        if streams_cint8.data_ptr() % 4:
+            # off the combine's 4-byte loads: one fine DM at a time
+            for f in range(cfg.n_fdm):
+                uv = self.uv_slab[:n_t]
+                fused_dequant_combine_per_fdm_half(
+                    streams_cint8, shifts[f], uv, scales=chgroup_scales,
+                    offsets_re=chgroup_offsets_re, offsets_im=chgroup_offsets_im, t_lo=t_lo,
+                    fftshift=True)
+                if cfg.imager_uv_prescale != 1.0:
+                    uv.mul_(cfg.imager_uv_prescale)
+                self._transform_to_cube(uv, 1, n_t, cube, f, t_lo)
+            return cube
+        for f0, n_f, t0, nt, work in self._chunks(t_lo, all_times=False):
+            _lib.check(_lib.lib().dsb_combine_dense_fdm(
+                _lib.ptr(streams_cint8), _lib.ptr(shifts[f0:f0 + n_f]), n_f,
+                _lib.ptr(chgroup_scales if calib else None),
+                _lib.ptr(chgroup_offsets_re if calib else None),
+                _lib.ptr(chgroup_offsets_im if calib else None), int(per_t), _lib.ptr(work), G, T,
+                N, nt, t0, 1, float(cfg.imager_uv_prescale), _lib.stream_of(self.device)),
+                "dsb_combine_dense_fdm")
+            self._transform_to_cube(work, n_f, nt, cube, f0, t0)
         return cube
 
+    # half spectra in flight between the combine, the column pass and the row
+    # pass: what stays in L2 (126 MB) beside the streams and the cube's writes
+    WORK_BYTES = 48 << 20
+
+    @classmethod
+    def _chunk_images(cls, N: int) -> int:
+        return max(1, min(cls.WORK_BYTES // (N * (N // 2 + 1) * 8), 65535))
+
+    def _chunks(self, t_lo: int, *, all_times: bool):
+        """The cube's (fine DM, time) images in chunks of at most WORK_BYTES of
+        half spectra: (f0, n_f, t0, n_t, work [n_f, n_t, N, N/2+1]).  Dense
+        streams: every fine DM of a time range together (they read the same
+        stream times, which then stay in L2: 318 us a pass at 16 chgroups, 8
+        fine DMs x 64 times of 256^2, against 1103 us one fine DM at a time).
+        all_times, for compact streams: every time of some fine DMs (the
+        streams fit L2 whole, and the combine works in 64-time tiles)."""
+        cfg = self.config
+        N, nh = cfg.n_grid, cfg.n_grid // 2 + 1
+        cap = self._chunk_images(N)
+        if all_times:
+            nt_c = min(cfg.t_det, cap)
+            nf_c = min(cfg.n_fdm, cap // nt_c)
+        else:
+            nf_c = min(cfg.n_fdm, cap)
+            nt_c = min(cfg.t_det, cap // nf_c)
+        buf = self.uv_slab.view(-1)
+        for t0 in range(t_lo, cfg.t_det, nt_c):
+            nt = min(nt_c, cfg.t_det - t0)
+            for f0 in range(0, cfg.n_fdm, nf_c):
+                n_f = min(nf_c, cfg.n_fdm - f0)
+                yield f0, n_f, t0, nt, buf[:n_f * nt * N * nh].view(n_f, nt, N, nh)
+
+    def _transform_to_cube(self, work, n_f: int, n_t: int, cube, f0: int, t0: int) -> None:
+        """Inverse real FFT of ``work`` [n_f, n_t, N, N/2+1] (overwritten) times
+        the mask into ``cube[t0:t0 + n_t, f0:f0 + n_f]``."""
+        N = self.config.n_grid
+        per_f = self.edge_mask_per_fdm is not None
+        mask = self.edge_mask_per_fdm[f0:f0 + n_f] if per_f else self.edge_mask_real
+        _lib.check(_lib.lib().dsb_irfft2_cube(
+            _lib.ptr(work), n_t * N * (N // 2 + 1), n_f, n_t, N,
+            _lib.ptr(twiddles(N, self.device)), _lib.ptr(mask), int(per_f), _lib.ptr(cube[t0:]),
+            int(cube.dtype == torch.float16), int(cube.shape[1]), f0,
+            _lib.stream_of(self.device)), "dsb_irfft2_cube")
 
     def _process_compact(self, streams, shifts, inv_lut, t_stream, t_lo, cube, calib):
         """The compact path of process_cube (imager_gpu.py:300-330, 487-520):
-        ``streams [N_chg, n_filled_max, t_pad, 2]`` int8 time-minor, every
-        fine DM combined in one launch (combine_sparse_v4) into a zeroed
-        half-spectrum buffer, then the transform and mask per fine DM."""
+        ``streams [N_chg, n_filled_max, t_pad, 2]`` int8 time-minor, combined
+        (combine_sparse_v4's kernel) into zeroed half spectra, then the
+        transform and mask."""
         cfg = self.config
         N = cfg.n_grid
         if streams.ndim != 4 or streams.shape[3] != 2:
@@ -443,23 +516,15 @@ class GpuImager:
         if getattr(self, "_csr_key", None) != key:
             self._csr = build_sparse_cell_csr(inv_lut, n_grid=N)
             self._csr_key = key
-        full = getattr(self, "_uv_full", None)
-        if full is None:
-            full = self._uv_full = torch.empty((cfg.n_fdm, cfg.t_det, N, N // 2 + 1),
-                                               dtype=torch.complex64, device=self.device)
-        full[:, t_lo:cfg.t_det].zero_()
-        combine_sparse_v4(streams, self._csr, shifts, t_rows=t_stream,
-                          t_out_len=cfg.t_det - t_lo, t_lo=t_lo, fftshift=True, out=full,
-                          out_row0=t_lo, shift_min=0, shift_max=0)
-        n_t = cfg.t_det - t_lo
-        for f in range(cfg.n_fdm):
-            uv = full[f, t_lo:cfg.t_det]
+        st = _lib.status_word(self.device)
+        for f0, n_f, t0, nt, work in self._chunks(t_lo, all_times=True):
+            work.zero_()
+            _combine_sparse(streams, self._csr, shifts[f0:f0 + n_f], t_rows=t_stream,
+                            t_out_len=nt, t_lo=t0, fftshift=True, out=work, out_row0=0, status=st)
             if cfg.imager_uv_prescale != 1.0:
-                uv.mul_(cfg.imager_uv_prescale)
-            img = irfft2_image(uv.contiguous(), N, out=self._img_buffer(n_t))[None]
-            mask = (self.edge_mask_real if self.edge_mask_per_fdm is None
-                    else self.edge_mask_per_fdm[f:f + 1])
-            mask_into_cube(img.contiguous(), mask, cube[t_lo:] if t_lo else cube, f)
+                work.mul_(cfg.imager_uv_prescale)
+            self._transform_to_cube(work, n_f, nt, cube, f0, t0)
+        _lib.check_status(st, "dsb_combine_sparse")
         return cube
 
 

@@ -272,6 +272,16 @@ int dsb_combine_dense(const void* streams, const int* shifts, const float* scale
                       int G, int t_stream, int t_det, int N, int t_lo, int fftshift,
                       cudaStream_t stream);
 
+/* The half-spectrum form of dsb_combine_dense for n_f fine DMs at once:
+ * shifts [n_f, G], out complex64 [n_f][n_t][N][N/2+1], times t_lo .. t_lo +
+ * n_t - 1, every value times prescale (imager_uv_prescale of GpuImager,
+ * src/dsart/image/imager_gpu.py:580).  Streams 4-byte aligned and N a
+ * multiple of 4, else DSB_E_UNSUPPORTED. */
+int dsb_combine_dense_fdm(const void* streams, const int* shifts, int n_f, const float* scales,
+                          const float* off_re, const float* off_im, int per_t, void* out, int G,
+                          int t_stream, int N, int n_t, int t_lo, int fftshift, float prescale,
+                          cudaStream_t stream);
+
 /* ---- a12/a13: fused combine + 2-D inverse real FFT ------------------------------
  * Replaces fused_dequant_combine_per_fdm_half + torch.fft.irfft2 inside
  * GpuImager.process_cube (src/dsart/image/fused_combine_cuda.py:1359,
@@ -343,6 +353,17 @@ int dsb_combine_dense(const void* streams, const int* shifts, const float* scale
  * complex64 exp(+2 pi i e/N).  N in {32, 64, 128, 256, 512}; n_img <= 65535. */
 int dsb_irfft2(void* half, int n_img, int N, const void* twiddles, float* out,
                cudaStream_t stream);
+
+/* dsb_irfft2 followed by dsb_mask_to_cube in one pass over the pixels: image
+ * (f, t) of half (at half + f * f_stride + t * N * (N/2+1), complex64, used
+ * as the work buffer) times mask (N x N, or mask_per_f: n_f x N x N) to
+ * cube[t][cube_f0 + f][N][N] (float16 or float32, cube_f_total fine DMs).
+ * mask 16-byte aligned, cube 16-byte (float16: 8-byte) aligned; n_f * n_t at
+ * most 65535.  Replaces the transform, mask and cube write of
+ * GpuImager.process_cube (src/dsart/image/imager_gpu.py:590-650). */
+int dsb_irfft2_cube(void* half, long long f_stride, int n_f, int n_t, int N, const void* twiddles,
+                    const float* mask, int mask_per_f, void* cube, int cube_f16, int cube_f_total,
+                    int cube_f0, cudaStream_t stream);
 
 /* The kernel's geometry at grid size n_grid, for building the tables above:
  * geom[0] fold (column passes, LC = N / fold), geom[1] threads per CTA,
