@@ -439,7 +439,7 @@ class GpuImager:
                     uv.mul_(cfg.imager_uv_prescale)
                 self._transform_to_cube(uv, 1, n_t, cube, f, t_lo)
             return cube
-        for f0, n_f, t0, nt, work in self._chunks(t_lo, all_times=False):
+        for f0, n_f, t0, nt, work in self._chunks(t_lo, self.uv_slab):
             _lib.check(_lib.lib().dsb_combine_dense_fdm(
                 _lib.ptr(streams_cint8), _lib.ptr(shifts[f0:f0 + n_f]), n_f,
                 _lib.ptr(chgroup_scales if calib else None),
@@ -450,32 +450,27 @@ class GpuImager:
             self._transform_to_cube(work, n_f, nt, cube, f0, t0)
         return cube
 
-    # half spectra in flight between the combine, the column pass and the row
-    # pass: what stays in L2 (126 MB) beside the streams and the cube's writes
-    WORK_BYTES = 48 << 20
+    # half spectra in flight between the dense combine, the column pass and the
+    # row pass: what stays in L2 (126 MB) beside the streams and the cube's
+    # writes
+    WORK_BYTES = 72 << 20
 
     @classmethod
     def _chunk_images(cls, N: int) -> int:
         return max(1, min(cls.WORK_BYTES // (N * (N // 2 + 1) * 8), 65535))
 
-    def _chunks(self, t_lo: int, *, all_times: bool):
-        """The cube's (fine DM, time) images in chunks of at most WORK_BYTES of
-        half spectra: (f0, n_f, t0, n_t, work [n_f, n_t, N, N/2+1]).  Dense
-        streams: every fine DM of a time range together (they read the same
-        stream times, which then stay in L2: 318 us a pass at 16 chgroups, 8
-        fine DMs x 64 times of 256^2, against 1103 us one fine DM at a time).
-        all_times, for compact streams: every time of some fine DMs (the
-        streams fit L2 whole, and the combine works in 64-time tiles)."""
+    def _chunks(self, t_lo: int, buf: torch.Tensor):
+        """The cube's (fine DM, time) images in chunks that fit ``buf``, every
+        fine DM of a time range together: (f0, n_f, t0, n_t, work [n_f, n_t,
+        N, N/2+1]).  With dense streams they read the same stream times, which
+        then stay in L2 (318 us a pass at 16 chgroups, 8 fine DMs x 64 times of
+        256^2, against 1103 us one fine DM at a time)."""
         cfg = self.config
         N, nh = cfg.n_grid, cfg.n_grid // 2 + 1
-        cap = self._chunk_images(N)
-        if all_times:
-            nt_c = min(cfg.t_det, cap)
-            nf_c = min(cfg.n_fdm, cap // nt_c)
-        else:
-            nf_c = min(cfg.n_fdm, cap)
-            nt_c = min(cfg.t_det, cap // nf_c)
-        buf = self.uv_slab.view(-1)
+        cap = min(buf.numel() // (N * nh), 65535)
+        nf_c = min(cfg.n_fdm, cap)
+        nt_c = min(cfg.t_det, cap // nf_c)
+        buf = buf.view(-1)
         for t0 in range(t_lo, cfg.t_det, nt_c):
             nt = min(nt_c, cfg.t_det - t0)
             for f0 in range(0, cfg.n_fdm, nf_c):
@@ -517,7 +512,14 @@ class GpuImager:
             self._csr = build_sparse_cell_csr(inv_lut, n_grid=N)
             self._csr_key = key
         st = _lib.status_word(self.device)
-        for f0, n_f, t0, nt, work in self._chunks(t_lo, all_times=True):
+        full = getattr(self, "_uv_full", None)
+        if full is None:
+            # every image at once: the combine stages each stream row once for
+            # all fine DMs and 64 times (0.60 ms a cube of 16 x 64 images of
+            # 256^2, against 0.85 ms in chunks of 48 MB)
+            full = self._uv_full = torch.empty((cfg.n_fdm * cfg.t_det, N, N // 2 + 1),
+                                               dtype=torch.complex64, device=self.device)
+        for f0, n_f, t0, nt, work in self._chunks(t_lo, full):
             work.zero_()
             _combine_sparse(streams, self._csr, shifts[f0:f0 + n_f], t_rows=t_stream,
                             t_out_len=nt, t_lo=t0, fftshift=True, out=work, out_row0=0, status=st)
