@@ -155,10 +155,22 @@ constexpr int TC_THREADS = 256;
 constexpr int TC_TMEM_COLS = 512;   // two accumulators of <= 256 columns
 constexpr int TC_SMEM_BUDGET = 224 * 1024;
 constexpr int TC_PRE = 4;          // 16-byte raw loads per thread per item (nant <= 128)
-constexpr int TC_CAP_ROWS = 4096;  // gridding rows of one (chgroup, subband) kept in smem
+// gridding rows of one (chgroup, subband) whose offsets are kept in smem: a
+// baseline meets about two cells over a chgroup's subbands, so four rows per
+// baseline, at most 12288 (24 KB).  Groups beyond it read their tables in
+// place, which costs a chain of global loads per row: with 4096 rows, too few
+// for some of the 512^2 patterns of 96 antennas, the gridding took 37 us of
+// every unit and set the kernel's time.
+__host__ __device__ constexpr int tc_cap_rows(int nant) {
+  const int n = 2 * nant * (nant + 1);
+  return n < 1024 ? 1024 : n > 12288 ? 12288 : n;
+}
 // Every CTA requests more than half an SM's shared memory so that exactly
 // one CTA (and one 512-column tensor-memory allocation) lives on each SM.
 constexpr int TC_MIN_SMEM = 120 * 1024;
+
+// Adjacent units whose outputs one 32-byte sector holds.
+constexpr int TC_QF = 4;
 
 struct TcArgs {
   const uint8_t* raw;
@@ -185,6 +197,13 @@ struct TcArgs {
   // antennas x csf channels x 4 bytes, arrive by one 4-D tensor copy into one
   // of nraw shared-memory stages of raw_stage bytes, nraw - 1 items ahead
   int tma, ppk, raw_stage, nraw;
+  // TMA form: tensor-memory columns of a CTA (two accumulators), CTAs per SM,
+  // unpacking threads, operand stages
+  int tmem_cols, ctas, unpackers, ws_nstage;
+  // mode 0: outputs of up to TC_QF consecutive units (adjacent elements in
+  // memory) staged in shared memory, [unit][baseline] of q_pitch, and written
+  // together; 0: each unit's straight from its accumulator
+  int q_pitch;
   int* status;
 };
 
@@ -233,13 +252,14 @@ struct TcFillPlan {
   int s_step;         // bytes between summed channels
 };
 
-DSB_DEV void tc_fill_plan(const TcArgs& A, TcFillPlan& P) {
+// thread: of the NT threads that share a chunk
+DSB_DEV void tc_fill_plan(const TcArgs& A, TcFillPlan& P, int thread, int NT) {
   const int nv = A.kc / 16;
   const uint32_t region = (uint32_t)A.rows * 128u;
   const long long pkt = (long long)A.nant * A.nchan * 4;
 #pragma unroll
   for (int r = 0; r < TC_PRE; ++r) {
-    const int idx = threadIdx.x + r * TC_THREADS;
+    const int idx = thread + r * NT;
     const int a = idx / nv, v = idx % nv;
     const int p = (v * 4) / A.csf, c = (v * 4) % A.csf;
     P.ld[r] = (int)(((long long)p * A.nant + a) * A.nchan * 4 + (long long)c * 4);
@@ -268,11 +288,11 @@ DSB_DEV void tc_load_planned(const TcArgs& A, const TcFillPlan& P, int g, int f,
 }
 
 DSB_DEV void tc_store_planned(const TcArgs& A, const TcFillPlan& P, uint8_t* st,
-                              const uint4 (&w)[TC_PRE]) {
+                              const uint4 (&w)[TC_PRE], int thread, int NT) {
   const int n = A.nant * (A.kc / 16);
 #pragma unroll
   for (int r = 0; r < TC_PRE; ++r) {
-    if (threadIdx.x + r * TC_THREADS < n) {
+    if (thread + r * NT < n) {
       uint4 R, I, N;
       R.x = nib_lo_s8x4(w[r].x); R.y = nib_lo_s8x4(w[r].y);
       R.z = nib_lo_s8x4(w[r].z); R.w = nib_lo_s8x4(w[r].w);
@@ -365,23 +385,25 @@ DSB_DEV void tc_fill(const TcArgs& A, uint8_t* st, int g, int f, int s, int q) {
 // other 16-column chunk (w >> 2 picks the parity).
 // Shared copies of the gridding CSR of the (chgroup, subband) last used.
 struct TcTab {
-  int* roff;        // (TC_CAP_ROWS + 1) row offsets relative to the group's first entry
-  uint16_t* bls;    // (nbase) baseline of each entry
   int* cached;      // group index whose tables are loaded (-1 none)
+  uint16_t* bls;    // (nbase) baseline of each entry
+  uint16_t* roff;   // (tc_cap_rows + 1) row offsets relative to the group's first entry
 };
 
-template <int MODE>
-DSB_DEV void tc_epilogue(const TcArgs& A, uint32_t tmem_base, int buf, int g, int f, int s,
-                         int2* vbuf, const TcTab& tab) {
+// NT threads (warps 0 .. NT / 32 - 1 of the CTA) take part; sync is their
+// barrier, done runs once the accumulator has been read.
+template <int MODE, int NT, typename Sync, typename Done>
+DSB_DEV void tc_epilogue(const TcArgs& A, uint32_t acc, int g, int f, int s, int2* vbuf,
+                         const TcTab& tab, Sync sync, Done done, int lu = 0, bool last = true) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int quarter = warp & 3, half = warp >> 2;
   const int nant = A.nant;
   const int b = quarter * 32 + lane;
   if (quarter * 32 < nant) {
-    const uint32_t lane_base =
-        tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * 256);
-    for (int c0 = half * 16; c0 < nant; c0 += 32) {
+    const uint32_t lane_base = acc + ((uint32_t)(quarter * 32) << 16);
+    for (int c0 = half * 16; c0 < nant; c0 += NT / 8) {
       if (c0 + 15 < quarter * 32) continue;  // whole chunk below this warp's rows
+      __syncwarp();
       uint32_t vr[16], vi[16];
       tmem_ld16(lane_base + (uint32_t)c0, vr);
       tmem_ld16(lane_base + (uint32_t)(nant + c0), vi);
@@ -394,6 +416,10 @@ DSB_DEV void tc_epilogue(const TcArgs& A, uint32_t tmem_base, int buf, int g, in
           const int bls = upper_bls(a, b);
           const int re = (int)vr[j], im = (int)vi[j];
           if constexpr (MODE == 0) {
+            if (A.q_pitch) {
+              vbuf[((A.unit_order ? s : f) & (TC_QF - 1)) * A.q_pitch + bls] = make_int2(re, im);
+              continue;
+            }
             A.out[(size_t)g * A.o_g + (size_t)f * A.o_f + (size_t)bls * A.o_b + (size_t)s * A.o_s] =
                 make_float2((float)re, (float)im);
           } else if (A.gains) {
@@ -415,6 +441,27 @@ DSB_DEV void tc_epilogue(const TcArgs& A, uint32_t tmem_base, int buf, int g, in
     }
   }
   tc_fence_before();
+  done();
+  if constexpr (MODE == 0) {
+    // the staged units 8 bytes each, four lanes to a baseline's sector, once
+    // the last of them (of their row, or of this CTA's) is in: 8-byte stores
+    // of one unit at a time kept L2 busy with quarter sectors (413 us for a
+    // native page, 175 us without any stores)
+    const int fast = A.unit_order ? s : f, j1 = fast & (TC_QF - 1);
+    last = last || fast == (A.unit_order ? A.ceff : A.n_fv) - 1;
+    if (A.q_pitch && (j1 == TC_QF - 1 || last)) {
+      sync();
+      const int j0 = max(0, j1 - lu), nbase = nant * (nant + 1) / 2;
+      float2* o = A.out + (size_t)g * A.o_g + (size_t)(A.unit_order ? f : s) *
+                                                   (A.unit_order ? A.o_f : A.o_s) + (fast - j1);
+      const int j = threadIdx.x & (TC_QF - 1);
+      if (j >= j0 && j <= j1)
+        for (int bls = threadIdx.x / TC_QF; bls < nbase; bls += NT / TC_QF) {
+          const int2 v = vbuf[j * A.q_pitch + bls];
+          o[(size_t)bls * A.o_b + j] = make_float2((float)v.x, (float)v.y);
+        }
+    }
+  }
   if constexpr (MODE == 1) {
     // per-cell sum over the baselines gridded into it (exact int32); the
     // group's CSR is copied to shared memory when the group changes (a CTA
@@ -424,13 +471,13 @@ DSB_DEV void tc_epilogue(const TcArgs& A, uint32_t tmem_base, int buf, int g, in
     const int cnt = A.ycnt[gs];
     const int e0 = A.row_off[row0];
     const int ne = A.row_off[row0 + cnt] - e0;
-    const bool use_tab = cnt <= TC_CAP_ROWS && ne <= A.nant * (A.nant + 1) / 2;
+    const bool use_tab = cnt <= tc_cap_rows(A.nant) && ne <= A.nant * (A.nant + 1) / 2;
     const bool reload = use_tab && *tab.cached != gs;
     if (reload) {
-      for (int k = threadIdx.x; k <= cnt; k += TC_THREADS) tab.roff[k] = A.row_off[row0 + k] - e0;
-      for (int j = threadIdx.x; j < ne; j += TC_THREADS) tab.bls[j] = (uint16_t)A.row_bls[e0 + j];
+      for (int k = threadIdx.x; k <= cnt; k += NT) tab.roff[k] = (uint16_t)(A.row_off[row0 + k] - e0);
+      for (int j = threadIdx.x; j < ne; j += NT) tab.bls[j] = (uint16_t)A.row_bls[e0 + j];
     }
-    __syncthreads();
+    sync();
     if (reload && threadIdx.x == 0) *tab.cached = gs;
     const long long tp = (A.t_base + f) & A.t_mask;
     float2* yrow = A.yout + tp * A.y_t_stride + row0;
@@ -440,7 +487,7 @@ DSB_DEV void tc_epilogue(const TcArgs& A, uint32_t tmem_base, int buf, int g, in
     if (A.gains) {
       // calibrated visibilities: float sums in CSR order
       const float2* fbuf = reinterpret_cast<const float2*>(vbuf);
-      for (int k = threadIdx.x; k < cnt; k += TC_THREADS) {
+      for (int k = threadIdx.x; k < cnt; k += NT) {
         const long long r = row0 + k;
         float sr = 0.f, si = 0.f;
         const int j0 = use_tab ? tab.roff[k] + e0 : A.row_off[r];
@@ -454,19 +501,39 @@ DSB_DEV void tc_epilogue(const TcArgs& A, uint32_t tmem_base, int buf, int g, in
         yrow[k] = make_float2(sr, si);
       }
     } else if (use_tab) {
-      for (int k = threadIdx.x; k < cnt; k += TC_THREADS) {
-        int sr = 0, si = 0;
-        const int j1 = tab.roff[k + 1];
-        for (int j = tab.roff[k]; j < j1; ++j) {
-          if (!DSB_INB(tab.bls[j], A.nant * (A.nant + 1) / 2, A.status)) continue;
-          const int2 v = vbuf[tab.bls[j]];
-          sr += v.x;
-          si += v.y;
+      // four rows at a time, first baselines first (most rows have one): the
+      // table and visibility loads of the four overlap
+      for (int k0 = threadIdx.x; k0 < cnt; k0 += 4 * NT) {
+        int j0[4], j1[4];
+        int2 v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int k = k0 + i * NT;
+          j0[i] = k < cnt ? (int)tab.roff[k] : 0;
+          j1[i] = k < cnt ? (int)tab.roff[k + 1] : 0;
         }
-        yrow[k] = make_float2((float)sr, (float)si);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          v[i] = make_int2(0, 0);
+          if (j0[i] < j1[i]) {
+            const int bl = tab.bls[j0[i]];
+            if (DSB_INB(bl, A.nant * (A.nant + 1) / 2, A.status)) v[i] = vbuf[bl];
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          for (int j = j0[i] + 1; j < j1[i]; ++j) {
+            if (!DSB_INB(tab.bls[j], A.nant * (A.nant + 1) / 2, A.status)) continue;
+            const int2 w = vbuf[tab.bls[j]];
+            v[i].x += w.x;
+            v[i].y += w.y;
+          }
+          const int k = k0 + i * NT;
+          if (k < cnt) yrow[k] = make_float2((float)v[i].x, (float)v[i].y);
+        }
       }
     } else {
-      for (int k = threadIdx.x; k < cnt; k += TC_THREADS) {
+      for (int k = threadIdx.x; k < cnt; k += NT) {
         const long long r = row0 + k;
         int sr = 0, si = 0;
         for (int j = A.row_off[r]; j < A.row_off[r + 1]; ++j) {
@@ -481,26 +548,23 @@ DSB_DEV void tc_epilogue(const TcArgs& A, uint32_t tmem_base, int buf, int g, in
   }
 }
 
-template <int MODE, bool TMA>
-__global__ void __launch_bounds__(TC_THREADS, 1)
-    corr_tc_kernel(const TcArgs A, const __grid_constant__ CUtensorMap tmap) {
+// The raw words loaded by the threads that unpack them (chunks that are not
+// whole packets of 16-byte channel runs).
+template <int MODE>
+__global__ void __launch_bounds__(TC_THREADS, 1) corr_tc_kernel(const TcArgs A) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* stages = smem;
-  // TMA: nraw raw stages after the operand stages (both 1024-byte multiples)
-  uint8_t* raw_st = stages + (size_t)A.nstage * A.stage_bytes;
-  uint64_t* bar_mma =
-      reinterpret_cast<uint64_t*>(raw_st + (TMA ? (size_t)A.nraw * A.raw_stage : 0));
+  uint64_t* bar_mma = reinterpret_cast<uint64_t*>(stages + (size_t)A.nstage * A.stage_bytes);
   uint64_t* bar_acc = bar_mma + A.nstage;
   uint64_t* bar_drain = bar_acc + 2;
-  uint64_t* bar_raw = bar_drain + 1;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_raw + (TMA ? A.nraw : 0));
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_drain + 1);
   int2* vbuf = reinterpret_cast<int2*>(tmem_slot + 4);
   TcTab tab{};
   if constexpr (MODE == 1) {
     tab.cached = reinterpret_cast<int*>(vbuf + A.nant * (A.nant + 1) / 2);
-    tab.roff = tab.cached + 4;
-    tab.bls = reinterpret_cast<uint16_t*>(tab.roff + TC_CAP_ROWS + 1);
+    tab.bls = reinterpret_cast<uint16_t*>(tab.cached + 4);
+    tab.roff = tab.bls + A.nant * (A.nant + 1) / 2;
   }
 
   const int tid = threadIdx.x, warp = tid >> 5;
@@ -514,8 +578,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     mbar_init(&bar_acc[0], 1);
     mbar_init(&bar_acc[1], 1);
     mbar_init(bar_drain, 1);
-    if constexpr (TMA)
-      for (int i = 0; i < A.nraw; ++i) mbar_init(&bar_raw[i], 1);
     fence_mbar_init();
   }
   tc_fence_before();
@@ -534,27 +596,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   const bool vec = (A.csf & 3) == 0 && (A.nchan & 3) == 0;
   const bool planned = vec && ((A.kc / 4) % A.csf) == 0;
   TcFillPlan plan{};
-  if (planned) tc_fill_plan(A, plan);
+  if (planned) tc_fill_plan(A, plan, tid, TC_THREADS);
   bool ok = true;
-  // TMA: item `item`'s raw bytes (ppk packets x nant x csf channels x 4 bytes
-  // of one chgroup page) into raw stage item % nraw, by thread 0
-  int issued = 0, it_stop = n_items;
-  auto issue_raw = [&](int item) {
-    const int lu = item / A.n_chunks, q = item % A.n_chunks;
-    int g, f, s;
-    tc_unit_coords(A, u_begin + lu, g, f, s);
-    const int r = item % A.nraw;
-    mbar_arrive_expect_tx(&bar_raw[r], (uint32_t)(A.ppk * A.nant * A.csf * 4));
-    tma_load_4d(raw_st + (size_t)r * A.raw_stage, &tmap, s * A.csf * 4, 0,
-                f * A.ppfv + q * A.ppk, g, &bar_raw[r]);
-  };
-  if constexpr (TMA) {
-    if (tid == 0)
-      for (; issued < A.nraw - 1 && issued < n_items; ++issued) issue_raw(issued);
-  }
   // the raw words of the next item are loaded while this one is unpacked
   uint4 pre[TC_PRE];
-  if (!TMA && vec && n_items > 0) {
+  if (vec && n_items > 0) {
     int g0, f0, s0;
     tc_unit_coords(A, u_begin, g0, f0, s0);
     if (planned) tc_load_planned(A, plan, g0, f0, s0, 0, pre);
@@ -569,22 +615,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     const int slot = it % A.nstage;
     bool w_ok = true;
     if (it >= A.nstage) w_ok = mbar_wait(&bar_mma[slot], (uint32_t)((it / A.nstage - 1) & 1));
-    if constexpr (TMA)
-      w_ok = w_ok && mbar_wait(&bar_raw[it % A.nraw], (uint32_t)((it / A.nraw) & 1));
-    if (!__syncthreads_and(w_ok)) { ok = false; it_stop = it; break; }
+    if (!__syncthreads_and(w_ok)) { ok = false; break; }
     uint8_t* st = stages + (size_t)slot * A.stage_bytes;
-    if constexpr (TMA) {
-      // every thread is done with item it - 1: its raw stage takes item
-      // it + nraw - 1
-      if (tid == 0 && issued < n_items) issue_raw(issued++);
-      const uint8_t* rs = raw_st + (size_t)(it % A.nraw) * A.raw_stage;
-      const int n_w = A.nant * (A.kc / 16);
-      uint4 cur[TC_PRE];
-#pragma unroll
-      for (int r = 0; r < TC_PRE; ++r)
-        if (tid + r * TC_THREADS < n_w) cur[r] = *reinterpret_cast<const uint4*>(rs + plan.lds[r]);
-      tc_store_planned(A, plan, st, cur);
-    } else if (vec) {
+    if (vec) {
       uint4 cur[TC_PRE];
 #pragma unroll
       for (int r = 0; r < TC_PRE; ++r) cur[r] = pre[r];
@@ -595,7 +628,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         if (planned) tc_load_planned(A, plan, ng, nf, ns, nq, pre);
         else tc_load(A, ng, nf, ns, nq, pre);
       }
-      if (planned) tc_store_planned(A, plan, st, cur);
+      if (planned) tc_store_planned(A, plan, st, cur, tid, TC_THREADS);
       else tc_store(A, st, cur);
     } else {
       tc_fill(A, st, g, f, s, q);
@@ -617,11 +650,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     if (q == A.n_chunks - 1 && lu >= 1) {
       const int pl = lu - 1;
       const bool a_ok = mbar_wait(&bar_acc[pl & 1], (uint32_t)((pl >> 1) & 1));
-      if (!__syncthreads_and(a_ok)) { ok = false; it_stop = it; break; }
+      if (!__syncthreads_and(a_ok)) { ok = false; break; }
       tc_fence_after();
       int pg, pf, ps;
       tc_unit_coords(A, u_begin + pl, pg, pf, ps);
-      tc_epilogue<MODE>(A, tmem_base, pl & 1, pg, pf, ps, vbuf, tab);
+      tc_epilogue<MODE, TC_THREADS>(A, tmem_base + (uint32_t)((pl & 1) * 256), pg, pf, ps, vbuf,
+                                    tab, [] { __syncthreads(); }, [] {});
     }
   }
   if (ok && my_units > 0) {
@@ -631,21 +665,18 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
       tc_fence_after();
       int pg, pf, ps;
       tc_unit_coords(A, u_begin + pl, pg, pf, ps);
-      tc_epilogue<MODE>(A, tmem_base, pl & 1, pg, pf, ps, vbuf, tab);
+      tc_epilogue<MODE, TC_THREADS>(A, tmem_base + (uint32_t)((pl & 1) * 256), pg, pf, ps, vbuf,
+                                    tab, [] { __syncthreads(); }, [] {});
     } else {
       ok = false;
     }
   }
   if (!ok) {
     if (tid == 0) dsb_flag(A.status, DSB_E_TIMEOUT);
-    // Drain every MMA this CTA issued before releasing tensor memory, and
-    // every tensor copy still writing into its shared memory.
+    // drain every MMA this CTA issued before releasing tensor memory
     if (tid == 0) {
       umma_commit(bar_drain);
       mbar_wait(bar_drain, 0u);
-      if constexpr (TMA)
-        for (int i = it_stop; i < issued; ++i)
-          mbar_wait(&bar_raw[i % A.nraw], (uint32_t)((i / A.nraw) & 1));
     }
   }
   tc_fence_before();
@@ -653,6 +684,195 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   if (warp == 0) {
     tc_fence_after();
     tmem_dealloc(tmem_base, TC_TMEM_COLS);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// The same correlator with the raw tiles staged by TMA and a role per warp:
+// the first warps write out (or grid) the finished unit, the next ones unpack
+// raw stages into operand stages, one thread issues the tensor copies and one
+// the products; stages pass between them by mbarriers.
+//
+// What bounds it: shared memory (per 128 samples of 96 antennas 12 KB of raw
+// bytes in, 49 KB of operands out, 81 KB read by the products) and the
+// products themselves, 0.6 us each per SM.  One role after the other between
+// CTA barriers, with the gridding's tables read in place, took 11.0 ms for 16
+// native pages gridded into 512^2 patterns and 445 us for one page; this takes
+// 4.1 ms and 288 us (2.7 ms and 175 us without the writing).
+//
+// Where two accumulators need fewer than 512 columns, the CTA takes only
+// those (a power of two) and several CTAs share an SM (TcArgs.ctas): a unit
+// of a small array is a single chunk whose latency one CTA cannot hide (16
+// antennas, 64 samples per unit: 3.7 us per unit with one CTA per SM).
+// ---------------------------------------------------------------------------
+// NU unpacking threads (TC_PRE words each): 256, or 64 where a chunk is at
+// most 256 words; the threads that write out; and the CTAs of that size an
+// SM's registers hold.  (Two or four groups of unpacking threads that take the
+// chunks in turn were slower: 4.1 -> 4.5 ms gridded, 288 -> 316 us a page.)
+template <int NU>
+struct WsCfg {
+  static constexpr int EPI = NU == 64 ? 128 : 256;
+  static constexpr int THREADS = EPI + NU + 64;
+  static constexpr int CTAS = NU == 64 ? 4 : 1;
+};
+
+template <int MODE, int NU>
+__global__ void __launch_bounds__(WsCfg<NU>::THREADS, WsCfg<NU>::CTAS) corr_ws_kernel(
+    const TcArgs A, const __grid_constant__ CUtensorMap tmap) {
+  constexpr int EPI = WsCfg<NU>::EPI;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* stages = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint8_t* raw_st = stages + (size_t)A.nstage * A.stage_bytes;
+  uint64_t* bar_full = reinterpret_cast<uint64_t*>(raw_st + (size_t)A.nraw * A.raw_stage);
+  uint64_t* bar_free = bar_full + A.nstage;
+  uint64_t* bar_raw = bar_free + A.nstage;
+  uint64_t* bar_rawfree = bar_raw + A.nraw;
+  uint64_t* bar_acc = bar_rawfree + A.nraw;   // [2] accumulator finished
+  uint64_t* bar_out = bar_acc + 2;            // [2] accumulator read
+  uint64_t* bar_drain = bar_out + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_drain + 1);
+  int2* vbuf = reinterpret_cast<int2*>(tmem_slot + 4);
+  TcTab tab{};
+  if constexpr (MODE == 1) {
+    tab.cached = reinterpret_cast<int*>(vbuf + A.nant * (A.nant + 1) / 2);
+    tab.bls = reinterpret_cast<uint16_t*>(tab.cached + 4);
+    tab.roff = tab.bls + A.nant * (A.nant + 1) / 2;
+  }
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (warp == 0) {
+    tmem_alloc(tmem_slot, (uint32_t)A.tmem_cols);
+    tmem_relinquish();
+  }
+  if (tid == 0) {
+    if constexpr (MODE == 1) *tab.cached = -1;
+    for (int i = 0; i < A.nstage; ++i) {
+      mbar_init(&bar_full[i], NU);
+      mbar_init(&bar_free[i], 1);
+    }
+    for (int i = 0; i < A.nraw; ++i) {
+      mbar_init(&bar_raw[i], 1);
+      mbar_init(&bar_rawfree[i], NU);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&bar_acc[i], 1);
+      mbar_init(&bar_out[i], EPI);
+    }
+    mbar_init(bar_drain, 1);
+    fence_mbar_init();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t acc_cols = (uint32_t)A.tmem_cols / 2;
+  // each CTA walks a contiguous range of units (consecutive fast-vis tiles
+  // of one (chgroup, subband) share the gridding tables)
+  const int n_units = A.n_chgroup * A.n_fv * A.ceff;
+  const int per_cta = (n_units + (int)gridDim.x - 1) / (int)gridDim.x;
+  const int u_begin = (int)blockIdx.x * per_cta;
+  const int my_units = max(0, min(per_cta, n_units - u_begin));
+  const int n_items = my_units * A.n_chunks;
+  bool ok = true;
+
+  if (warp < EPI / 32) {
+    for (int lu = 0; lu < my_units; ++lu) {
+      const int buf = lu & 1;
+      ok = mbar_wait(&bar_acc[buf], (uint32_t)((lu >> 1) & 1));
+      // (named barrier: the warps agree, and the previous unit's reads
+      // of vbuf are done before it is written again)
+      int all;
+      asm volatile(
+          "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\t"
+          "barrier.cta.red.and.pred q, 1, %2, p;\n\tselp.b32 %0, 1, 0, q;\n\t}"
+          : "=r"(all)
+          : "r"((int)ok), "n"(EPI)
+          : "memory");
+      ok = all != 0;
+      if (!ok) break;
+      tc_fence_after();
+      int g, f, s;
+      tc_unit_coords(A, u_begin + lu, g, f, s);
+      tc_epilogue<MODE, EPI>(
+          A, tmem_base + (uint32_t)buf * acc_cols, g, f, s, vbuf, tab,
+          [] { asm volatile("barrier.cta.sync 1, %0;" ::"n"(EPI) : "memory"); },
+          [&] { mbar_arrive(&bar_out[buf]); }, lu, lu == my_units - 1);
+    }
+  } else if (warp < (EPI + NU) / 32) {
+    const int ut = tid - EPI;
+    TcFillPlan plan;
+    tc_fill_plan(A, plan, ut, NU);
+    const int n_w = A.nant * (A.kc / 16);
+    for (int it = 0; it < n_items; ++it) {
+      const int slot = it % A.nstage, r = it % A.nraw;
+      if (it >= A.nstage) ok = mbar_wait(&bar_free[slot], (uint32_t)((it / A.nstage - 1) & 1));
+      ok = ok && mbar_wait(&bar_raw[r], (uint32_t)((it / A.nraw) & 1));
+      if (!__all_sync(0xffffffffu, ok)) {
+        ok = false;
+        break;
+      }
+      const uint8_t* rs = raw_st + (size_t)r * A.raw_stage;
+      uint4 cur[TC_PRE];
+#pragma unroll
+      for (int k = 0; k < TC_PRE; ++k)
+        if (ut + k * NU < n_w) cur[k] = *reinterpret_cast<const uint4*>(rs + plan.lds[k]);
+      tc_store_planned(A, plan, stages + (size_t)slot * A.stage_bytes, cur, ut, NU);
+      fence_proxy_async_smem();
+      mbar_arrive(&bar_full[slot]);
+      mbar_arrive(&bar_rawfree[r]);
+    }
+  } else if (warp == (EPI + NU) / 32) {
+    if (lane == 0) {
+      // item's raw bytes: ppk packets x nant x csf channels x 4 bytes of one
+      // chgroup page
+      int issued = 0;
+      for (int it = 0; it < n_items; ++it) {
+        const int r = it % A.nraw;
+        if (it >= A.nraw) ok = mbar_wait(&bar_rawfree[r], (uint32_t)((it / A.nraw - 1) & 1));
+        if (!ok) break;
+        const int lu = it / A.n_chunks, q = it % A.n_chunks;
+        int g, f, s;
+        tc_unit_coords(A, u_begin + lu, g, f, s);
+        mbar_arrive_expect_tx(&bar_raw[r], (uint32_t)(A.ppk * A.nant * A.csf * 4));
+        tma_load_4d(raw_st + (size_t)r * A.raw_stage, &tmap, s * A.csf * 4, 0,
+                    f * A.ppfv + q * A.ppk, g, &bar_raw[r]);
+        ++issued;
+      }
+      // no copy may be in flight into this CTA's shared memory when it ends
+      // (each of the last nraw copies' phases; all earlier ones were waited
+      // for before their stage was taken again)
+      for (int it = max(0, issued - A.nraw); it < issued; ++it)
+        mbar_wait(&bar_raw[it % A.nraw], (uint32_t)((it / A.nraw) & 1));
+    }
+  } else if (lane == 0) {
+    const uint32_t idesc = idesc_i8(128u, (uint32_t)(2 * A.nant));
+    for (int it = 0; it < n_items; ++it) {
+      const int lu = it / A.n_chunks, q = it % A.n_chunks;
+      const int slot = it % A.nstage, buf = lu & 1;
+      if (q == 0 && lu >= 2) ok = mbar_wait(&bar_out[buf], (uint32_t)(((lu >> 1) - 1) & 1));
+      ok = ok && mbar_wait(&bar_full[slot], (uint32_t)((it / A.nstage) & 1));
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t d = tmem_base + (uint32_t)buf * acc_cols;
+      const uint32_t sbase = smem_u32(stages + (size_t)slot * A.stage_bytes);
+      for (int m = 0; m < A.n_mma; ++m) {
+        const uint32_t kb = (uint32_t)m * 32u;
+        const uint64_t desc = sdesc_k_sw128(sbase + (kb >> 7) * (uint32_t)A.rows * 128u + (kb & 127u));
+        umma_i8_ss(d, desc, desc, idesc, (q > 0 || m > 0) ? 1u : 0u);
+      }
+      umma_commit(&bar_free[slot]);
+      if (q == A.n_chunks - 1) umma_commit(&bar_acc[buf]);
+    }
+    // every product issued here ends before tensor memory is given back
+    umma_commit(bar_drain);
+    mbar_wait(bar_drain, 0u);
+  }
+  if (!ok) dsb_flag(A.status, DSB_E_TIMEOUT);
+  __syncwarp();
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, (uint32_t)A.tmem_cols);
   }
 }
 
@@ -1160,12 +1380,12 @@ int launch_status() {
   return e == cudaSuccess ? DSB_OK : DSB_E_CUDA;
 }
 
-// Shared memory beyond the operand stages: mode 1 keeps the upper-triangle
+// Shared memory beyond the operand stages: mode 0 the staged outputs, mode 1 the upper-triangle
 // visibilities of one unit (int2) and the gridding tables of one group.
 int tc_extra_bytes(const TcArgs& A, int mode) {
-  if (mode != 1) return 0;
+  if (mode != 1) return A.q_pitch * TC_QF * 8;
   const int nbase = A.nant * (A.nant + 1) / 2;
-  return nbase * 8 + 16 + (TC_CAP_ROWS + 1) * 4 + nbase * 2 + 16;
+  return nbase * 8 + 16 + nbase * 2 + (tc_cap_rows(A.nant) + 1) * 2 + 16;
 }
 
 // Fill the derived geometry; returns DSB_OK or an error code.
@@ -1189,20 +1409,59 @@ int tc_plan(TcArgs& A, int mode) {
   const int budget = TC_SMEM_BUDGET - extra - 1024 - 256;
   A.nstage = std::min(4, budget / A.stage_bytes);
   if (A.nstage < 2) return DSB_E_UNSUPPORTED;
-  // raw staging by TMA when a chunk is whole packets of 16-byte channel runs
-  // and four raw stages still leave two operand stages
   A.tma = 0;
-  if ((A.csf % 4) == 0 && (A.nchan % 4) == 0 && ((A.kc / 4) % A.csf) == 0 && A.nant <= 256) {
-    A.ppk = (A.kc / 4) / A.csf;
-    A.raw_stage = (A.ppk * A.nant * A.csf * 4 + 1023) & ~1023;
-    A.nraw = 4;
-    const int ns = std::min(4, (budget - A.nraw * A.raw_stage) / A.stage_bytes);
-    if (ns >= 2) {
-      A.tma = 1;
-      A.nstage = ns;
-    }
-  }
+  A.q_pitch = 0;
   return DSB_OK;
+}
+
+// Plan corr_ws_kernel (A.tma) when a chunk of kc samples is whole packets of
+// 16-byte channel runs and four raw stages leave two operand stages: as many
+// CTAs per SM as tensor memory, registers and shared memory hold.  q_pitch:
+// the staged outputs' pitch (0: none).
+bool ws_plan(TcArgs& A, int mode, int kc, int q_pitch) {
+  const int kprime = 2 * A.t_int * A.csf;
+  if (kc <= 0 || kc > kprime || kprime % kc || kc % 16 || (A.csf % 4) || (A.nchan % 4) ||
+      ((kc / 4) % A.csf))
+    return false;
+  TcArgs P = A;
+  P.kc = kc;
+  P.n_chunks = kprime / kc;
+  P.nkblk = (2 * kc + 127) / 128;
+  P.stage_bytes = P.nkblk * P.rows * 128;
+  P.n_mma = 2 * kc / 32;
+  P.q_pitch = q_pitch;
+  P.ppk = (kc / 4) / P.csf;
+  P.raw_stage = (P.ppk * P.nant * P.csf * 4 + 1023) & ~1023;
+  P.nraw = 4;
+  P.unpackers = P.nant * (kc / 16) <= 64 * TC_PRE ? 64 : 256;
+  P.tmem_cols = 32;
+  while (P.tmem_cols < 4 * P.nant) P.tmem_cols *= 2;
+  for (P.ctas = std::min(P.unpackers == 64 ? WsCfg<64>::CTAS : WsCfg<256>::CTAS,
+                         TC_TMEM_COLS / P.tmem_cols);
+       P.ctas >= 1; --P.ctas) {
+    const int room = std::min(TC_SMEM_BUDGET, 228 * 1024 / P.ctas - 1024) -
+                     tc_extra_bytes(P, mode) - 1024 - 256;
+    const int ns = std::min(4, (room - P.nraw * P.raw_stage) / P.stage_bytes);
+    if (ns < 2) continue;
+    P.tma = 1;
+    P.ws_nstage = ns;
+    A = P;
+    return true;
+  }
+  return false;
+}
+
+// The TMA form's plan, if it has one: mode 0 with outputs of adjacent units
+// staged where they are adjacent in memory (with 96 antennas that takes
+// chunks of 64 samples instead of 128).
+void ws_choose(TcArgs& A, int mode) {
+  const int nbase = A.nant * (A.nant + 1) / 2;
+  // pitch = 4 mod 16 eight-byte words: four units' reads in different banks
+  const int pitch = (nbase + 15) / 16 * 16 + 4;
+  if (mode == 0 && (A.unit_order ? A.o_s : A.o_f) == 1 &&
+      (ws_plan(A, mode, A.kc, pitch) || ws_plan(A, mode, 64, pitch)))
+    return;
+  ws_plan(A, mode, A.kc, 0);
 }
 
 // The driver's tensor-map encoder, looked up once through the runtime.
@@ -1242,24 +1501,35 @@ bool tc_raw_tmap(const TcArgs& A, CUtensorMap* m) {
             CU_TENSOR_MAP_L2_PROMOTION_L2_64B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Launch corr_tc_kernel<MODE, TMA> on the planned geometry.
+// Launch on the planned geometry: n_units units over at most max_ctas CTAs
+// (0: what the device holds).
 template <int MODE>
-int tc_launch(TcArgs& A, int grid, cudaStream_t stream) {
+int tc_launch(TcArgs& A, int n_units, int max_ctas, cudaStream_t stream) {
   CUtensorMap tmap;
   memset(&tmap, 0, sizeof(tmap));
-  if (A.tma && !tc_raw_tmap(A, &tmap)) A.tma = 0;
-  const int raw = A.tma ? A.nraw * A.raw_stage : 0;
-  const int smem = std::max(A.nstage * A.stage_bytes + raw + 1024 + 256 + tc_extra_bytes(A, MODE),
-                            TC_MIN_SMEM);
+  const TcArgs plain = A;
+  ws_choose(A, MODE);
+  if (A.tma && !tc_raw_tmap(A, &tmap)) A = plain;
   if (A.tma) {
-    cudaFuncSetAttribute(corr_tc_kernel<MODE, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         smem);
-    corr_tc_kernel<MODE, true><<<grid, TC_THREADS, smem, stream>>>(A, tmap);
-  } else {
-    cudaFuncSetAttribute(corr_tc_kernel<MODE, false>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    corr_tc_kernel<MODE, false><<<grid, TC_THREADS, smem, stream>>>(A, tmap);
+    A.nstage = A.ws_nstage;
+    // at least what keeps more than `ctas` CTAs (and their tensor memory) off an SM
+    const int smem = std::max(A.nstage * A.stage_bytes + A.nraw * A.raw_stage + 1024 + 256 +
+                                  tc_extra_bytes(A, MODE),
+                              228 * 1024 / (A.ctas + 1));
+    const int grid = std::min(n_units, max_ctas > 0 ? max_ctas : A.ctas * num_sms());
+    auto go = [&](auto kern, int threads) {
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+      kern<<<grid, threads, smem, stream>>>(A, tmap);
+      return launch_status();
+    };
+    return A.unpackers == 64 ? go(corr_ws_kernel<MODE, 64>, WsCfg<64>::THREADS)
+                             : go(corr_ws_kernel<MODE, 256>, WsCfg<256>::THREADS);
   }
+  const int smem = std::max(A.nstage * A.stage_bytes + 1024 + 256 + tc_extra_bytes(A, MODE),
+                            TC_MIN_SMEM);
+  cudaFuncSetAttribute(corr_tc_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  corr_tc_kernel<MODE><<<std::min(n_units, max_ctas > 0 ? max_ctas : num_sms()), TC_THREADS, smem,
+                         stream>>>(A);
   return launch_status();
 }
 
@@ -1387,7 +1657,7 @@ int dsb_corr_tc(const void* raw, long long raw_g_stride, int n_chgroup, int npkt
   int rc = tc_plan(A, 0);
   if (rc) return rc;
   const int n_units = n_chgroup * A.n_fv * A.ceff;
-  return tc_launch<0>(A, std::min(n_units, max_ctas > 0 ? max_ctas : num_sms()), stream);
+  return tc_launch<0>(A, n_units, max_ctas, stream);
 }
 
 int dsb_corr_tc_grid(const void* raw, long long raw_g_stride, int n_chgroup, int npkt, int nant,
@@ -1410,7 +1680,7 @@ int dsb_corr_tc_grid(const void* raw, long long raw_g_stride, int n_chgroup, int
   int rc = tc_plan(A, 1);
   if (rc) return rc;
   const int n_units = n_chgroup * A.n_fv * A.ceff;
-  return tc_launch<1>(A, std::min(n_units, max_ctas > 0 ? max_ctas : num_sms()), stream);
+  return tc_launch<1>(A, n_units, max_ctas, stream);
 }
 
 }  // extern "C"
