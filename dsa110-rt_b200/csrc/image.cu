@@ -274,8 +274,12 @@ constexpr int IMG_MAX_G = 64;
 //  * N = 512: FOLD 8 (64-row passes), 512 threads, one CTA per SM with all
 //    512 TMEM columns, 32-bit entry metadata (8 bits of column); the combine's
 //    S arrays (int32 real and imaginary parts) take 192 KB of shared memory.
-//  * N = 64, 256: FOLD 4, 256 threads, three CTAs per SM with 128 TMEM
-//    columns each, 16-bit entry metadata.
+//  * N = 256: FOLD 4, 256 threads, three CTAs per SM with 128 TMEM columns
+//    each, 16-bit entry metadata.
+//  * N = 64: the same with 64 threads and up to 16 CTAs per SM of 32 columns
+//    each.  An image is a chain of short steps (a few hundred S entries, 12
+//    barriers), so the images in flight decide the rate: with 256 threads and
+//    three CTAs per SM 16,896 images took 389 us, now 231.
 // TMEM: warps w, w + 4, w + 8, ... reach the same 32 lanes; each takes an
 // equal share of the CTA's columns, two 32-bit columns per complex S entry.
 template <int N>
@@ -287,10 +291,11 @@ struct ImgGeom {
   static constexpr int P = NC + 2;                // buffer row pitch (float2), = 2 mod 16
   static constexpr int R1 = (N == 64) ? 8 : 16;   // threads per row transform
   static constexpr int R2 = N / R1;               // points per thread
-  static constexpr int THREADS = (N == 512) ? 512 : 256;
-  static constexpr int CTAS = (N == 512) ? 1 : 3; // resident CTAs per SM
-  static constexpr int TMEM_COLS = (N == 512) ? 512 : 128;
-  static constexpr int WARP_COLS = TMEM_COLS / (THREADS / 128);  // columns per warp
+  static constexpr int THREADS = (N == 512) ? 512 : (N == 256) ? 256 : 64;
+  static constexpr int CTAS = (N == 512) ? 1 : (N == 256) ? 3 : 16; // resident CTAs per SM
+  static constexpr int TMEM_COLS = (N == 512) ? 512 : (N == 256) ? 128 : 32;
+  // columns per warp (warps 4 apart share lanes)
+  static constexpr int WARP_COLS = TMEM_COLS / (THREADS > 128 ? THREADS / 128 : 1);
   static constexpr int MAXE = WARP_COLS / 2;      // S entries per thread
   static constexpr bool META32 = (N == 512);
   // entry metadata fields: column | n' << NP_SH | q << Q_SH | last << LAST_SH
