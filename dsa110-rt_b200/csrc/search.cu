@@ -686,31 +686,31 @@ __global__ void padded_cumsum_kernel(const T* __restrict__ x, int n, long long i
 // is the L1 rate of its 2 K loads per output (then memory: every prefix read
 // and 6 to 8 bytes written once).  One output per thread, with two 64-bit
 // divisions and 2 K 4-byte loads from L2 each, took 309 us for 128 outputs of
-// 4 x 256^2 cells at boxcars 1..16; this takes 107 us.
+// 4 x 256^2 cells at boxcars 1..16; this takes 95 us (tiles of 4, 16, 32 and 64
+// times: 100, 108, 123, 120).
 //
 // CHECK: every prefix row read must lie in [0, cs_rows); an output whose
 // widths / offsets would read outside gets S/N NaN and winner -1 instead
 // (the rows outside belong to no call's data: the shared scratch array of
 // dsb_boxcar_argmax_noalloc).
-constexpr int BA_THREADS = 128, BA_T = 16, BA_MAX_K = 32;
+constexpr int BA_THREADS = 128, BA_T = 8, BA_MAX_K = 32;
 
 template <int V, bool OUT_F16, bool CHECK>
 __global__ void __launch_bounds__(BA_THREADS) multi_boxcar_argmax_kernel(
     const float* __restrict__ cs, long long inner, const int* __restrict__ widths,
     const int* __restrict__ offsets, const float* __restrict__ sinv, int K, int n_out, int t_base,
     void* __restrict__ out_max, int16_t* __restrict__ out_win, long long cs_rows, int n_tt) {
-  __shared__ int s_lo[BA_MAX_K], s_w[BA_MAX_K];
+  // each width's first and last row relative to the output's, as offsets into
+  // cs, and its scale
+  __shared__ longlong2 s_off[BA_MAX_K];
   __shared__ float s_si[BA_MAX_K];
   const bool tab = K <= BA_MAX_K;   // longer lists are read in place
   if (tab && (int)threadIdx.x < K) {
-    s_lo[threadIdx.x] = offsets[threadIdx.x];
-    s_w[threadIdx.x] = widths[threadIdx.x];
+    const long long lo = offsets[threadIdx.x];
+    s_off[threadIdx.x] = make_longlong2(lo * inner, (lo + widths[threadIdx.x]) * inner);
     s_si[threadIdx.x] = sinv[threadIdx.x];
   }
   __syncthreads();
-  const int* lo_p = tab ? s_lo : offsets;
-  const int* w_p = tab ? s_w : widths;
-  const float* si_p = tab ? s_si : sinv;
   // time tiles fastest: the CTAs that run together share rows in L2
   const long long e = ((long long)(blockIdx.x / n_tt) * BA_THREADS + threadIdx.x) * V;
   const int t0 = (int)(blockIdx.x % n_tt) * BA_T, t1 = min(n_out, t0 + BA_T);
@@ -718,6 +718,7 @@ __global__ void __launch_bounds__(BA_THREADS) multi_boxcar_argmax_kernel(
   using VT = typename std::conditional<V == 4, float4, float>::type;
   for (int t = t0; t < t1; ++t) {
     const long long ta = (long long)t + t_base;
+    const float* row = cs + ta * inner + e;
     float best[V];
     int win[V];
 #pragma unroll
@@ -727,20 +728,25 @@ __global__ void __launch_bounds__(BA_THREADS) multi_boxcar_argmax_kernel(
     }
 #pragma unroll 4
     for (int k = 0; k < K; ++k) {
-      const long long lo = ta + lo_p[k], hi = lo + w_p[k];
-      if (CHECK && (lo < 0 || hi < 0 || lo >= cs_rows || hi >= cs_rows)) {
+      if constexpr (CHECK) {
+        const long long lo = ta + offsets[k], hi = lo + widths[k];
+        if (lo < 0 || hi < 0 || lo >= cs_rows || hi >= cs_rows) {
 #pragma unroll
-        for (int v = 0; v < V; ++v) {
-          best[v] = __int_as_float(0x7fc00000);
-          win[v] = -1;
+          for (int v = 0; v < V; ++v) {
+            best[v] = __int_as_float(0x7fc00000);
+            win[v] = -1;
+          }
+          break;
         }
-        break;
       }
-      const VT h4 = *reinterpret_cast<const VT*>(cs + hi * inner + e);
-      const VT l4 = *reinterpret_cast<const VT*>(cs + lo * inner + e);
+      const longlong2 o = tab ? s_off[k]
+                              : make_longlong2(offsets[k] * inner,
+                                               ((long long)offsets[k] + widths[k]) * inner);
+      const VT h4 = *reinterpret_cast<const VT*>(row + o.y);
+      const VT l4 = *reinterpret_cast<const VT*>(row + o.x);
       const float* h = reinterpret_cast<const float*>(&h4);
       const float* l = reinterpret_cast<const float*>(&l4);
-      const float si = si_p[k];
+      const float si = tab ? s_si[k] : sinv[k];
 #pragma unroll
       for (int v = 0; v < V; ++v) {
         const float s = (h[v] - l[v]) * si;
