@@ -501,19 +501,21 @@ DSB_DEV void tc_epilogue(const TcArgs& A, uint32_t acc, int g, int f, int s, int
         yrow[k] = make_float2(sr, si);
       }
     } else if (use_tab) {
-      // four rows at a time, first baselines first (most rows have one): the
-      // table and visibility loads of the four overlap
-      for (int k0 = threadIdx.x; k0 < cnt; k0 += 4 * NT) {
-        int j0[4], j1[4];
-        int2 v[4];
+      // RW rows at a time, first baselines first (most rows have one): their
+      // table and visibility loads overlap (one at a time where a small array
+      // has few rows per thread)
+      constexpr int RW = NT == 128 ? 1 : 4;
+      for (int k0 = threadIdx.x; k0 < cnt; k0 += RW * NT) {
+        int j0[RW], j1[RW];
+        int2 v[RW];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < RW; ++i) {
           const int k = k0 + i * NT;
           j0[i] = k < cnt ? (int)tab.roff[k] : 0;
           j1[i] = k < cnt ? (int)tab.roff[k + 1] : 0;
         }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < RW; ++i) {
           v[i] = make_int2(0, 0);
           if (j0[i] < j1[i]) {
             const int bl = tab.bls[j0[i]];
@@ -521,7 +523,7 @@ DSB_DEV void tc_epilogue(const TcArgs& A, uint32_t acc, int g, int f, int s, int
           }
         }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < RW; ++i) {
           for (int j = j0[i] + 1; j < j1[i]; ++j) {
             if (!DSB_INB(tab.bls[j], A.nant * (A.nant + 1) / 2, A.status)) continue;
             const int2 w = vbuf[tab.bls[j]];
@@ -889,6 +891,7 @@ struct SplitTcArgs {
   int off_re, off_im;
   int nchan, npkt, nant, nant_p, ppfv, fuse, csf, ceff;
   int n_fv, n_units, kprime, n_chunks, rows, nstage, stage_bytes;
+  int q_pitch;               // staged outputs' pitch (0: none), as in TcArgs
   float2* out;
   int* status;
 };
@@ -1167,6 +1170,85 @@ DSB_DEV uint4 mn_shift(size_t o, const uint32_t (&w)[2 * ESZ + 1]) {
   return make_uint4(a.x, a.y, b.x, b.y);
 }
 
+// The writing warps (the CTA's first NT threads): accumulator lane b, columns
+// a (Re), 128 + a (Im); the upper triangle b <= a goes to bls(a, b).  With
+// staged outputs (A.q_pitch) those of up to TC_QF adjacent units leave
+// together, four lanes to a baseline's 32-byte sector.  False if a wait ran
+// out.
+template <int NT>
+DSB_DEV bool mn_write_units(const SplitTcArgs& A, uint32_t tmem_base, int u_begin, int my_units,
+                            uint64_t* bar_acc, uint64_t* bar_out, float2* vbuf) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int quarter = warp & 3, part = warp >> 2;
+  const int nant = A.nant, nbase = nant * (nant + 1) / 2;
+  const int b = quarter * 32 + lane;
+  for (int lu = 0; lu < my_units; ++lu) {
+    const int buf = lu & 1;
+    const bool ok = mbar_wait(&bar_acc[buf], (uint32_t)((lu >> 1) & 1));
+    // (the warps agree, and the previous unit's reads of vbuf are done)
+    int all;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\t"
+        "barrier.cta.red.and.pred q, 1, %2, p;\n\tselp.b32 %0, 1, 0, q;\n\t}"
+        : "=r"(all)
+        : "r"((int)ok), "n"(NT)
+        : "memory");
+    if (!all) return false;
+    tc_fence_after();
+    int fv, ch0, pol0, npol_u;
+    split_unit(A, u_begin + lu, fv, ch0, pol0, npol_u);
+    const size_t step = A.fuse ? (size_t)A.ceff : (size_t)A.nchan * 2;
+    float2* o = A.out + (A.fuse ? (size_t)fv * nbase * A.ceff + ch0 / A.csf
+                                : ((size_t)fv * nbase * A.nchan + ch0) * 2 + pol0);
+    // place among the adjacent units of its row of outputs
+    const int n_fast = A.fuse ? A.ceff : 2 * A.nchan;
+    const int fast = (u_begin + lu) % n_fast, j1 = fast & (TC_QF - 1);
+    const uint32_t lane_base =
+        tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * 256);
+    for (int c0 = quarter * 32 + 16 * part; c0 < nant; c0 += NT / 8) {
+      __syncwarp();
+      uint32_t vr[16], vi[16];
+      tmem_ld16(lane_base + (uint32_t)c0, vr);
+      tmem_ld16(lane_base + 128u + (uint32_t)c0, vi);
+      tmem_ld_wait();
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const int a = c0 + j;
+        if (a < b || a >= nant) continue;
+        const float2 z = make_float2(__uint_as_float(vr[j]), __uint_as_float(vi[j]));
+        if (A.q_pitch) vbuf[j1 * A.q_pitch + upper_bls(a, b)] = z;
+        else o[(size_t)upper_bls(a, b) * step] = z;
+      }
+    }
+    tc_fence_before();
+    mbar_arrive(&bar_out[buf]);
+    if (A.q_pitch && (j1 == TC_QF - 1 || fast == n_fast - 1 || lu == my_units - 1)) {
+      asm volatile("barrier.cta.sync 1, %0;" ::"n"(NT) : "memory");
+      const int q = threadIdx.x & (TC_QF - 1);
+      if (q >= max(0, j1 - lu) && q <= j1)
+        for (int bls = threadIdx.x / TC_QF; bls < nbase; bls += NT / TC_QF)
+          o[(size_t)bls * step + q - j1] = vbuf[q * A.q_pitch + bls];
+    }
+  }
+  return true;
+}
+
+// The products of one stage of `rows` samples (part_bytes apart, antenna
+// atoms rows * 128 bytes apart) into accumulator columns d (Re), d + 128 (Im).
+DSB_DEV void mn_products(uint32_t d, uint32_t idesc, uint32_t stage, uint32_t part_bytes,
+                         uint32_t rows, int n16, bool first) {
+  constexpr uint32_t NEG_A = 1u << 13;
+  for (int m = 0; m < n16; ++m) {
+    const uint64_t R = sdesc_mn_sw128(stage + (uint32_t)m * 2048u, rows * 128, 1024);
+    const uint64_t I = sdesc_mn_sw128(stage + part_bytes + (uint32_t)m * 2048u, rows * 128, 1024);
+    const uint32_t acc = (!first || m > 0) ? 1u : 0u;
+    umma_f16_ss(d, R, R, idesc, acc);
+    umma_f16_ss(d, I, I, idesc, 1u);
+    umma_f16_ss(d + 128u, R, I, idesc, acc);
+    umma_f16_ss(d + 128u, I, R, idesc | NEG_A, 1u);
+  }
+}
+
 // ESZ: bytes of a voltage part (1 int8, 2 float16); COPY: float16 rows in
 // whole 16-byte chunks, staged by asynchronous copies.
 template <int ESZ, bool COPY>
@@ -1207,38 +1289,7 @@ __global__ void __launch_bounds__(MN_THREADS, 1) corr_split_mn_kernel(const Spli
   bool ok = true;
 
   if (warp < MN_EPI / 32) {
-    // ---- write finished units: accumulator lane b, columns a (Re), 128 + a
-    //      (Im); the upper triangle b <= a goes to bls(a, b) ----
-    const int nant = A.nant, nbase = nant * (nant + 1) / 2;
-    const int b = warp * 32 + lane;
-    for (int lu = 0; ok && lu < my_units; ++lu) {
-      const int buf = lu & 1;
-      ok = __all_sync(0xffffffffu, mbar_wait(&bar_acc[buf], (uint32_t)((lu >> 1) & 1)));
-      if (!ok) break;
-      tc_fence_after();
-      int fv, ch0, pol0, npol_u;
-      split_unit(A, u_begin + lu, fv, ch0, pol0, npol_u);
-      const size_t step = A.fuse ? (size_t)A.ceff : (size_t)A.nchan * 2;
-      float2* o = A.out + (A.fuse ? (size_t)fv * nbase * A.ceff + ch0 / A.csf
-                                  : ((size_t)fv * nbase * A.nchan + ch0) * 2 + pol0);
-      const uint32_t lane_base = tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)(buf * 256);
-      for (int c0 = warp * 32; c0 < nant; c0 += 16) {   // columns a >= this warp's rows
-        __syncwarp();
-        uint32_t vr[16], vi[16];
-        tmem_ld16(lane_base + (uint32_t)c0, vr);
-        tmem_ld16(lane_base + 128u + (uint32_t)c0, vi);
-        tmem_ld_wait();
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const int a = c0 + j;
-          if (a < b || a >= nant) continue;
-          o[(size_t)upper_bls(a, b) * step] =
-              make_float2(__uint_as_float(vr[j]), __uint_as_float(vi[j]));
-        }
-      }
-      tc_fence_before();
-      mbar_arrive(&bar_out[buf]);
-    }
+    ok = mn_write_units<MN_EPI>(A, tmem_base, u_begin, my_units, bar_acc, bar_out, nullptr);
   } else if (warp < (MN_EPI + MN_LOAD) / 32) {
     // ---- stage samples: thread (j, r) copies antennas 8j .. 8j + 7 of rows
     //      r, r + 16, ... of the stage ----
@@ -1326,7 +1377,6 @@ __global__ void __launch_bounds__(MN_THREADS, 1) corr_split_mn_kernel(const Spli
     const uint32_t n_b = (uint32_t)((A.nant + 15) & ~15);
     const uint32_t idesc = (1u << 4) | (1u << 15) | (1u << 16) | ((n_b >> 3) << 17) |
                            ((128u >> 4) << 24);
-    constexpr uint32_t NEG_A = 1u << 13;
     for (int it = 0; ok && it < n_items; ++it) {
       const int lu = it / A.n_chunks, q = it % A.n_chunks;
       const int slot = it % MN_NST, buf = lu & 1;
@@ -1334,18 +1384,9 @@ __global__ void __launch_bounds__(MN_THREADS, 1) corr_split_mn_kernel(const Spli
       ok = ok && mbar_wait(&bar_full[slot], (uint32_t)((it / MN_NST) & 1));
       if (!ok) break;
       tc_fence_after();
-      const uint32_t dr = tmem_base + (uint32_t)(buf * 256), di = dr + 128u;
-      const uint32_t sr = smem_u32(stages + (size_t)slot * MN_STAGE);
-      const int n16 = (min(MN_KC, A.kprime - q * MN_KC) + 15) >> 4;
-      for (int m = 0; m < n16; ++m) {
-        const uint64_t R = sdesc_mn_sw128(sr + (uint32_t)m * 2048u, MN_KC * 128, 1024);
-        const uint64_t I = sdesc_mn_sw128(sr + MN_PART + (uint32_t)m * 2048u, MN_KC * 128, 1024);
-        const uint32_t acc = (q > 0 || m > 0) ? 1u : 0u;
-        umma_f16_ss(dr, R, R, idesc, acc);
-        umma_f16_ss(dr, I, I, idesc, 1u);
-        umma_f16_ss(di, R, I, idesc, acc);
-        umma_f16_ss(di, I, R, idesc | NEG_A, 1u);
-      }
+      mn_products(tmem_base + (uint32_t)(buf * 256), idesc,
+                  smem_u32(stages + (size_t)slot * MN_STAGE), MN_PART, MN_KC,
+                  (min(MN_KC, A.kprime - q * MN_KC) + 15) >> 4, q == 0);
       umma_commit(&bar_free[slot]);
       if (q == A.n_chunks - 1) umma_commit(&bar_acc[buf]);
     }
@@ -1355,6 +1396,132 @@ __global__ void __launch_bounds__(MN_THREADS, 1) corr_split_mn_kernel(const Spli
     mbar_wait(bar_drain, 0u);
   }
   if (!ok && lane == 0) dsb_flag(A.status, DSB_E_TIMEOUT);
+  __syncwarp();
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, TC_TMEM_COLS);
+  }
+}
+
+// The same on float16 voltages whose samples TMA can bring in: rows of a
+// multiple of 8 antennas, 16-byte aligned, and stages of whole runs of packets
+// (split_tma_plan).  One thread issues up to four copies per stage (real and
+// imaginary parts, one or two antenna atoms), so that the load runs at memory
+// speed: asynchronous copies by 256 threads took 431 us for a native page by
+// themselves.  The stages are short (32 samples) to leave room for the staged
+// outputs of four units.  Native float16 page: 0.57 -> 0.36 ms.
+constexpr int ST_EPI = 256, ST_THREADS = ST_EPI + 64, ST_MAX_STAGES = 12;
+constexpr int ST_EXTRA = 1024 + (2 * ST_MAX_STAGES + 5) * 8 + 32;
+
+__global__ void __launch_bounds__(ST_THREADS, 1) corr_split_tma_kernel(
+    const SplitTcArgs A, const __grid_constant__ CUtensorMap map_re,
+    const __grid_constant__ CUtensorMap map_im) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* stages = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint64_t* bar_full = reinterpret_cast<uint64_t*>(stages + (size_t)A.nstage * A.stage_bytes);
+  uint64_t* bar_free = bar_full + A.nstage;
+  uint64_t* bar_acc = bar_free + A.nstage;   // [2] accumulator finished
+  uint64_t* bar_out = bar_acc + 2;           // [2] accumulator written out
+  uint64_t* bar_drain = bar_out + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_drain + 1);
+  float2* vbuf = reinterpret_cast<float2*>(tmem_slot + 4);   // [TC_QF][q_pitch]
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (warp == 0) {
+    tmem_alloc(tmem_slot, TC_TMEM_COLS);
+    tmem_relinquish();
+  }
+  if (tid == 0) {
+    for (int i = 0; i < A.nstage; ++i) {
+      mbar_init(&bar_full[i], 1);
+      mbar_init(&bar_free[i], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&bar_acc[i], 1);
+      mbar_init(&bar_out[i], ST_EPI);
+    }
+    mbar_init(bar_drain, 1);
+    fence_mbar_init();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  const int per_cta = (A.n_units + (int)gridDim.x - 1) / (int)gridDim.x;
+  const int u_begin = (int)blockIdx.x * per_cta;
+  const int my_units = max(0, min(per_cta, A.n_units - u_begin));
+  const int n_atoms = A.nant > 64 ? 2 : 1;
+  const uint32_t atom = (uint32_t)A.rows * 128u, part = 2 * atom;   // bytes
+  bool ok = true;
+
+  if (warp < ST_EPI / 32) {
+    ok = mn_write_units<ST_EPI>(A, tmem_base, u_begin, my_units, bar_acc, bar_out, vbuf);
+  } else if (warp == ST_EPI / 32) {
+    if (lane == 0) {
+      int issued = 0, slot = 0;
+      uint32_t ph = 1u;   // parity of the stage's previous use (the first passes have none)
+      for (int lu = 0; ok && lu < my_units; ++lu) {
+        int fv, ch0, pol0, npol_u;
+        split_unit(A, u_begin + lu, fv, ch0, pol0, npol_u);
+        // sample rows of the unit: packet fastest, then pol, then (ch, t)
+        int pk = 0, pl = 0;
+        for (int q = 0; q < A.n_chunks; ++q) {
+          if (issued >= A.nstage) ok = mbar_wait(&bar_free[slot], ph);
+          if (!ok) break;
+          const int x1 = fv * A.ppfv + pk;
+          const int x2 = npol_u == 2 ? (pl & 1) : pol0, x3 = 2 * ch0 + (npol_u == 2 ? pl >> 1 : pl);
+          uint8_t* st = stages + (size_t)slot * A.stage_bytes;
+          mbar_arrive_expect_tx(&bar_full[slot], 2u * (uint32_t)n_atoms * atom);
+          for (int a = 0; a < n_atoms; ++a) {
+            tma_load_4d(st + a * atom, &map_re, 64 * a, x1, x2, x3, &bar_full[slot]);
+            tma_load_4d(st + part + a * atom, &map_im, 64 * a, x1, x2, x3, &bar_full[slot]);
+          }
+          pk += A.rows;   // whole packet runs: a stage ends inside a plane or at its end
+          while (pk >= A.ppfv) {
+            pk -= A.ppfv;
+            ++pl;
+          }
+          ++issued;
+          if (++slot == A.nstage) {
+            slot = 0;
+            ph ^= 1u;
+          }
+        }
+      }
+      // no copy may be in flight into this CTA's shared memory when it ends
+      for (int it = max(0, issued - A.nstage); it < issued; ++it)
+        mbar_wait(&bar_full[it % A.nstage], (uint32_t)((it / A.nstage) & 1));
+    }
+  } else if (lane == 0) {
+    const uint32_t n_b = (uint32_t)((A.nant + 15) & ~15);
+    const uint32_t idesc = (1u << 4) | (1u << 15) | (1u << 16) | ((n_b >> 3) << 17) |
+                           ((128u >> 4) << 24);
+    int slot = 0;
+    uint32_t ph = 0u;
+    for (int lu = 0; ok && lu < my_units; ++lu) {
+      const int buf = lu & 1;
+      if (lu >= 2) ok = mbar_wait(&bar_out[buf], (uint32_t)(((lu >> 1) - 1) & 1));
+      for (int q = 0; ok && q < A.n_chunks; ++q) {
+        ok = mbar_wait(&bar_full[slot], ph);
+        if (!ok) break;
+        tc_fence_after();
+        mn_products(tmem_base + (uint32_t)(buf * 256), idesc,
+                    smem_u32(stages + (size_t)slot * A.stage_bytes), part, (uint32_t)A.rows,
+                    A.rows / 16, q == 0);
+        umma_commit(&bar_free[slot]);
+        if (++slot == A.nstage) {
+          slot = 0;
+          ph ^= 1u;
+        }
+      }
+      if (ok) umma_commit(&bar_acc[buf]);
+    }
+    // every product issued here ends before tensor memory is given back
+    umma_commit(bar_drain);
+    mbar_wait(bar_drain, 0u);
+  }
+  if (!ok) dsb_flag(A.status, DSB_E_TIMEOUT);
   __syncwarp();
   tc_fence_before();
   __syncthreads();
@@ -1533,6 +1700,49 @@ int tc_launch(TcArgs& A, int n_units, int max_ctas, cudaStream_t stream) {
   return launch_status();
 }
 
+// Plan corr_split_tma_kernel and its tensor maps, if the unit's samples come
+// in stages of `rows` (16 or 32) that are whole packet runs of one box: a
+// part as a 4-D float16 tensor (antenna, packet, pol, channel x t).
+bool split_tma_plan(SplitTcArgs& A, CUtensorMap* re, CUtensorMap* im) {
+  auto fn = tmap_encoder();
+  if (!fn || A.nant % 8) return false;
+  SplitTcArgs P = A;
+  P.rows = P.kprime % 32 == 0 ? 32 : 16;
+  if (P.kprime % P.rows) return false;
+  const int npol = P.fuse ? 2 : 1;
+  int pk, pol, cht;   // box
+  if (P.ppfv % P.rows == 0) {
+    pk = P.rows; pol = 1; cht = 1;
+  } else if (P.rows % P.ppfv == 0) {
+    const int planes = P.rows / P.ppfv;
+    if (planes % npol) return false;
+    pk = P.ppfv; pol = npol; cht = planes / npol;
+  } else {
+    return false;
+  }
+  P.n_chunks = P.kprime / P.rows;
+  P.stage_bytes = 4 * P.rows * 128;
+  const int room = 227 * 1024 - ST_EXTRA, nbase = P.nant * (P.nant + 1) / 2;
+  P.q_pitch = (nbase + 15) / 16 * 16 + 4;
+  if (room - P.q_pitch * TC_QF * 8 < 4 * P.stage_bytes) P.q_pitch = 0;
+  P.nstage = std::min(ST_MAX_STAGES, (room - P.q_pitch * TC_QF * 8) / P.stage_bytes);
+  const cuuint64_t row = (cuuint64_t)P.nant * 2, plane = row * (cuuint64_t)P.npkt;
+  const cuuint64_t dims[4] = {(cuuint64_t)P.nant, (cuuint64_t)P.npkt, 2u,
+                              (cuuint64_t)P.nchan * 2};
+  const cuuint64_t strides[3] = {row, plane, 2 * plane};
+  const cuuint32_t box[4] = {64u, (cuuint32_t)pk, (cuuint32_t)pol, (cuuint32_t)cht};
+  const cuuint32_t es[4] = {1u, 1u, 1u, 1u};
+  auto enc = [&](CUtensorMap* m, const void* p) {
+    return fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<void*>(p), dims, strides, box, es,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) ==
+           CUDA_SUCCESS;
+  };
+  if (!enc(re, P.re) || !enc(im, P.im)) return false;
+  A = P;
+  return true;
+}
+
 }  // namespace
 
 // ===========================================================================
@@ -1636,7 +1846,20 @@ int dsb_corr_split(const void* re, const void* im, int in_dtype, int nchan, int 
     return launch_status();
   };
   if (in_dtype == DSB_DT_INT8) return go(corr_split_mn_kernel<1, false>);
-  if (copy) return go(corr_split_mn_kernel<2, true>);
+  if (copy) {
+    CUtensorMap map_re, map_im;
+    if (split_tma_plan(A, &map_re, &map_im)) {
+      // more than half an SM's shared memory: one CTA (and its 512 tensor
+      // memory columns) per SM
+      const int smem = std::max(A.nstage * A.stage_bytes + A.q_pitch * TC_QF * 8 + ST_EXTRA,
+                                TC_MIN_SMEM);
+      cudaFuncSetAttribute(corr_split_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           smem);
+      corr_split_tma_kernel<<<grid, ST_THREADS, smem, stream>>>(A, map_re, map_im);
+      return launch_status();
+    }
+    return go(corr_split_mn_kernel<2, true>);
+  }
   return go(corr_split_mn_kernel<2, false>);
 }
 
