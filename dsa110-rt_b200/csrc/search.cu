@@ -1375,17 +1375,19 @@ __global__ void __launch_bounds__(L1_THREADS) clipped_std_kernel(const L1Src src
   __shared__ __align__(16) float v[L1_MAX];
   __shared__ double red[L1_THREADS / 32];
   __shared__ int s_lo, s_hi;
+  if (threadIdx.x == 0) {
+    s_lo = 0;
+    s_hi = 0;
+  }
+  __syncthreads();
   const float* row = src.x + (long long)blockIdx.x * (GATHER ? src.f_stride : m);
-  int P = 1;
-  while (P < m) P <<= 1;
   // Thread t holds samples 4t .. 4t + 3 in registers (every load issues
   // before the first is used); the padding past m is +inf.  The bitonic
   // network sorts all L1_MAX entries: its stages with partner distance j < 4
   // run inside the thread, 4 <= j <= 64 across the warp by shuffles, and only
   // j >= 128 through shared memory with a barrier (15 of the 78 stages).
-  // The smallest P entries are the P entries of the P-padded sort, so the
-  // result is the same as sorting P.
   static_assert(L1_MAX == 4 * L1_THREADS, "four samples per thread");
+  static_assert(L1_THREADS == 1024, "one sum per lane of a warp");
   float r[4];
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
@@ -1401,6 +1403,11 @@ __global__ void __launch_bounds__(L1_THREADS) clipped_std_kernel(const L1Src src
 #pragma unroll
   for (int q = 0; q < 4; ++q)
     if (!(r[q] == r[q]) || isinf(r[q])) r[q] = __int_as_float(0x7f800000);  // non-finite -> +inf
+  {  // s_hi: the finite samples (the sort's barriers follow)
+    const int n_fin = (int)!isinf(r[0]) + (int)!isinf(r[1]) + (int)!isinf(r[2]) + (int)!isinf(r[3]);
+    const int w = __reduce_add_sync(0xffffffffu, n_fin);
+    if ((threadIdx.x & 31) == 0) atomicAdd(&s_hi, w);
+  }
   const int i0 = 4 * threadIdx.x;
   float4* v4 = reinterpret_cast<float4*>(v);
   // compare-exchange of positions (i, i ^ j), i the lower: ascending where
@@ -1456,19 +1463,6 @@ __global__ void __launch_bounds__(L1_THREADS) clipped_std_kernel(const L1Src src
   }
   v4[threadIdx.x] = make_float4(r[0], r[1], r[2], r[3]);
   __syncthreads();
-  // finite count
-  if (threadIdx.x == 0) {
-    int n_fin = 0;
-    int lo = 0, hi = P;
-    while (lo < hi) {
-      const int mid = (lo + hi) / 2;
-      if (isinf(v[mid]) && v[mid] > 0) hi = mid; else lo = mid + 1;
-    }
-    n_fin = lo;
-    s_lo = 0;
-    s_hi = n_fin;
-  }
-  __syncthreads();
   float sigma = 0.f, med = 0.f;
   for (int it = 0; it <= n_iter; ++it) {
     const int lo = s_lo, hi = s_hi;
@@ -1487,24 +1481,42 @@ __global__ void __launch_bounds__(L1_THREADS) clipped_std_kernel(const L1Src src
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
     __syncthreads();
-    if (threadIdx.x == 0) {
-      double tot = 0.0;
-      for (int w = 0; w < L1_THREADS / 32; ++w) tot += red[w];
-      red[0] = tot;
-    }
-    __syncthreads();
-    sigma = sqrtf((float)red[0] / (float)cnt);
-    __syncthreads();
+    // every warp adds the warps' sums itself (one barrier, no serial chain)
+    double tot = red[threadIdx.x & 31];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
+    sigma = sqrtf((float)tot / (float)cnt);
     if (it == n_iter) break;
-    if (threadIdx.x == 0) {
+    // the clipped range: 32 samples from each end at a time, by warp 0
+    if (threadIdx.x < 32) {
       const float lo_v = med - n_sigma * sigma, hi_v = med + n_sigma * sigma;
       int a = lo, b = hi;
-      while (a < hi && v[a] < lo_v) ++a;
-      while (b > a && v[b - 1] > hi_v) --b;
-      s_lo = a;
-      s_hi = b;
+      for (;;) {
+        const int x = a + (int)threadIdx.x;
+        const int n = __ffs(~__ballot_sync(0xffffffffu, x < hi && v[x] < lo_v));
+        if (n == 0) {
+          a += 32;
+          continue;
+        }
+        a += n - 1;
+        break;
+      }
+      for (;;) {
+        const int x = b - 1 - (int)threadIdx.x;
+        const int n = __ffs(~__ballot_sync(0xffffffffu, x >= a && v[x] > hi_v));
+        if (n == 0) {
+          b -= 32;
+          continue;
+        }
+        b -= n - 1;
+        break;
+      }
+      if (threadIdx.x == 0) {
+        s_lo = a;
+        s_hi = b;
+      }
     }
-    __syncthreads();
+    __syncthreads();   // the new range, and red may be written again
   }
   if (threadIdx.x == 0) {
     float o = (sigma == sigma) ? sigma : 0.f;
