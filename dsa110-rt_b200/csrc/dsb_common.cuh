@@ -280,6 +280,15 @@ DSB_DEV void tmem_ld16_wait(uint32_t taddr, uint32_t (&r)[16]) {
       : "memory");
 }
 
+// Wait for the loads issued so far; r, one of their targets, passes through
+// the statement so that none of its uses can be scheduled before the wait.
+DSB_DEV void tmem_ld_wait16(uint32_t (&r)[16]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]),
+                 "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]),
+                 "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])::"memory");
+}
+
 // Store 16 consecutive 32-bit TMEM columns of this warp's 32 lanes.
 DSB_DEV void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
   asm volatile(

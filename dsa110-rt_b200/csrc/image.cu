@@ -175,8 +175,19 @@ DSB_DEV void idftR(float2 (&a)[R]) {
   else idft4(a[0], a[1], a[2], a[3]);
 }
 
-// a * W_8 = a * (1 + i) / sqrt(2)
-DSB_DEV float2 cmul_w8(float2 a) { return make_float2(R2 * (a.x - a.y), R2 * (a.x + a.y)); }
+// W_8^k, the quarter turns exact
+__device__ __constant__ float2 kW8[8] = {
+    {1.0f, 0.0f},  {R2, R2},   {0.0f, 1.0f},  {-R2, R2},
+    {-1.0f, 0.0f}, {-R2, -R2}, {0.0f, -1.0f}, {R2, -R2}};
+
+// The float2 at shared address p = v where ok, without a branch
+DSB_DEV void st_shared_if(uint32_t p, float2 v, bool ok) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %3, 0;\n\t@q st.shared.v2.f32 [%0], {%1, %2};\n\t}\n" ::"r"(
+          p),
+      "f"(v.x), "f"(v.y), "r"((int)ok)
+      : "memory");
+}
 
 // Stage-2 ring elements (FMT): 0 complex64; 1 the BF16 storage form (bf16
 // re/im pairs in 32 bits); 2 the cint8 wire form (int8 re/im pairs in 16
@@ -300,8 +311,8 @@ struct ImgGeom {
   static constexpr bool META32 = (N == 512);
   // entry metadata fields: column | n' << NP_SH | q << Q_SH | last << LAST_SH
   // (32-bit form also: packed << ROT_SH | parity(u + w) << ROT_SH + 1)
-  static constexpr int NP_SH = META32 ? 8 : 7;
-  static constexpr int Q_SH = META32 ? 14 : 13;
+  [[maybe_unused]] static constexpr int NP_SH = META32 ? 8 : 7;
+  [[maybe_unused]] static constexpr int Q_SH = META32 ? 14 : 13;
   static constexpr int LAST_SH = META32 ? 17 : 15;
   static constexpr int ROT_SH = 18;
   static constexpr int CG = THREADS / C1;         // column groups
@@ -328,9 +339,10 @@ struct ImgGeom {
                 "entry metadata field widths");
   static_assert(MAXE % 8 == 0 && MAXE <= 64, "whole 8-entry chunks, 64-bit rotation masks");
   static_assert(LC <= 64, "one 64-bit occupancy mask per column");
-  // buf | tw (N) | rtw (R1*R2) | ctw (C1*C1) | slice pointers | cell bases |
+  // buf | tw (N) | rtw (R1*R2) | ctw (C1*C1) | rot (FOLD*FOLD) | slice pointers | cell bases |
   // ends of the chgroups' cells | slice scales | TMEM address | k
-  static constexpr size_t SMEM = BUFB + (size_t)(N + R1 * R2 + C1 * C1) * 8 + IMG_MAX_G * 8 +
+  static constexpr size_t SMEM = BUFB + (size_t)(N + R1 * R2 + C1 * C1 + FOLD * FOLD) * 8 +
+                                 IMG_MAX_G * 8 +
                                  (IMG_MAX_G + 1) * 4 + IMG_MAX_G * 4 + IMG_MAX_G * 4 + 16;
   static_assert(SMEM <= 227 * 1024, "shared memory of one CTA");
   static_assert(!META32 || (size_t)BUF * 8 + FC_BYTES + (size_t)MAX_SLOTS * 2 <= BUFB,
@@ -373,7 +385,8 @@ __global__ void __launch_bounds__(ImgGeom<N>::THREADS, ImgGeom<N>::CTAS)
   // rtw[m2*R1 + j] = W_N^(j m2), ctw[m1*C1 + j] = W_LC^(j m1)
   float2* rtw = tw + N;
   float2* ctw = rtw + R1 * R2;
-  const Elem** s_slice = reinterpret_cast<const Elem**>(ctw + C1 * C1);
+  float2* s_rot = ctw + C1 * C1;   // W_FOLD^(q p) at [p][q]
+  const Elem** s_slice = reinterpret_cast<const Elem**>(s_rot + FOLD * FOLD);
   int* s_cbase = reinterpret_cast<int*>(s_slice + IMG_MAX_G);
   int* s_end = s_cbase + IMG_MAX_G + 1;
   float* s_scale = reinterpret_cast<float*>(s_end + IMG_MAX_G);
@@ -388,6 +401,7 @@ __global__ void __launch_bounds__(ImgGeom<N>::THREADS, ImgGeom<N>::CTAS)
     rtw[i] = A.tw[((i % R1) * (i / R1)) & (N - 1)];
   for (int i = tid; i < C1 * C1; i += THREADS)
     ctw[i] = A.tw[((i % C1) * (i / C1) * (N / LC)) & (N - 1)];
+  if (tid < FOLD * FOLD) s_rot[tid] = kW8[(tid % FOLD) * (tid / FOLD) * (8 / FOLD) & 7];
   for (int g = tid; g <= A.G; g += THREADS) s_cbase[g] = A.cell_base[g];
   for (int g = tid; g < A.G; g += THREADS) s_end[g] = A.cell_base[g] + A.n_filled[g];
   // this thread's S entries [sb, sb + sn), whole slots
@@ -429,6 +443,27 @@ __global__ void __launch_bounds__(ImgGeom<N>::THREADS, ImgGeom<N>::CTAS)
   tc_fence_after();
   const uint32_t tbase = *s_tmem + ((uint32_t)((warp & 3) * 32) << 16) +
                          (uint32_t)((warp >> 2) * Gm::WARP_COLS);
+
+  // the fold's compact tables (32-bit form): each thread's nibble words and
+  // every slot's offset, in the part of buf past the column buffer.  Where the
+  // combine's S arrays end before them too they are loaded once per CTA, else
+  // once per image after S has left (16-byte copies; slot_off is padded to 8).
+  const size_t tab_bytes = (size_t)Gm::MAXC * THREADS * 4 + (size_t)((n_sl + 7) / 8) * 16;
+  const bool tab_resident =
+      Gm::META32 && (size_t)A.s_stride * 8 + tab_bytes <= Gm::BUFB;
+  uint32_t* s_code = reinterpret_cast<uint32_t*>(
+      smem_raw + (tab_resident ? (Gm::BUFB - tab_bytes) / 16 * 16 : (size_t)Gm::BUF * 8));
+  auto load_tables = [&] {
+    const uint8_t* gt = reinterpret_cast<const uint8_t*>(A.gmeta) + Gm::GM_BYTES;
+    const uint32_t* g_code = reinterpret_cast<const uint32_t*>(gt);
+    for (int c = 0; c < nch; ++c) s_code[c * THREADS + tid] = __ldg(g_code + c * THREADS + tid);
+    const uint4* g_slot =
+        reinterpret_cast<const uint4*>(gt + Gm::FC_BYTES + Gm::TS_BYTES + Gm::ROT_BYTES);
+    uint4* s_slot4 = reinterpret_cast<uint4*>(s_code + Gm::MAXC * THREADS);
+    for (int i = tid; i < (n_sl + 7) / 8; i += THREADS) s_slot4[i] = __ldg(g_slot + i);
+  };
+  if constexpr (Gm::META32)
+    if (tab_resident) load_tables();   // (the image loop's barriers follow)
 
   const int n_tot = A.cell_base[A.G];
   // 0.5 / N^2 is a power of two, applied to S on its way into TMEM: scaling
@@ -614,126 +649,88 @@ __global__ void __launch_bounds__(ImgGeom<N>::THREADS, ImgGeom<N>::CTAS)
     }
     __syncthreads();  // S is read: buf is free for the passes
     if constexpr (Gm::META32) {
-      // the fold's compact tables into the part of buf past the column buffer
-      // (the combine's S arrays overlapped it): this thread's nibble words,
-      // and every slot's offset (16-byte copies; slot_off is padded to 8)
-      uint32_t* s_code = reinterpret_cast<uint32_t*>(buf + Gm::BUF);
-      const uint8_t* gt = reinterpret_cast<const uint8_t*>(A.gmeta) + Gm::GM_BYTES;
-      const uint32_t* g_code = reinterpret_cast<const uint32_t*>(gt);
-      for (int c = 0; c < nch; ++c) s_code[c * THREADS + tid] = __ldg(g_code + c * THREADS + tid);
-      const uint4* g_slot =
-          reinterpret_cast<const uint4*>(gt + Gm::FC_BYTES + Gm::TS_BYTES + Gm::ROT_BYTES);
-      uint4* s_slot4 = reinterpret_cast<uint4*>(s_code + Gm::MAXC * THREADS);
-      for (int i = tid; i < (n_sl + 7) / 8; i += THREADS) s_slot4[i] = __ldg(g_slot + i);
-      __syncthreads();
+      if (!tab_resident) {
+        load_tables();
+        __syncthreads();
+      }
     }
 
     for (int p = 0; p < FOLD; ++p) {
       // ---- 2a. fold S into the occupied slots (n', col) of buf: each slot's
       //      entries are consecutive in one thread's range, written once
       //      after the last of them ----
-      // (one copy of the loop per pass, so that the rotation W_FOLD^(q p)
-      // needs as little work as the pass allows: none for p = 0, a sign for
-      // p = FOLD/2, a swap and signs for the other even multiples, and one
-      // multiply by W_8 for the odd ones)
-      auto fold = [&](auto pass) {
-        constexpr unsigned PP = decltype(pass)::value;
+      // Entry q of a slot turns by W_FOLD^(q p): one complex multiply-add
+      // with a factor from a table in shared memory (exact for the quarter
+      // turns, so only N = 512 rounds there).  No branch depends on an
+      // entry: absent entries are zeros with q = 0 that end no slot, and a
+      // slot's store is predicated.  (A branch-free copy of the loop per
+      // pass, and a branch per ended slot: FOLD_TIME.)
+      {
+        const float2* rot = s_rot + p * FOLD;
+        const uint32_t buf32 = smem_u32(buf);
         float2 acc = make_float2(0.f, 0.f);
-        if constexpr (Gm::META32) {
-          // compact tables in shared memory: one nibble word per chunk, and
-          // the offset of each of this thread's slots, in order
-          const uint32_t* s_code = reinterpret_cast<const uint32_t*>(buf + Gm::BUF);
-          const uint16_t* s_soff = reinterpret_cast<const uint16_t*>(s_code + Gm::MAXC * THREADS);
-          int si = sl0;
-          for (int c = 0; c < nch; ++c) {
+        // compact tables in shared memory (32-bit form): a nibble word per
+        // chunk, and the offset of each of this thread's slots, in order
+        const uint16_t* s_soff = reinterpret_cast<const uint16_t*>(s_code + Gm::MAXC * THREADS);
+        int si = sl0;
+        auto entry = [&](float x, float y, unsigned q, bool last, unsigned off) {
+          const float2 w = rot[q];
+          acc.x = fmaf(-y, w.y, fmaf(x, w.x, acc.x));
+          acc.y = fmaf(y, w.x, fmaf(x, w.y, acc.y));
+          st_shared_if(buf32 + off * 8u, acc, last);
+          acc.x = last ? 0.f : acc.x;
+          acc.y = last ? 0.f : acc.y;
+        };
+        auto chunk = [&](int c, const uint32_t (&r)[16], const unsigned (&m)[8]) {
+          if constexpr (Gm::META32) {
             const uint32_t cw = s_code[c * THREADS + tid];
-            uint32_t r[16];
-            tmem_ld16_wait(tbase + 16 * c, r);
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-              if (8 * c + j < sn) {
-                const unsigned code = (cw >> (4 * j)) & 15u;
-                float2 v = make_float2(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
-                if constexpr (PP != 0) {
-                  // W_8^k = i^(k >> 1) x (W_8 if k is odd), k = q p mod 8
-                  const unsigned k = ((code & 7u) * PP) & 7u;
-                  if constexpr (PP & 1u) {
-                    if (k & 1u) v = cmul_w8(v);
-                  }
-                  v = crot_rt(v, k >> 1);
-                }
-                acc = cadd(acc, v);
-                if (code & 8u) {
-                  if (DSB_INB(si, n_sl, A.status)) {
-                    const unsigned off = s_soff[si];
-                    if (DSB_INB(off, Gm::BUF, A.status)) buf[off] = acc;
-                  }
-                  ++si;
-                  acc = make_float2(0.f, 0.f);
-                }
-              }
+              const unsigned code = cw >> (4 * j);
+              bool last = code & 8u;
+              const unsigned off = s_soff[si];
+              si += last;
+#ifdef DSB_CHECK
+              last = last && DSB_INB(si - 1, n_sl, A.status) && DSB_INB(off, Gm::BUF, A.status);
+#endif
+              entry(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]), code & 7u, last, off);
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              entry(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]),
+                    (m[j] >> Gm::Q_SH) & (FOLD - 1), (m[j] >> Gm::LAST_SH) & 1u,
+                    ((m[j] >> Gm::NP_SH) & (LC - 1)) * P + (m[j] & (NC - 1)));
+          }
+        };
+        // two chunks in registers where there is room for them (N = 512)
+        uint32_t ra[16];
+        unsigned ma[8];
+        if constexpr (Gm::META32) {
+          uint32_t rb[16];
+          tmem_ld16(tbase, ra);
+          for (int c = 0; c < nch; c += 2) {
+            tmem_ld_wait16(ra);
+            if (c + 1 < nch) tmem_ld16(tbase + 16 * (c + 1), rb);
+            chunk(c, ra, ma);
+            if (c + 1 < nch) {
+              tmem_ld_wait16(rb);
+              if (c + 2 < nch) tmem_ld16(tbase + 16 * (c + 2), ra);
+              chunk(c + 1, rb, ma);
             }
           }
-          return;
-        }
-        unsigned md_next[8];
-        load_meta8<N>(gmeta, 0, tid, md_next);
-        for (int c = 0; c < nch; ++c) {
-          unsigned mw[8];
+        } else {
+          unsigned mn[8];
+          load_meta8<N>(gmeta, 0, tid, mn);
+          for (int c = 0; c < nch; ++c) {
 #pragma unroll
-          for (int j = 0; j < 8; ++j) mw[j] = md_next[j];
-          // next chunk's metadata loads under this one's
-          if (c + 1 < nch) load_meta8<N>(gmeta, c + 1, tid, md_next);
-          uint32_t r[16];
-          tmem_ld16_wait(tbase + 16 * c, r);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            if (8 * c + j < sn) {
-              const unsigned m = mw[j];
-              float2 v = make_float2(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
-              const unsigned q = (m >> Gm::Q_SH) & (FOLD - 1);
-              if constexpr (PP != 0) {
-                if constexpr (FOLD == 4) {
-                  if constexpr (PP == 2) {
-                    const unsigned sgn = (q & 1u) << 31;  // i^(2q) = (-1)^q
-                    v = make_float2(__uint_as_float(__float_as_uint(v.x) ^ sgn),
-                                    __uint_as_float(__float_as_uint(v.y) ^ sgn));
-                  } else {
-                    v = crot_rt(v, q * PP);
-                  }
-                } else {
-                  // W_8^k = i^(k >> 1) x (W_8 if k is odd), k = q p mod 8
-                  const unsigned k = (q * PP) & 7u;
-                  if constexpr (PP & 1u) {
-                    if (k & 1u) v = cmul_w8(v);
-                  }
-                  v = crot_rt(v, k >> 1);
-                }
-              }
-              acc = cadd(acc, v);
-              if ((m >> Gm::LAST_SH) & 1u) {
-                buf[((m >> Gm::NP_SH) & (LC - 1)) * P + (m & (NC - 1))] = acc;
-                acc = make_float2(0.f, 0.f);
-              }
-            }
+            for (int j = 0; j < 8; ++j) ma[j] = mn[j];
+            // next chunk's metadata loads under this one
+            if (c + 1 < nch) load_meta8<N>(gmeta, c + 1, tid, mn);
+            tmem_ld16_wait(tbase + 16 * c, ra);
+            chunk(c, ra, ma);
           }
         }
-      };
-      switch (p) {
-        case 0: fold(std::integral_constant<unsigned, 0>{}); break;
-        case 1: fold(std::integral_constant<unsigned, 1>{}); break;
-        case 2: fold(std::integral_constant<unsigned, 2>{}); break;
-        case 3: fold(std::integral_constant<unsigned, 3>{}); break;
-        default:
-          if constexpr (FOLD == 8) {
-            switch (p) {
-              case 4: fold(std::integral_constant<unsigned, 4>{}); break;
-              case 5: fold(std::integral_constant<unsigned, 5>{}); break;
-              case 6: fold(std::integral_constant<unsigned, 6>{}); break;
-              default: fold(std::integral_constant<unsigned, 7>{}); break;
-            }
-          }
-          break;
       }
       __syncthreads();
       // ---- 2b. column transforms of pass p (in place in buf); only the
@@ -780,8 +777,15 @@ __global__ void __launch_bounds__(ImgGeom<N>::THREADS, ImgGeom<N>::CTAS)
       //      FOLD*2pr + p and FOLD*(2pr+1) + p.  N = R1 * R2: thread rj holds
       //      points rj + R1 k2 (k2 < R2), takes their R2-point transform,
       //      twiddles it by W_N^(rj m2), and after the transpose owns the
-      //      R1-point transforms of columns m2 = rj + R1 h, which give the
-      //      outputs m2 + R2 m1 ----
+      //      R1-point transforms of columns m2 = rj + R1 h, or H rj + h
+      //      (h < H = R2 / R1; adjacent outputs, stored as pairs), which give
+      //      the outputs m2 + R2 m1 ----
+      constexpr int H = R2 / R1;
+      // N = 512 stores from registers: 8-byte stores, 128 bytes per group
+      // and row (4-byte ones cost 297 of the kernel's 2012 us per 2304 images)
+      constexpr bool ADJ = N == 512;
+      // column m2's XOR in the transpose: its reading thread
+      auto swz = [](int m2) { return (ADJ ? m2 / H : m2) & (R1 - 1); };
       for (int pr = rgi; pr < LC / 2; pr += Gm::RG) {
         float2* reg = buf + 2 * pr * P;
         const float2* ra = reg;
@@ -809,33 +813,29 @@ __global__ void __launch_bounds__(ImgGeom<N>::THREADS, ImgGeom<N>::CTAS)
         for (int m2 = 1; m2 < R2; ++m2) a[m2] = cmul(a[m2], rtw[m2 * R1 + rj]);
         __syncwarp(rmask);  // every lane has read the pair's rows
 #pragma unroll
-        for (int m2 = 0; m2 < R2; ++m2) reg[m2 * R1 + (rj ^ (m2 & (R1 - 1)))] = a[m2];
+        for (int m2 = 0; m2 < R2; ++m2) reg[m2 * R1 + (rj ^ swz(m2))] = a[m2];
         __syncwarp(rmask);
-        constexpr int H = R2 / R1;
         float2 b[H][R1];
 #pragma unroll
         for (int h = 0; h < H; ++h) {
-          const int m2 = rj + R1 * h;
+          const int m2 = ADJ ? H * rj + h : rj + R1 * h;
 #pragma unroll
           for (int jj = 0; jj < R1; ++jj) b[h][jj] = reg[m2 * R1 + (jj ^ rj)];
         }
         const size_t ibase = ((size_t)fl * A.n_t + t) * N;
         float* ra_out = A.out + (ibase + FOLD * (2 * pr) + p) * N;
         float* rb_out = A.out + (ibase + FOLD * (2 * pr + 1) + p) * N;
-        if constexpr (N == 512) {
-          // outputs straight from registers: for each (h, m1) the group's
-          // 16 lanes hold 16 consecutive pixels of each row (64 bytes), so
-          // no staging through shared memory (whose pipe the transposes
-          // already keep busy)
+        if constexpr (ADJ) {
+          // outputs straight from registers, so no staging through shared
+          // memory (whose pipe the transposes already keep busy)
+          static_assert(!ADJ || H == 2, "pairs of adjacent outputs");
 #pragma unroll
-          for (int h = 0; h < H; ++h) {
-            idftR<R1>(b[h]);
+          for (int h = 0; h < H; ++h) idftR<R1>(b[h]);
 #pragma unroll
-            for (int m1 = 0; m1 < R1; ++m1) {
-              const int x = rj + R1 * h + R2 * m1;
-              ra_out[x] = b[h][m1].x;
-              rb_out[x] = b[h][m1].y;
-            }
+          for (int m1 = 0; m1 < R1; ++m1) {
+            const int x = H * rj + R2 * m1;
+            *reinterpret_cast<float2*>(ra_out + x) = make_float2(b[0][m1].x, b[H - 1][m1].x);
+            *reinterpret_cast<float2*>(rb_out + x) = make_float2(b[0][m1].y, b[H - 1][m1].y);
           }
         } else {
           __syncwarp(rmask);
