@@ -258,6 +258,9 @@ class FastCorrKernel:
     nbada_pol: int = BADA_NPOL
     accum_dtype: torch.dtype = torch.float32
     _nbase: int = field(init=False)
+    # (stream, zeroed status words, how many are taken), see _status_word
+    _words: Optional[tuple] = field(default=None, init=False, repr=False, compare=False)
+    _last: Optional[tuple] = field(default=None, init=False, repr=False, compare=False)
 
     def __post_init__(self) -> None:
         self.device = _lib.cuda_device(self.device)
@@ -276,10 +279,31 @@ class FastCorrKernel:
     def nbase(self) -> int:
         return self._nbase
 
+    @property
+    def _last_status(self) -> Optional[torch.Tensor]:
+        return None if self._last is None else self._last[0][self._last[1]]
+
     def check_status(self) -> None:
-        st = getattr(self, "_last_status", None)
+        st = self._last_status
         if st is not None:
             _lib.check_status(st, "FastCorrKernel")
+
+    _N_WORDS = 256
+
+    def _status_word(self, stream: int) -> Tuple[torch.Tensor, int]:
+        """A zeroed device status word of this launch's own, (words, index).
+        Zeroing one per launch cost it an allocation and a fill kernel (20.9
+        -> 14.3 us per call at 16 antennas x 64 packets); 256 are zeroed at a time, on the stream that uses them, and none is
+        used twice.  A captured launch gets its own, which every replay
+        zeroes.  (The held tuple is read once: calls from two threads may
+        share a word, never run past the last.)"""
+        if torch.cuda.is_current_stream_capturing():
+            return _lib.status_word(self.device), 0
+        held = self._words
+        if held is None or held[0] != stream or held[2] >= self._N_WORDS:
+            held = (stream, torch.zeros(self._N_WORDS, dtype=torch.int32, device=self.device), 0)
+        self._words = (stream, held[1], held[2] + 1)
+        return held[1], held[2]
 
     def compute_split(self, real_v: torch.Tensor, imag_v: torch.Tensor, *,
                       n_fv_chunk: Optional[int] = None, fuse_stokes_i: bool = False,
@@ -306,12 +330,13 @@ class FastCorrKernel:
         else:
             out = torch.empty((n_fv, self._nbase, self.nchan, 2), dtype=torch.complex64,
                               device=self.device)
-        st = _lib.status_word(self.device)
+        stream = torch.cuda.current_stream(self.device).cuda_stream
+        words, i = st = self._status_word(stream)
         _lib.check(_lib.lib().dsb_corr_split(
-            _lib.ptr(re), _lib.ptr(im), _DT[re.dtype], self.nchan, re.shape[3], self.nants,
+            re.data_ptr(), im.data_ptr(), _DT[re.dtype], self.nchan, re.shape[3], self.nants,
             self.t_int_fast_native, int(bool(fuse_stokes_i)), int(chan_sum_factor),
-            _lib.ptr(out), _lib.ptr(st), _lib.stream_of(self.device)), "dsb_corr_split")
-        self._last_status = st
+            out.data_ptr(), words.data_ptr() + 4 * i, stream), "dsb_corr_split")
+        self._last = st
         return out
 
     def compute_raw(self, raw: torch.Tensor, *, chan_sum_factor: int, npkt: Optional[int] = None,
@@ -350,12 +375,13 @@ class FastCorrKernel:
             raise ValueError(f"layout {layout!r} not in ('tbc', 'bct')")
         if out is None:
             out = torch.empty(shape, dtype=torch.complex64, device=self.device)
-        st = _lib.status_word(self.device)
+        stream = torch.cuda.current_stream(self.device).cuda_stream
+        words, i = st = self._status_word(stream)
         _lib.check(_lib.lib().dsb_corr_tc(
-            _lib.ptr(raw), npkt * page, n_g, npkt, self.nants, self.nchan,
-            self.t_int_fast_native, chan_sum_factor, order, _lib.ptr(out), *strides, max_ctas,
-            _lib.ptr(st), _lib.stream_of(self.device)), "dsb_corr_tc")
-        self._last_status = st
+            raw.data_ptr(), npkt * page, n_g, npkt, self.nants, self.nchan,
+            self.t_int_fast_native, chan_sum_factor, order, out.data_ptr(), *strides, max_ctas,
+            words.data_ptr() + 4 * i, stream), "dsb_corr_tc")
+        self._last = st
         return out if raw.ndim == 6 else out[0]
 
 
