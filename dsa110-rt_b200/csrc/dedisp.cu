@@ -69,6 +69,10 @@ DSB_DEV void cp_async8(void* dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src)
                : "memory");
 }
+DSB_DEV void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src)
+               : "memory");
+}
 DSB_DEV void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 DSB_DEV void cp_async_wait() {
@@ -423,6 +427,7 @@ struct S1Args {
   long long t0;           // absolute time of the first output
   int n_t, n_dm, ceff;
   int win_len;            // S1_TT + largest shift spread over a DM group
+  int sbc;                // subbands per staged chunk (0: all at once)
   double2* sky_ring;      // (D rows, window) or null
   int sky_window, sky_head, sky_count, sky_subtract;
   int* status;
@@ -437,7 +442,13 @@ __host__ __device__ inline size_t s1_smem_bytes(int ceff, int dg, int win_len) {
   return (size_t)ceff * dg * 4 + (size_t)S1_MAX_C * 8 + (size_t)ceff * win_len * 32 + 16;
 }
 
-template <bool BF16, int DG>
+// CHUNK: where every subband's window together leaves one CTA per SM (few
+// coarse DMs over a wide range: the small plain configuration's 8 DMs of 600
+// pc cm^-3 / 32 need 219 KB), the subbands are staged A.sbc at a time in two
+// buffers, the next ones copied under the current ones' sums, which stay in
+// registers: two CTAs per SM and no exposed load.  300 -> 245 us per block of
+// that configuration (512 times, 32 DMs, 314 cells).
+template <bool BF16, int DG, bool CHUNK>
 __global__ void __launch_bounds__(S1_THREADS) stage1_rows_kernel(const S1Args A) {
   constexpr int L = S1_THREADS / DG;  // time lanes per DM
   static_assert(L >= 8 && L <= 32 && S1_TT % L == 0, "unsupported DM group");
@@ -448,7 +459,8 @@ __global__ void __launch_bounds__(S1_THREADS) stage1_rows_kernel(const S1Args A)
   int* s_len = s_lo + S1_MAX_C;                             // [s] window length
   float4* win0 = reinterpret_cast<float4*>(s1_smem + ((size_t)ceff * DG * 4 +
                                                       (size_t)S1_MAX_C * 8 + 15) / 16 * 16);
-  float4* win1 = win0 + (size_t)ceff * A.win_len;            // cells 2-3
+  const int n_win = CHUNK ? 2 * A.sbc : ceff;                // windows staged
+  float4* win1 = win0 + (size_t)n_win * A.win_len;           // cells 2-3
 
   const int g = A.blk_g[blockIdx.x];
   const int c0 = A.blk_c0[blockIdx.x];
@@ -506,78 +518,145 @@ __global__ void __launch_bounds__(S1_THREADS) stage1_rows_kernel(const S1Args A)
   const float4* Y4 = reinterpret_cast<const float4*>(A.Y);
   const long long ycol = (long long)A.y_base[g] + c0;   // a multiple of 4
 
-  for (int tt = 0; tt < A.n_t; tt += S1_TT) {
-    __syncthreads();  // the previous tile's windows are no longer read
-    // stage the windows: entry (sb, tau) = Y at time t0 + tt + lo[sb] + tau,
-    // flattened over (sb, tau) so that each thread's loads are independent
-    {
-      constexpr int U = 4;
-      const int n_e = ceff * A.win_len;
-      for (int e0 = 0; e0 < n_e; e0 += U * S1_THREADS) {
-        float4 v0[U], v1[U];
-        int ei[U];
+  // the sums (a0, a1) of the four cells at tile time tl, into ring slot `slot`
+  auto emit = [&](float4 a0, float4 a1, long long slot) {
+    sr[0] += a0.x; si[0] += a0.y; sr[1] += a0.z; si[1] += a0.w;
+    sr[2] += a1.x; si[2] += a1.y; sr[3] += a1.z; si[3] += a1.w;
+    float4 o0 = a0, o1 = a1;
+    if (sub) {
+      o0 = make_float4((float)((double)a0.x - mr[0]), (float)((double)a0.y - mi[0]),
+                       (float)((double)a0.z - mr[1]), (float)((double)a0.w - mi[1]));
+      o1 = make_float4((float)((double)a1.x - mr[2]), (float)((double)a1.y - mi[2]),
+                       (float)((double)a1.z - mr[3]), (float)((double)a1.w - mi[3]));
+    }
+    amax = fmaxf(amax, fmaxf(fmaxf(fabsf(o0.x), fabsf(o0.y)), fmaxf(fabsf(o0.z), fabsf(o0.w))));
+    amax = fmaxf(amax, fmaxf(fmaxf(fabsf(o1.x), fabsf(o1.y)), fmaxf(fabsf(o1.z), fabsf(o1.w))));
+    const long long o = seg + slot * pitch;  // element of cell c0, a multiple of 4
+    if (!(DSB_INB(slot, dep, A.status) && DSB_INB(c0 + 3, pitch, A.status))) return;
+    if constexpr (BF16) {
+      reinterpret_cast<uint4*>(A.D)[o / 4] =
+          make_uint4(bf16_pair(o0.x, o0.y), bf16_pair(o0.z, o0.w), bf16_pair(o1.x, o1.y),
+                     bf16_pair(o1.z, o1.w));
+    } else {
+      float4* D4 = reinterpret_cast<float4*>(A.D);
+      D4[o / 2] = o0;
+      D4[o / 2 + 1] = o1;
+    }
+  };
+
+  if constexpr (CHUNK) {
+    constexpr int KT = S1_TT / L;
+    static_assert(KT <= 4, "a thread's sums stay in registers");
+    const int lane = tid & 31, warp = tid >> 5;
+    const int n_ch = (ceff + A.sbc - 1) / A.sbc;
+    const int n_items = (A.n_t + S1_TT - 1) / S1_TT * n_ch;   // (tile, subbands)
+    auto load = [&](int item) {
+      const int tt = item / n_ch * S1_TT, s0 = item % n_ch * A.sbc;
+      const int w0 = (item & 1) * A.sbc;
+      for (int q = warp; q < min(A.sbc, ceff - s0); q += S1_THREADS / 32) {
+        const int sb = s0 + q;
+        for (int tau = lane; tau < s_len[sb]; tau += 32) {
+          const long long r2 = ((((A.t0 + tt + s_lo[sb] + tau) & A.y_mask) * A.y_rows) + ycol +
+                                (long long)sb * pitch) / 2;
+          if (!DSB_INB(r2 + 1, (A.y_mask + 1) * A.y_rows / 2, A.status)) continue;
+          const int e = (w0 + q) * A.win_len + tau;
+          cp_async16(win0 + e, Y4 + r2);
+          cp_async16(win1 + e, Y4 + r2 + 1);
+        }
+      }
+      cp_async_commit();
+    };
+    float4 acc[KT][2];
+    __syncthreads();   // the shift tables
+    load(0);
+    for (int item = 0; item < n_items; ++item) {
+      const int tt = item / n_ch * S1_TT, ch = item % n_ch, s0 = ch * A.sbc;
+      if (item + 1 < n_items) {
+        load(item + 1);
+        cp_async_wait<1>();
+      } else {
+        cp_async_wait<0>();
+      }
+      __syncthreads();
+      if (active) {
+        if (ch == 0) {
 #pragma unroll
-        for (int q = 0; q < U; ++q) {
-          const int e = e0 + q * S1_THREADS + tid;
-          ei[q] = -1;
-          if (e < n_e) {
-            const int sb = e / A.win_len, tau = e - sb * A.win_len;
-            if (tau < s_len[sb]) {
-              const long long r2 = ((((A.t0 + tt + s_lo[sb] + tau) & A.y_mask) * A.y_rows) +
-                                    ycol + (long long)sb * pitch) / 2;
-              if (DSB_INB(r2 + 1, (A.y_mask + 1) * A.y_rows / 2, A.status)) {
-                v0[q] = Y4[r2];
-                v1[q] = Y4[r2 + 1];
-                ei[q] = e;
+          for (int k = 0; k < KT; ++k) acc[k][0] = acc[k][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        const int w0 = (item & 1) * A.sbc;
+        for (int q = 0; q < min(A.sbc, ceff - s0); ++q) {
+          const int idx = (w0 + q) * A.win_len + ln + s_sh[(s0 + q) * DG + dl];
+#pragma unroll
+          for (int k = 0; k < KT; ++k) {
+            acc[k][0] = f4_add(acc[k][0], win0[idx + L * k]);
+            acc[k][1] = f4_add(acc[k][1], win1[idx + L * k]);
+          }
+        }
+        if (ch == n_ch - 1) {
+          long long slot = (A.t0 + tt + ln + sh2) % dep;
+          if (slot < 0) slot += dep;
+#pragma unroll
+          for (int k = 0; k < KT; ++k, slot += L) {
+            if (slot >= dep) slot -= dep;
+            if (tt + ln + L * k < A.n_t) emit(acc[k][0], acc[k][1], slot);
+          }
+        }
+      }
+      __syncthreads();   // the windows just read are the next item's target
+    }
+  } else {
+    for (int tt = 0; tt < A.n_t; tt += S1_TT) {
+      __syncthreads();  // the previous tile's windows are no longer read
+      // stage the windows: entry (sb, tau) = Y at time t0 + tt + lo[sb] + tau,
+      // flattened over (sb, tau) so that each thread's loads are independent
+      {
+        constexpr int U = 4;
+        const int n_e = ceff * A.win_len;
+        for (int e0 = 0; e0 < n_e; e0 += U * S1_THREADS) {
+          float4 v0[U], v1[U];
+          int ei[U];
+#pragma unroll
+          for (int q = 0; q < U; ++q) {
+            const int e = e0 + q * S1_THREADS + tid;
+            ei[q] = -1;
+            if (e < n_e) {
+              const int sb = e / A.win_len, tau = e - sb * A.win_len;
+              if (tau < s_len[sb]) {
+                const long long r2 = ((((A.t0 + tt + s_lo[sb] + tau) & A.y_mask) * A.y_rows) +
+                                      ycol + (long long)sb * pitch) / 2;
+                if (DSB_INB(r2 + 1, (A.y_mask + 1) * A.y_rows / 2, A.status)) {
+                  v0[q] = Y4[r2];
+                  v1[q] = Y4[r2 + 1];
+                  ei[q] = e;
+                }
               }
             }
           }
-        }
 #pragma unroll
-        for (int q = 0; q < U; ++q) {
-          if (ei[q] >= 0) {
-            win0[ei[q]] = v0[q];
-            win1[ei[q]] = v1[q];
+          for (int q = 0; q < U; ++q) {
+            if (ei[q] >= 0) {
+              win0[ei[q]] = v0[q];
+              win1[ei[q]] = v1[q];
+            }
           }
         }
       }
-    }
-    __syncthreads();
-    if (!active) continue;
-    long long slot = (A.t0 + tt + ln + sh2) % dep;
-    if (slot < 0) slot += dep;
-    for (int k = 0; k < S1_TT / L; ++k, slot += L) {
-      if (slot >= dep) slot -= dep;
-      const int tl = ln + L * k;
-      if (tt + tl >= A.n_t) break;
-      float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f), a1 = a0;
-      for (int sb = 0; sb < ceff; ++sb) {
-        const int idx = sb * A.win_len + tl + s_sh[sb * DG + dl];
-        const float4 v0 = win0[idx], v1 = win1[idx];
-        a0 = f4_add(a0, v0);  // packed pairs: 4 adds instead of 8
-        a1 = f4_add(a1, v1);
-      }
-      sr[0] += a0.x; si[0] += a0.y; sr[1] += a0.z; si[1] += a0.w;
-      sr[2] += a1.x; si[2] += a1.y; sr[3] += a1.z; si[3] += a1.w;
-      float4 o0 = a0, o1 = a1;
-      if (sub) {
-        o0 = make_float4((float)((double)a0.x - mr[0]), (float)((double)a0.y - mi[0]),
-                         (float)((double)a0.z - mr[1]), (float)((double)a0.w - mi[1]));
-        o1 = make_float4((float)((double)a1.x - mr[2]), (float)((double)a1.y - mi[2]),
-                         (float)((double)a1.z - mr[3]), (float)((double)a1.w - mi[3]));
-      }
-      amax = fmaxf(amax, fmaxf(fmaxf(fabsf(o0.x), fabsf(o0.y)), fmaxf(fabsf(o0.z), fabsf(o0.w))));
-      amax = fmaxf(amax, fmaxf(fmaxf(fabsf(o1.x), fabsf(o1.y)), fmaxf(fabsf(o1.z), fabsf(o1.w))));
-      const long long o = seg + slot * pitch;  // element of cell c0, a multiple of 4
-      if (!(DSB_INB(slot, dep, A.status) && DSB_INB(c0 + 3, pitch, A.status))) continue;
-      if constexpr (BF16) {
-        reinterpret_cast<uint4*>(A.D)[o / 4] =
-            make_uint4(bf16_pair(o0.x, o0.y), bf16_pair(o0.z, o0.w), bf16_pair(o1.x, o1.y),
-                       bf16_pair(o1.z, o1.w));
-      } else {
-        float4* D4 = reinterpret_cast<float4*>(A.D);
-        D4[o / 2] = o0;
-        D4[o / 2 + 1] = o1;
+      __syncthreads();
+      if (!active) continue;
+      long long slot = (A.t0 + tt + ln + sh2) % dep;
+      if (slot < 0) slot += dep;
+      for (int k = 0; k < S1_TT / L; ++k, slot += L) {
+        if (slot >= dep) slot -= dep;
+        const int tl = ln + L * k;
+        if (tt + tl >= A.n_t) break;
+        float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f), a1 = a0;
+        for (int sb = 0; sb < ceff; ++sb) {
+          const int idx = sb * A.win_len + tl + s_sh[sb * DG + dl];
+          const float4 v0 = win0[idx], v1 = win1[idx];
+          a0 = f4_add(a0, v0);  // packed pairs: 4 adds instead of 8
+          a1 = f4_add(a1, v1);
+        }
+        emit(a0, a1, slot);
       }
     }
   }
@@ -707,17 +786,30 @@ int dsb_stage1_rows(const void* Y, long long y_rows, long long y_mask, int n_blo
   A.t0 = t0; A.n_t = n_t; A.n_dm = n_dm; A.ceff = ceff; A.win_len = win_len;
   A.sky_ring = (double2*)sky_ring; A.sky_window = sky_window; A.sky_head = sky_head;
   A.sky_count = sky_count; A.sky_subtract = sky_subtract; A.status = status;
+  // chunks where the whole windows leave room for one CTA per SM only (and
+  // a DM group narrow enough to keep its sums in registers): as many subbands
+  // as two buffers in half an SM hold, at most one per warp
+  size_t bytes = smem;
+  const size_t tables = s1_smem_bytes(ceff, dm_group, 0), per_sb = (size_t)2 * win_len * 32;
+  if (dm_group <= 16 && smem > 113 * 1024 && tables + per_sb <= 113 * 1024) {
+    A.sbc = (int)std::min<size_t>(S1_THREADS / 32, (113 * 1024 - tables) / per_sb);
+    A.sbc = std::min(A.sbc, ceff);
+    bytes = tables + (size_t)A.sbc * per_sb;
+  }
   auto pick = [&](auto bf) {
     constexpr bool B = decltype(bf)::value;
-    return dm_group == 32 ? stage1_rows_kernel<B, 32>
-         : dm_group == 16 ? stage1_rows_kernel<B, 16> : stage1_rows_kernel<B, 8>;
+    if (A.sbc)
+      return dm_group == 16 ? stage1_rows_kernel<B, 16, true> : stage1_rows_kernel<B, 8, true>;
+    return dm_group == 32   ? stage1_rows_kernel<B, 32, false>
+           : dm_group == 16 ? stage1_rows_kernel<B, 16, false>
+                            : stage1_rows_kernel<B, 8, false>;
   };
   auto kern = d_bf16 ? pick(std::true_type{}) : pick(std::false_type{});
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) !=
       cudaSuccess)
     return DSB_E_CUDA;
   dim3 grid(n_blocks, (n_dm + dm_group - 1) / dm_group);
-  kern<<<grid, S1_THREADS, smem, stream>>>(A);
+  kern<<<grid, S1_THREADS, bytes, stream>>>(A);
   return launch_status();
 }
 

@@ -663,8 +663,9 @@ __global__ void __launch_bounds__(ImgGeom<N>::THREADS, ImgGeom<N>::CTAS)
       // with a factor from a table in shared memory (exact for the quarter
       // turns, so only N = 512 rounds there).  No branch depends on an
       // entry: absent entries are zeros with q = 0 that end no slot, and a
-      // slot's store is predicated.  (A branch-free copy of the loop per
-      // pass, and a branch per ended slot: FOLD_TIME.)
+      // slot's store is predicated.  (A copy of the loop per pass with a
+      // branch per ended slot: 2031 us per 2304 images of 512^2 against 2011,
+      // 463 per 2176 of 256^2 against 450.)
       {
         const float2* rot = s_rot + p * FOLD;
         const uint32_t buf32 = smem_u32(buf);
