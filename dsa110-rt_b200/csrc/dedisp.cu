@@ -437,6 +437,9 @@ constexpr int S1_THREADS = 256;
 constexpr int S1_MAX_C = 64;
 constexpr int S1_TT = 64;   // output times per tile
 constexpr int S1_DG = 32;   // largest DM group (coarse DMs per CTA)
+// CTAs per SM of the chunked form with 8 DMs (80 registers): the 312 CTAs of
+// the small configuration then run in one wave (two per SM: 245 us, not 190)
+constexpr int S1_CHUNK_CTAS8 = 3;
 
 __host__ __device__ inline size_t s1_smem_bytes(int ceff, int dg, int win_len) {
   return (size_t)ceff * dg * 4 + (size_t)S1_MAX_C * 8 + (size_t)ceff * win_len * 32 + 16;
@@ -446,10 +449,11 @@ __host__ __device__ inline size_t s1_smem_bytes(int ceff, int dg, int win_len) {
 // coarse DMs over a wide range: the small plain configuration's 8 DMs of 600
 // pc cm^-3 / 32 need 219 KB), the subbands are staged A.sbc at a time in two
 // buffers, the next ones copied under the current ones' sums, which stay in
-// registers: two CTAs per SM and no exposed load.  300 -> 245 us per block of
+// registers: several CTAs per SM and no exposed load.  300 -> 190 us per block of
 // that configuration (512 times, 32 DMs, 314 cells).
 template <bool BF16, int DG, bool CHUNK>
-__global__ void __launch_bounds__(S1_THREADS) stage1_rows_kernel(const S1Args A) {
+__global__ void __launch_bounds__(S1_THREADS, CHUNK && DG == 8 ? S1_CHUNK_CTAS8 : 2)
+    stage1_rows_kernel(const S1Args A) {
   constexpr int L = S1_THREADS / DG;  // time lanes per DM
   static_assert(L >= 8 && L <= 32 && S1_TT % L == 0, "unsupported DM group");
   extern __shared__ __align__(16) uint8_t s1_smem[];
@@ -791,8 +795,9 @@ int dsb_stage1_rows(const void* Y, long long y_rows, long long y_mask, int n_blo
   // as two buffers in half an SM hold, at most one per warp
   size_t bytes = smem;
   const size_t tables = s1_smem_bytes(ceff, dm_group, 0), per_sb = (size_t)2 * win_len * 32;
-  if (dm_group <= 16 && smem > 113 * 1024 && tables + per_sb <= 113 * 1024) {
-    A.sbc = (int)std::min<size_t>(S1_THREADS / 32, (113 * 1024 - tables) / per_sb);
+  const size_t room = 227 * 1024 / (dm_group == 8 ? S1_CHUNK_CTAS8 : 2) - 1024;
+  if (dm_group <= 16 && smem > 113 * 1024 && tables + per_sb <= room) {
+    A.sbc = (int)std::min<size_t>(S1_THREADS / 32, (room - tables) / per_sb);
     A.sbc = std::min(A.sbc, ceff);
     bytes = tables + (size_t)A.sbc * per_sb;
   }
