@@ -311,8 +311,8 @@ struct ImgGeom {
   static constexpr bool META32 = (N == 512);
   // entry metadata fields: column | n' << NP_SH | q << Q_SH | last << LAST_SH
   // (32-bit form also: packed << ROT_SH | parity(u + w) << ROT_SH + 1)
-  [[maybe_unused]] static constexpr int NP_SH = META32 ? 8 : 7;
-  [[maybe_unused]] static constexpr int Q_SH = META32 ? 14 : 13;
+  static constexpr int NP_SH = META32 ? 8 : 7;
+  static constexpr int Q_SH = META32 ? 14 : 13;
   static constexpr int LAST_SH = META32 ? 17 : 15;
   static constexpr int ROT_SH = 18;
   static constexpr int CG = THREADS / C1;         // column groups
@@ -350,6 +350,7 @@ struct ImgGeom {
   static_assert(GM_BYTES % 16 == 0 && FC_BYTES % 16 == 0 && TS_BYTES % 16 == 0 &&
                     ROT_BYTES % 16 == 0,
                 "every table after gmeta starts 16-byte aligned");
+  static_assert(Q_SH > NP_SH && LAST_SH > Q_SH, "entry fields in order");
   static_assert(!META32 || ROT_SH == LAST_SH + 1,
                 "the 32-bit entry's rotation bits follow its last bit");
 };
