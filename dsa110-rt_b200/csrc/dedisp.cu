@@ -48,16 +48,20 @@ __global__ void grid_vis_kernel(const float2* __restrict__ vis, int n_fv, long l
 // lanes run over the sources of a row, which are consecutive in memory where
 // a baseline's subbands share a cell.  A warp then owns DPW DMs and its lanes
 // the times, so that the adds read consecutive 8-byte words (no bank
-// conflicts); the shared-memory pipe is what is left to bound it: 1.32 ms for
-// the same page.  Each cell's sources are added in CSR order, as before.
+// conflicts).  A batch is as many of the CTA's sources as fit, each in a
+// window of its own length, across cell ends: half as many batches as with
+// windows of the longest length and a batch end at each cell's (1.32 -> 0.98
+// ms for the same page).  What is left is the adds' shared-memory reads (0.73
+// ms without the copies) beside the copies (0.63 ms without the adds).  Each
+// cell's sources are added in CSR order, as before.
 constexpr int DV_TT = 64;        // output times per CTA
 constexpr int DV_CELLS = 4;      // cells per CTA (32 bytes of an output row)
 constexpr int DV_THREADS = 256;
 constexpr int DV_SLOTS = 6144;   // float2 slots of one window buffer (offsets fit 16 bits)
-constexpr int DV_MAXB = 96;      // sources per batch
+constexpr int DV_MAXB = 96;      // most sources of a batch
 constexpr int DV_MAX_C = 512;    // subbands whose shift tables fit
 
-// dynamic shared memory: two window buffers, two offset tables [source][DM],
+// dynamic shared memory: two window buffers, two offset tables [warp][source][its DMs],
 // the subbands' shifts relative to their smallest [subband][DM] and their
 // smallest and largest shift
 __host__ __device__ inline size_t dv_smem_bytes(int ceff, int dg) {
@@ -65,9 +69,8 @@ __host__ __device__ inline size_t dv_smem_bytes(int ceff, int dg) {
          (size_t)ceff * 8 + 16;
 }
 
-DSB_DEV void cp_async8(void* dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src)
-               : "memory");
+DSB_DEV void cp_async8(uint32_t dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
 }
 DSB_DEV void cp_async16(void* dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src)
@@ -88,19 +91,19 @@ __global__ void __launch_bounds__(DV_THREADS, 2)
   constexpr int DG = DPW * (DV_THREADS / 32);  // DMs per CTA
   constexpr int TPL = DV_TT / 32;              // times per lane
   extern __shared__ __align__(16) uint8_t dv_smem[];
-  __shared__ int s_w;                          // window pitch of a source
+  __shared__ int s_w, s_off[DV_CELLS + 1];     // the widest spread; the cells' sources
   float2* win = reinterpret_cast<float2*>(dv_smem);                    // [2][DV_SLOTS]
-  uint16_t* boff = reinterpret_cast<uint16_t*>(win + 2 * DV_SLOTS);    // [2][DV_MAXB][DG]
+  uint16_t* boff = reinterpret_cast<uint16_t*>(win + 2 * DV_SLOTS);    // [2][8][DV_MAXB][DPW]
   uint16_t* rel = boff + 2 * DV_MAXB * DG;                             // [ceff][DG]
   int* s_lo = reinterpret_cast<int*>(rel + (size_t)ceff * DG);         // [ceff]
   int* s_hi = s_lo + ceff;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int t0 = (int)(blockIdx.x % n_tiles) * DV_TT;
-  const int cell0 = (int)(blockIdx.x / n_tiles) * DV_CELLS;
   const int nt = min(DV_TT, t_dedisp - t0);
-  const int nc = min(DV_CELLS, n_filled - cell0);
   const int d0 = blockIdx.y * DG;
   const int nd = min(DG, n_dm - d0);
+  const int cell0 = (int)(blockIdx.x / n_tiles) * DV_CELLS;
+  const int nc = min(DV_CELLS, n_filled - cell0);
 
   // each subband's shift range over this CTA's DMs, and the window pitch:
   // the longest window, made odd so that lanes on consecutive sources write
@@ -123,8 +126,7 @@ __global__ void __launch_bounds__(DV_THREADS, 2)
   }
   atomicMax(&s_w, w_max);
   __syncthreads();
-  const int W = (s_w + DV_TT) | 1;
-  const int NB = min(DV_SLOTS / W, DV_MAXB);   // sources per batch; 0: the direct path
+  const bool windowed = s_w + DV_TT <= DV_SLOTS;
   const int c_end = cell0 + nc;
   float2 acc[DPW][TPL], res[DV_CELLS][DPW][TPL];
 #pragma unroll
@@ -139,95 +141,127 @@ __global__ void __launch_bounds__(DV_THREADS, 2)
       for (int h = 0; h < TPL; ++h) res[c][k][h] = make_float2(0.f, 0.f);
   auto finish = [&](int c) {
 #pragma unroll
+    for (int x = 0; x < DV_CELLS; ++x)
+      if (x == c)
+#pragma unroll
+        for (int k = 0; k < DPW; ++k)
+#pragma unroll
+          for (int h = 0; h < TPL; ++h) res[x][k][h] = acc[k][h];
+#pragma unroll
     for (int k = 0; k < DPW; ++k)
 #pragma unroll
-      for (int h = 0; h < TPL; ++h) {
-        res[c - cell0][k][h] = acc[k][h];
-        acc[k][h] = make_float2(0.f, 0.f);
-      }
+      for (int h = 0; h < TPL; ++h) acc[k][h] = make_float2(0.f, 0.f);
   };
   auto row_of = [&](long long r) {
     return r < n_prev ? prev + r * nsrc : cur + (r - n_prev) * nsrc;
   };
 
-  if (NB > 0) {
+  if (windowed) {
     for (int i = tid; i < ceff * DG; i += DV_THREADS) {
       const int sb = i / DG, d = i % DG;
       rel[i] = (uint16_t)(d < nd ? shifts[(long long)sb * n_dm + d0 + d] - s_lo[sb] : 0);
     }
+    if (tid <= DV_CELLS) s_off[tid] = off[min(cell0 + tid, c_end)];
     __syncthreads();
-    // batch (c, j): sources j .. j + NB - 1 of cell c (fewer at its end)
-    auto load = [&](int buf, int c, int j) {
-      const int nb = min(NB, off[c + 1] - j);
+    const int j_end = s_off[DV_CELLS];
+    auto src_at = [&](int j) { return j + lane < j_end ? __ldg(src + j + lane) : 0; };
+    int pre = src_at(s_off[0]);   // this lane's source of the next batch
+    // The batch that starts at source j: as many of the CTA's sources as fit
+    // the buffer, returned.  Every warp works out the same layout, a lane per
+    // source, copies its share of the rows and notes its own DMs' offsets.
+    auto load = [&](int buf, int j) {
       float2* wb = win + buf * DV_SLOTS;
-      int lo = 0x7fffffff, hi = -0x7fffffff;
-      for (int i = lane; i < nb; i += 32) {
-        const int sb = src[j + i] % ceff;
-        lo = min(lo, s_lo[sb]);
-        hi = max(hi, s_hi[sb]);
-      }
-      lo = __reduce_min_sync(0xffffffffu, lo);
-      hi = __reduce_max_sync(0xffffffffu, hi);
-      for (int i = tid & 15; i < nb; i += 16) {
-        const int sj = src[j + i], sb = sj % ceff;
-        const int l = s_lo[sb], n = s_hi[sb] - l + nt;   // rows t0 + l .. t0 + l + n - 1
-        for (int r = lo + (tid >> 4); r < hi + nt; r += DV_THREADS / 16) {
-          const int k = r - l;
-          if (k >= 0 && k < n) cp_async8(wb + i * W + k, row_of((long long)t0 + r) + sj);
+      uint16_t* bo = boff + (buf * (DV_THREADS / 32) + warp) * DV_MAXB * DPW;
+      int nb = 0, base0 = 0;
+      for (int ch = 0; ch < DV_MAXB; ch += 32) {
+        const int sj = ch ? src_at(j + ch) : pre, sb = sj % ceff;
+        const int l = s_lo[sb], spread = s_hi[sb] - l;
+        int n = spread + nt;   // rows t0 + l .. t0 + l + n - 1
+        // padded so that a row's copies by consecutive lanes meet in no bank
+        const int w = n + ((__shfl_down_sync(0xffffffffu, l, 1) - l + 1 - n) & 15);
+        int end = w;
+#pragma unroll
+        for (int o = 1; o < 32; o *= 2) {
+          const int v = __shfl_up_sync(0xffffffffu, end, o);
+          if (lane >= o) end += v;
         }
-      }
-      uint16_t* bo = boff + buf * DV_MAXB * DG;
-      for (int x = tid; x < nb * DG; x += DV_THREADS) {
-        const int i = x / DG;
-        bo[x] = (uint16_t)(i * W + rel[(src[j + i] % ceff) * DG + x % DG]);
+        const int base = base0 + end - w;
+        const bool fits = j + ch + lane < j_end && base + spread + DV_TT <= DV_SLOTS;
+        const int cnt = __popc(__ballot_sync(0xffffffffu, fits));
+        if (cnt == 0) break;
+        if (fits) {
+          if constexpr (DPW == 4) {   // no carry between the halves: offsets fit 16 bits
+            const uint2 d = *reinterpret_cast<const uint2*>(rel + sb * DG + warp * DPW);
+            const uint32_t b2 = (uint32_t)base * 0x10001u;
+            *reinterpret_cast<uint2*>(bo + (ch + lane) * DPW) = make_uint2(d.x + b2, d.y + b2);
+          } else {
+#pragma unroll
+            for (int k = 0; k < DPW; ++k)
+              bo[(ch + lane) * DPW + k] = (uint16_t)(base + rel[sb * DG + warp * DPW + k]);
+          }
+        }
+        if (!fits) n = 0;
+        const int lo = __reduce_min_sync(0xffffffffu, fits ? l : 0x7fffffff);
+        const int hi = __reduce_max_sync(0xffffffffu, fits ? l + n : -0x7fffffff);
+        const uint32_t dst = smem_u32(wb) + 8 * (base - l);
+        auto copy = [&](const float2* rows, int first, int last) {   // rows: that of shift 0
+          const float2* p = rows + (long long)first * nsrc + sj;
+          for (int r = first; r < last; r += DV_THREADS / 32, p += (DV_THREADS / 32) * nsrc)
+            if ((unsigned)(r - l) < (unsigned)n) cp_async8(dst + 8 * r, p);
+        };
+        const int in_prev = max(lo, min(hi, n_prev - t0));
+        copy(prev + (long long)t0 * nsrc, lo + warp, in_prev);
+        // the first of this warp's rows in cur
+        const int first = lo + warp + max(0, (in_prev - lo - warp + 7) / 8) * 8;
+        copy(cur + ((long long)t0 - n_prev) * nsrc, first, hi);
+        nb += cnt;
+        base0 += __shfl_sync(0xffffffffu, end, 31);
+        if (cnt < 32) break;
       }
       cp_async_commit();
+      pre = src_at(j + nb);
+      return nb;
     };
-    auto advance = [&](int& c, int& j) {   // to the next batch; c == c_end at the end
-      j += NB;
-      while (c < c_end && j >= off[c + 1]) {
-        ++c;
-        if (c < c_end) j = off[c];
-      }
-    };
-    int c = cell0, j = off[cell0] - NB;
-    advance(c, j);
-    int buf = 0;
-    if (c < c_end) load(0, c, j);
-    while (c < c_end) {
-      int cn = c, jn = j;
-      advance(cn, jn);
-      if (cn < c_end) {
-        load(buf ^ 1, cn, jn);
+    int j = s_off[0], buf = 0, cl = 0;
+    int nb = j < j_end ? load(0, j) : 0;
+    while (j < j_end) {
+      const int jn = j + nb;
+      int nbn = 0;
+      if (jn < j_end) {
+        nbn = load(buf ^ 1, jn);
         cp_async_wait<1>();
       } else {
         cp_async_wait<0>();
       }
       __syncthreads();
       if (warp * DPW < nd) {
-        const int nb = min(NB, off[c + 1] - j);
         const float2* wb = win + buf * DV_SLOTS + lane;
-        const uint16_t* bo = boff + buf * DV_MAXB * DG + warp * DPW;
+        const uint16_t* bo = boff + (buf * (DV_THREADS / 32) + warp) * DV_MAXB * DPW;
+        for (int i = 0;;) {
+          const int e = s_off[cl + 1] - j, stop = min(nb, e);
 #pragma unroll 2
-        for (int i = 0; i < nb; ++i) {
-          uint16_t o[DPW];
-          if constexpr (DPW == 4) {
-            const uint2 w = *reinterpret_cast<const uint2*>(bo + i * DG);
-            o[0] = (uint16_t)w.x; o[1] = (uint16_t)(w.x >> 16);
-            o[2] = (uint16_t)w.y; o[3] = (uint16_t)(w.y >> 16);
-          } else {
+          for (; i < stop; ++i) {
+            uint16_t o[DPW];
+            if constexpr (DPW == 4) {
+              const uint2 w = *reinterpret_cast<const uint2*>(bo + i * DPW);
+              o[0] = (uint16_t)w.x; o[1] = (uint16_t)(w.x >> 16);
+              o[2] = (uint16_t)w.y; o[3] = (uint16_t)(w.y >> 16);
+            } else {
 #pragma unroll
-            for (int k = 0; k < DPW; ++k) o[k] = bo[i * DG + k];
+              for (int k = 0; k < DPW; ++k) o[k] = bo[i * DPW + k];
+            }
+#pragma unroll
+            for (int k = 0; k < DPW; ++k)
+#pragma unroll
+              for (int h = 0; h < TPL; ++h) acc[k][h] = f2_add(acc[k][h], wb[o[k] + 32 * h]);
           }
-#pragma unroll
-          for (int k = 0; k < DPW; ++k)
-#pragma unroll
-            for (int h = 0; h < TPL; ++h) acc[k][h] = f2_add(acc[k][h], wb[o[k] + 32 * h]);
+          if (i < e) break;   // the cell goes on in the next batch
+          finish(cl);
+          if (++cl == nc) break;
         }
       }
-      if (cn != c) finish(c);
-      c = cn;
       j = jn;
+      nb = nbn;
       buf ^= 1;
       __syncthreads();   // the buffer just read is the next batch's target
     }
@@ -244,7 +278,7 @@ __global__ void __launch_bounds__(DV_THREADS, 2)
               acc[k][h] = f2_add(acc[k][h], row_of((long long)t0 + lane + 32 * h +
                                                    sh[warp * DPW + k])[sj]);
       }
-      finish(c);
+      finish(c - cell0);
     }
   }
   // four lanes exchange (cell, time) so that they write the 4 cells of one

@@ -51,14 +51,15 @@ def test_tiles(n_dm, t_d, n_filled):
 
 @pytest.mark.parametrize("n_dm", [3, 32])
 def test_cells_longer_than_a_batch(n_dm):
-    # pitch 64 + 300: 16 sources a batch; pitch 65: the 96-source cap
+    # windows of up to 64 + 300: a few tens of sources a batch; of 64: the
+    # 96-source cap
     _run(n_dm, 70, 6, ceff=5, nb=20, spread=300, per_cell=120, n_prev=200)
     _run(n_dm, 70, 6, ceff=5, nb=20, spread=0, per_cell=250, n_prev=0)
 
 
 @pytest.mark.parametrize("spread", [6078, 6081, 70000])
 def test_windows_wider_than_the_buffer(spread):
-    # 64 + 6078 | 1 = 6143 float2 is the widest staged window, beyond it the
+    # 64 + 6080 = 6144 float2 is the widest staged window, beyond it the
     # sources are read in place
     _run(9, 66, 5, ceff=2, nb=1, spread=spread, per_cell=3, n_prev=1000)
 
@@ -66,3 +67,11 @@ def test_windows_wider_than_the_buffer(spread):
 @pytest.mark.parametrize("ceff", [512, 513])
 def test_many_subbands(ceff):
     _run(5, 40, 5, ceff=ceff, nb=2, spread=11, per_cell=30, n_prev=20)
+
+
+@pytest.mark.parametrize("per_cell", [1, 31, 32, 33, 96, 97])
+@pytest.mark.parametrize("spread", [40, 6080])
+def test_batches_across_cells(per_cell, spread):
+    # batches that end inside, at and beyond cell ends, a lane of the layout
+    # per source
+    _run(5, 66, 9, ceff=4, nb=17, spread=spread, per_cell=per_cell, n_prev=30)
