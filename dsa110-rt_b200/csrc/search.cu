@@ -1157,6 +1157,34 @@ __global__ void __launch_bounds__(256, DetCfg<LOGW>::MINB)
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   // npix % 32 == 0, so inner is whole warps: a warp is in or out as a whole
   if (e >= inner) return;
+  const long long fidx = e / npix, p = e % npix;
+  const int p0 = (int)(p - lane);  // the warp's first cell (a multiple of 32)
+  const int total = n + MAXW;
+  const int warm_end = t_base + MAXW;
+  const int out_end = t_base + n_out + MAXW;
+  const int n_blk = (min(total, out_end) + DB - 1) / DB;
+  // block b holds inputs x[b DB - 1 - PL .. b DB + DB - 2 - PL]; a block with
+  // none inside the cube completes its phase with no copy (its inputs are
+  // never read)
+  // The first blocks' copies leave before the mask, the scales and the
+  // Layer-2 entries are loaded (558 -> 547 us for 8 fine DMs x 256 outputs of
+  // 512^2 at boxcars to 16: a CTA lives for some 25 us).
+  auto issue = [&](int b) {
+    uint64_t* bar = bars + b % DET_NST;
+    const int y0 = b * DB - 1 - PL;
+    if (y0 < n && y0 + DB > 0) {
+      mbar_arrive_expect_tx(bar, SB * 4);
+      tma_load_3d(stages + (b % DET_NST) * SB, &tmap, p0, y0, (int)fidx, bar);
+    } else {
+      mbar_arrive(bar);
+    }
+  };
+  if (lane == 0) {
+    for (int s = 0; s < DET_NST; ++s) mbar_init(bars + s, 1);
+    fence_mbar_init();
+    for (int b = 0; b < min(DET_NST - 1, n_blk); ++b) issue(b);
+  }
+  __syncwarp();
   int s_i = 0, s_end = 0, s_t = 0x7fffffff;
   const int eg = (int)e + pix_off;
   if (l2.out) {
@@ -1167,8 +1195,6 @@ __global__ void __launch_bounds__(256, DetCfg<LOGW>::MINB)
     s_i = lo;
     if (s_i < s_end && __ldg(&l2.ent[s_i].x) == eg) s_t = __ldg(&l2.ent[s_i].y);
   }
-  const long long fidx = e / npix, p = e % npix;
-  const int p0 = (int)(p - lane);  // the warp's first cell (a multiple of 32)
   float mval = mask ? mask[fidx * mask_f_stride + p] : 1.0f;
   if (sig_f) mval = mval / sig_f[fidx];
   float tau[K];
@@ -1186,29 +1212,6 @@ __global__ void __launch_bounds__(256, DetCfg<LOGW>::MINB)
   auto ring = [&](int i) -> float& { return (i & 1) ? rg[i >> 1].y : rg[i >> 1].x; };
   double run = 0.0;
   float last = 0.f;
-  const int total = n + MAXW;
-  const int warm_end = t_base + MAXW;
-  const int out_end = t_base + n_out + MAXW;
-  const int n_blk = (min(total, out_end) + DB - 1) / DB;
-  // block b holds inputs x[b DB - 1 - PL .. b DB + DB - 2 - PL]; a block with
-  // none inside the cube completes its phase with no copy (its inputs are
-  // never read)
-  auto issue = [&](int b) {
-    uint64_t* bar = bars + b % DET_NST;
-    const int y0 = b * DB - 1 - PL;
-    if (y0 < n && y0 + DB > 0) {
-      mbar_arrive_expect_tx(bar, SB * 4);
-      tma_load_3d(stages + (b % DET_NST) * SB, &tmap, p0, y0, (int)fidx, bar);
-    } else {
-      mbar_arrive(bar);
-    }
-  };
-  if (lane == 0) {
-    for (int s = 0; s < DET_NST; ++s) mbar_init(bars + s, 1);
-    fence_mbar_init();
-    for (int b = 0; b < min(DET_NST - 1, n_blk); ++b) issue(b);
-  }
-  __syncwarp();
   // the screen, the threshold hits and the Layer-2 samples of one output
   // from its boxcar sums
   auto decide = [&](const BoxSums<K>& d, int ta, auto with_samples) {
