@@ -710,7 +710,9 @@ __global__ void __launch_bounds__(ImgGeom<N>::THREADS, ImgGeom<N>::CTAS)
         unsigned ma[8];
         if constexpr (Gm::META32) {
           uint32_t rb[16];
-          tmem_ld16(tbase, ra);
+          // (a warp without entries loads nothing: every load is waited for
+          // before its registers or tensor memory have another use)
+          if (nch > 0) tmem_ld16(tbase, ra);
           for (int c = 0; c < nch; c += 2) {
             tmem_ld_wait16(ra);
             if (c + 1 < nch) tmem_ld16(tbase + 16 * (c + 1), rb);
