@@ -434,7 +434,10 @@ __global__ void __launch_bounds__(ImgGeom<N>::THREADS, ImgGeom<N>::CTAS)
     rot32 = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint8_t*>(A.gmeta) +
                                                  Gm::GM_BYTES + Gm::FC_BYTES + Gm::TS_BYTES) +
                   tid);
-  const int nch = (__reduce_max_sync(0xffffffffu, sn) + 7) >> 3;  // 8-entry chunks, per warp
+  // 8-entry chunks, per warp.  The 32-bit form's fold loads a warp's first
+  // chunk ahead of its loop, so there every warp has one (of zeros where it
+  // owns no entry): no tensor-memory load is left without its wait.
+  const int nch = (max(Gm::META32 ? 1 : 0, __reduce_max_sync(0xffffffffu, sn)) + 7) >> 3;
   if (warp == 0) {
     tmem_alloc(s_tmem, Gm::TMEM_COLS);
     tmem_relinquish();
@@ -457,7 +460,12 @@ __global__ void __launch_bounds__(ImgGeom<N>::THREADS, ImgGeom<N>::CTAS)
   auto load_tables = [&] {
     const uint8_t* gt = reinterpret_cast<const uint8_t*>(A.gmeta) + Gm::GM_BYTES;
     const uint32_t* g_code = reinterpret_cast<const uint32_t*>(gt);
-    for (int c = 0; c < nch; ++c) s_code[c * THREADS + tid] = __ldg(g_code + c * THREADS + tid);
+    for (int c = 0; c < nch; ++c) {
+      // nibbles past this thread's entries end no slot, whatever the table has
+      const int keep = max(0, sn - 8 * c);
+      s_code[c * THREADS + tid] = __ldg(g_code + c * THREADS + tid) &
+                                  (keep < 8 ? (1u << (4 * keep)) - 1u : 0xffffffffu);
+    }
     const uint4* g_slot =
         reinterpret_cast<const uint4*>(gt + Gm::FC_BYTES + Gm::TS_BYTES + Gm::ROT_BYTES);
     uint4* s_slot4 = reinterpret_cast<uint4*>(s_code + Gm::MAXC * THREADS);
@@ -663,10 +671,10 @@ __global__ void __launch_bounds__(ImgGeom<N>::THREADS, ImgGeom<N>::CTAS)
       // Entry q of a slot turns by W_FOLD^(q p): one complex multiply-add
       // with a factor from a table in shared memory (exact for the quarter
       // turns, so only N = 512 rounds there).  No branch depends on an
-      // entry: absent entries are zeros with q = 0 that end no slot, and a
-      // slot's store is predicated.  (A copy of the loop per pass with a
-      // branch per ended slot: 2031 us per 2304 images of 512^2 against 2011,
-      // 463 per 2176 of 256^2 against 450.)
+      // entry: absent entries are zeros that end no slot, whatever their table
+      // entries hold, and a slot's store is predicated.  (A copy of the loop
+      // per pass with a branch per ended slot: 2031 us per 2304 images of
+      // 512^2 against 2011, 463 per 2176 of 256^2 against 450.)
       {
         const float2* rot = s_rot + p * FOLD;
         const uint32_t buf32 = smem_u32(buf);
@@ -698,10 +706,11 @@ __global__ void __launch_bounds__(ImgGeom<N>::THREADS, ImgGeom<N>::CTAS)
               entry(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]), code & 7u, last, off);
             }
           } else {
+            constexpr unsigned LAST = 1u << Gm::LAST_SH;
 #pragma unroll
             for (int j = 0; j < 8; ++j)
               entry(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]),
-                    (m[j] >> Gm::Q_SH) & (FOLD - 1), (m[j] >> Gm::LAST_SH) & 1u,
+                    (m[j] >> Gm::Q_SH) & (FOLD - 1), (m[j] & LAST) != 0u && j < sn - 8 * c,
                     ((m[j] >> Gm::NP_SH) & (LC - 1)) * P + (m[j] & (NC - 1)));
           }
         };
@@ -710,9 +719,7 @@ __global__ void __launch_bounds__(ImgGeom<N>::THREADS, ImgGeom<N>::CTAS)
         unsigned ma[8];
         if constexpr (Gm::META32) {
           uint32_t rb[16];
-          // (a warp without entries loads nothing: every load is waited for
-          // before its registers or tensor memory have another use)
-          if (nch > 0) tmem_ld16(tbase, ra);
+          tmem_ld16(tbase, ra);
           for (int c = 0; c < nch; c += 2) {
             tmem_ld_wait16(ra);
             if (c + 1 < nch) tmem_ld16(tbase + 16 * (c + 1), rb);

@@ -1,7 +1,9 @@
-"""dsb_image_fft on hand-made patterns: so few half cells that whole warps of
-the kernel own no entry, against the Hermitian half spectrum and numpy's
-irfft2 in float64."""
+"""dsb_image_fft on hand-made patterns, against the Hermitian half spectrum and
+numpy's irfft2 in float64: so few half cells that whole warps of the kernel
+own no entry, and tables whose unused entries hold anything (a caller's own
+tables: the header gives only the entries in a thread's range a meaning)."""
 
+import copy
 import types
 
 import numpy as np
@@ -94,3 +96,25 @@ def test_images_of_few_half_cells(N, n_cells, n_g, fftshift):
     want = _reference(pats, cells, N, fftshift)
     # float32 transforms: 2e-6 of the largest pixel, as for the streaming ring
     assert np.abs(got - want).max() <= 2e-6 * np.abs(want).max()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("N,n_cells,n_g", [(512, 300, 2), (512, 2500, 3), (256, 700, 2),
+                                           (64, 120, 3)])
+def test_unused_table_entries_may_hold_anything(N, n_cells, n_g):
+    rng, pats, cells = _case(N, n_cells, n_g, 2)
+    T = build_image_tables(pats, N)
+    want = _images(T, pats, cells, N, 9, True)
+    U = copy.deepcopy(T)
+    cnt = np.diff(T.thr_b)
+    epv = T.gmeta.shape[2]
+    i = (np.arange(T.gmeta.shape[0])[:, None, None] * epv + np.arange(epv)[None, None, :])
+    unused = i >= cnt[None, :, None]
+    assert unused.any()
+    U.gmeta[unused] = rng.integers(0, np.iinfo(U.gmeta.dtype).max, int(unused.sum()))
+    if T.fold_code is not None:
+        for c in range(T.fold_code.shape[0]):
+            keep = np.clip(cnt - 8 * c, 0, 8)
+            used = ((np.uint64(1) << (4 * keep).astype(np.uint64)) - np.uint64(1)).astype(np.uint32)
+            U.fold_code[c] |= ~used & rng.integers(0, 1 << 32, cnt.size).astype(np.uint32)
+    np.testing.assert_array_equal(_images(U, pats, cells, N, 9, True), want)
