@@ -651,6 +651,25 @@ __global__ void __launch_bounds__(CS_THREADS) combine_sparse_kernel(
   }
 }
 
+// Whether two tables differ: each read once, 16 bytes per access where both
+// start on that boundary (n16 words; the rest by bytes).
+__global__ void __launch_bounds__(256) tables_differ_kernel(const uint8_t* __restrict__ a,
+                                                            const uint8_t* __restrict__ b,
+                                                            long long n16, long long n_bytes,
+                                                            int* __restrict__ differ) {
+  const long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long step = (long long)gridDim.x * blockDim.x;
+  uint32_t d = 0u;
+#pragma unroll 4
+  for (long long i = i0; i < n16; i += step) {
+    const uint4 x = __ldg(reinterpret_cast<const uint4*>(a) + i);
+    const uint4 y = __ldg(reinterpret_cast<const uint4*>(b) + i);
+    d |= (x.x ^ y.x) | (x.y ^ y.y) | (x.z ^ y.z) | (x.w ^ y.w);
+  }
+  for (long long i = 16 * n16 + i0; i < n_bytes; i += step) d |= (uint32_t)(a[i] ^ b[i]);
+  if (d) *differ = 1;
+}
+
 // ===========================================================================
 // padded cumsum / boxcars (detector/forward.py:250-455,
 // detector/triton_boxcar.py:47-360).  Each prefix is accumulated in float64
@@ -1655,6 +1674,19 @@ int dsb_combine_sparse(const void* dense, const int* cell_uw, const int* cell_pt
         static_cast<const int16_t*>(dense), cell_uw, cell_ptr, ent_g, ent_k, ent_km, shifts, out,
         n_act, n_sb, t_rows, t_pad, n_filled_max, N, n_fdm, t_out_len, t_lo, fftshift, out_rows,
         out_row0, status);
+  return launch_status();
+}
+
+int dsb_tables_differ(const void* a, const void* b, long long n_bytes, int* differ,
+                      cudaStream_t stream) {
+  if (!a || !b || !differ || n_bytes < 0) return DSB_E_ARG;
+  if (n_bytes == 0) return DSB_OK;
+  const bool vec = ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15) == 0;
+  const long long n16 = vec ? n_bytes / 16 : 0, n = std::max(n16, n_bytes - 16 * n16);
+  const unsigned blocks = (unsigned)std::min<long long>((n + 255) / 256, 148 * 8);
+  tables_differ_kernel<<<blocks, 256, 0, stream>>>(static_cast<const uint8_t*>(a),
+                                                   static_cast<const uint8_t*>(b), n16, n_bytes,
+                                                   differ);
   return launch_status();
 }
 

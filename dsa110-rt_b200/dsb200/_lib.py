@@ -66,6 +66,7 @@ _SIGNATURES = {
     "dsb_combine_sparse": [_vp, _vp, _vp, _vp, _vp, _vp, _c_int, _vp, _vp, _c_int, _c_int,
                            _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int,
                            _c_int, _c_int, _vp, _vp],
+    "dsb_tables_differ": [_vp, _vp, _c_ll, _vp, _vp],
     "dsb_encode_rows": [_vp, _c_ll, _c_int, _c_int, _c_int, _vp, _vp, _vp],
     "dsb_cluster_mst": [_vp, _c_int, _c_int, _c_int, _vp, _vp],
     "dsb_cal_apply": [_vp, _vp, _vp, _vp, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int,
@@ -160,7 +161,10 @@ def status_word(dev: torch.device) -> torch.Tensor:
 
 
 def check_status(status: torch.Tensor, what: str) -> None:
-    code = int(status.item())
+    check_status_code(int(status.item()), what)
+
+
+def check_status_code(code: int, what: str) -> None:
     if code != 0:
         msg = lib().dsb_strerror(code).decode()
         raise DsbError(f"{what}: device status {msg} (code {code})")

@@ -507,11 +507,16 @@ class GpuImager:
                              "calibration needs the dense combine")
         if t_stream < cfg.t_det:
             raise ValueError(f"compact_t_stream={t_stream} < T_det={cfg.t_det}")
-        key = (int(inv_lut.data_ptr()), tuple(inv_lut.shape), N)
-        if getattr(self, "_csr_key", None) != key:
-            self._csr = build_sparse_cell_csr(inv_lut, n_grid=N)
-            self._csr_key = key
-        st = _lib.status_word(self.device)
+
+        def combine(csr, st):
+            for f0, n_f, t0, nt, work in self._chunks(t_lo, full):
+                work.zero_()
+                _combine_sparse(streams, csr, shifts[f0:f0 + n_f], t_rows=t_stream, t_out_len=nt,
+                                t_lo=t0, fftshift=True, out=work, out_row0=0, status=st)
+                if cfg.imager_uv_prescale != 1.0:
+                    work.mul_(cfg.imager_uv_prescale)
+                self._transform_to_cube(work, n_f, nt, cube, f0, t0)
+
         full = getattr(self, "_uv_full", None)
         if full is None:
             # every image at once: the combine stages each stream row once for
@@ -519,13 +524,28 @@ class GpuImager:
             # 256^2, against 0.85 ms in chunks of 48 MB)
             full = self._uv_full = torch.empty((cfg.n_fdm * cfg.t_det, N, N // 2 + 1),
                                                dtype=torch.complex64, device=self.device)
-        for f0, n_f, t0, nt, work in self._chunks(t_lo, full):
-            work.zero_()
-            _combine_sparse(streams, self._csr, shifts[f0:f0 + n_f], t_rows=t_stream,
-                            t_out_len=nt, t_lo=t0, fftshift=True, out=work, out_row0=0, status=st)
-            if cfg.imager_uv_prescale != 1.0:
-                work.mul_(cfg.imager_uv_prescale)
-            self._transform_to_cube(work, n_f, nt, cube, f0, t0)
+        # The CSR is kept with a copy of the table it was built from.  Whether
+        # the table still holds the same values is decided on the device, after
+        # the images, and read with their status (no further wait): a table may
+        # be rewritten in place, or another come to lie at its address.
+        held = getattr(self, "_lut_csr", None)
+        if held is not None and inv_lut.is_cuda and \
+                (held[0].shape, held[0].dtype, held[0].device) == \
+                (inv_lut.shape, inv_lut.dtype, inv_lut.device):
+            st = torch.zeros(2, dtype=torch.int32, device=self.device)   # status, changed
+            combine(held[1], st)
+            lut = inv_lut.contiguous()
+            _lib.check(_lib.lib().dsb_tables_differ(
+                _lib.ptr(held[0]), _lib.ptr(lut), lut.numel() * lut.element_size(),
+                _lib.ptr(st[1:]), _lib.stream_of(self.device)), "dsb_tables_differ")
+            both = int(st.view(torch.int64).item())    # one word to read
+            if not both >> 32:
+                _lib.check_status_code(both, "dsb_combine_sparse")
+                return cube
+        lut = inv_lut.detach().clone(memory_format=torch.contiguous_format)
+        self._lut_csr = (lut, build_sparse_cell_csr(lut, n_grid=N))
+        st = _lib.status_word(self.device)
+        combine(self._lut_csr[1], st)
         _lib.check_status(st, "dsb_combine_sparse")
         return cube
 

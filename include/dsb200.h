@@ -266,6 +266,13 @@ int dsb_combine_sparse(const void* dense, const int* cell_uw, const int* cell_pt
                        int t_pad, int n_filled_max, int N, int n_fdm, int t_out_len, int t_lo,
                        int fftshift, int out_rows, int out_row0, int* status,
                        cudaStream_t stream);
+
+/* *differ = 1 if the n_bytes bytes at a and b differ anywhere (else *differ
+ * is left alone): whether the table a kept CSR was built from is still the
+ * caller's.  No counterpart in the reference (its caller keeps the CSR). */
+int dsb_tables_differ(const void* a, const void* b, long long n_bytes, int* differ,
+                      cudaStream_t stream);
+
 int dsb_combine_dense(const void* streams, const int* shifts, const float* scales,
                       const float* off_re, const float* off_im, int per_t, void* out,
                       int out_f16, int half,
