@@ -303,10 +303,22 @@ def irfft2_image(half: torch.Tensor, n_grid: int, out: Optional[torch.Tensor] = 
     return out
 
 
+_CUBE_DTYPES = (torch.float16, torch.float32)
+
+
+def _require_pixels(t: torch.Tensor, name: str, dtypes=_CUBE_DTYPES) -> None:
+    """A contiguous CUDA tensor whose type the kernels know: they would read or
+    write any other's pixels at the wrong width (bfloat16's past the end)."""
+    if isinstance(t, torch.Tensor) and t.dtype not in dtypes:
+        raise ValueError(f"{name} dtype {t.dtype} not in {dtypes}")
+    _lib.require_cuda(t, name)
+
+
 def mask_into_cube(img: torch.Tensor, mask: torch.Tensor, cube: torch.Tensor, f0: int) -> None:
     """``cube[t, f0+f, :, :] = img[f, t] * mask[(f,)]`` (imager_gpu.py:604-650)."""
-    _lib.require_cuda(img, "img")
-    _lib.require_cuda(cube, "cube")
+    _require_pixels(img, "img", (torch.float32,))
+    _require_pixels(mask, "mask", (torch.float32,))
+    _require_pixels(cube, "cube")
     n_f, n_t, H, W = img.shape
     per_f = int(mask.ndim == 3)
     _lib.check(_lib.lib().dsb_mask_to_cube(
@@ -365,6 +377,8 @@ class GpuImager:
         """Allocate the persistent buffers and the edge mask (no compute)."""
         if config.complex_dtype != torch.complex64:
             raise ValueError("this imager transforms in float32: complex_dtype must be complex64")
+        if config.cube_dtype not in _CUBE_DTYPES:
+            raise ValueError(f"cube_dtype {config.cube_dtype} not in {_CUBE_DTYPES}")
         dev = config.resolved_device()
         N = config.n_grid
         edge = compute_edge_mask(n_grid=N, kernel_support=config.kernel_support,
@@ -483,6 +497,8 @@ class GpuImager:
         N = self.config.n_grid
         per_f = self.edge_mask_per_fdm is not None
         mask = self.edge_mask_per_fdm[f0:f0 + n_f] if per_f else self.edge_mask_real
+        _require_pixels(mask, "edge mask", (torch.float32,))
+        _require_pixels(cube, "output cube")
         _lib.check(_lib.lib().dsb_irfft2_cube(
             _lib.ptr(work), n_t * N * (N // 2 + 1), n_f, n_t, N,
             _lib.ptr(twiddles(N, self.device)), _lib.ptr(mask), int(per_f), _lib.ptr(cube[t0:]),
@@ -773,7 +789,7 @@ def detect_cube(cube: torch.Tensor, *, log_max_width: int, sigma_inv: torch.Tens
     """Fused padded-cumsum boxcars (widths 1..2**log_max_width), max over
     widths and threshold compaction on a ``[T, F, H, W]`` cube; candidate
     ``pix`` is the flat ``(f, h, w)`` index plus ``pix_offset``."""
-    _lib.require_cuda(cube, "cube")
+    _require_pixels(cube, "cube")
     n = cube.shape[0]
     inner = cube[0].numel()
     _lib.check(_lib.lib().dsb_detect(_lib.ptr(cube), int(cube.dtype == torch.float16), n, 1,
@@ -794,8 +810,8 @@ def detect_images(img: torch.Tensor, mask: torch.Tensor, *, log_max_width: int,
     all) and divided by ``sigma_f[F]`` (the Layer-1 sigma) when given.  With
     ``layer2`` the detector also writes that object's per-kernel score
     samples of these fine DMs (``pix_offset`` = first fine DM x H x W)."""
-    _lib.require_cuda(img, "img")
-    _lib.require_cuda(mask, "mask")
+    _require_pixels(img, "img")
+    _require_pixels(mask, "mask", (torch.float32,))
     F, T, H, W = img.shape
     npix = H * W
     if mask.numel() not in (npix, F * npix):
