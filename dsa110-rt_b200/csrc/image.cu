@@ -1033,18 +1033,42 @@ __global__ void __launch_bounds__(DenseGeom<N>::COL_THREADS)
 // detector cube [t][f][N][N] times a mask (one, or one per fine DM).
 struct DenseOut {
   float* img;
-  int img_vec;             // img starts on a 16-byte boundary
   void* cube;
   const float* mask;
   int mask_per_f, cube_f_total, cube_f0;
 };
 enum { DENSE_IMG = 0, DENSE_CUBE_F32 = 1, DENSE_CUBE_F16 = 2 };
 
+// Four consecutive pixels, in one access (VEC) where they start on its boundary.
+template <bool VEC>
+DSB_DEV float4 get4(const float* p) {
+  return VEC ? __ldg(reinterpret_cast<const float4*>(p))
+             : make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
+}
+template <bool VEC>
+DSB_DEV void put4(float* p, float4 v) {
+  if constexpr (VEC) {
+    *reinterpret_cast<float4*>(p) = v;
+  } else {
+    p[0] = v.x; p[1] = v.y; p[2] = v.z; p[3] = v.w;
+  }
+}
+template <bool VEC>
+DSB_DEV void put4(__half* p, float4 v) {
+  const __half2 x = __floats2half2_rn(v.x, v.y), y = __floats2half2_rn(v.z, v.w);
+  if constexpr (VEC) {
+    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&x),
+                                              *reinterpret_cast<const uint32_t*>(&y));
+  } else {
+    p[0] = __low2half(x); p[1] = __high2half(x); p[2] = __low2half(y); p[3] = __high2half(y);
+  }
+}
+
 // With the mask and the cube's layout and type applied here, an image's
 // pixels are written once (a separate pass read them back from L2 and wrote
 // them again: 18.6 us per 64 images of 256^2 beside this pass's 11.6; both are
 // now 8.7 us).
-template <int N, int OUT>
+template <int N, int OUT, bool VEC>
 __global__ void __launch_bounds__(DenseGeom<N>::ROW_THREADS)
     irfft2_rows_kernel(const DenseImages I, const float2* __restrict__ twn, const DenseOut O) {
   using Dg = DenseGeom<N>;
@@ -1084,40 +1108,24 @@ __global__ void __launch_bounds__(DenseGeom<N>::ROW_THREADS)
     float4 b = make_float4(p.y * scale, p.w * scale, q.y * scale, q.w * scale);
     const size_t px = (size_t)(2 * pr) * N + i;
     if constexpr (OUT == DENSE_IMG) {
-      float* o = O.img + (size_t)blockIdx.y * N * N + px;
-      if (O.img_vec) {
-        *reinterpret_cast<float4*>(o) = a;
-        *reinterpret_cast<float4*>(o + N) = b;
-      } else {
-        o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w;
-        o[N] = b.x; o[N + 1] = b.y; o[N + 2] = b.z; o[N + 3] = b.w;
-      }
+      put4<VEC>(O.img + (size_t)blockIdx.y * N * N + px, a);
+      put4<VEC>(O.img + (size_t)blockIdx.y * N * N + px + N, b);
     } else {
       const int f = blockIdx.y / I.n_t, t = blockIdx.y % I.n_t;
       const float* m = O.mask + (O.mask_per_f ? (size_t)f * N * N : 0) + px;
-      const float4 ma = __ldg(reinterpret_cast<const float4*>(m));
-      const float4 mb = __ldg(reinterpret_cast<const float4*>(m + N));
+      const float4 ma = get4<VEC>(m), mb = get4<VEC>(m + N);
       a = make_float4(a.x * ma.x, a.y * ma.y, a.z * ma.z, a.w * ma.w);
       b = make_float4(b.x * mb.x, b.y * mb.y, b.z * mb.z, b.w * mb.w);
       const size_t o = ((size_t)t * O.cube_f_total + O.cube_f0 + f) * N * N + px;
-      if constexpr (OUT == DENSE_CUBE_F32) {
-        *reinterpret_cast<float4*>(static_cast<float*>(O.cube) + o) = a;
-        *reinterpret_cast<float4*>(static_cast<float*>(O.cube) + o + N) = b;
-      } else {
-        auto put = [](__half* d, float4 v) {
-          __half2 x = __floats2half2_rn(v.x, v.y), y = __floats2half2_rn(v.z, v.w);
-          *reinterpret_cast<uint2*>(d) = make_uint2(*reinterpret_cast<uint32_t*>(&x),
-                                                    *reinterpret_cast<uint32_t*>(&y));
-        };
-        put(static_cast<__half*>(O.cube) + o, a);
-        put(static_cast<__half*>(O.cube) + o + N, b);
-      }
+      using C = typename std::conditional<OUT == DENSE_CUBE_F32, float, __half>::type;
+      put4<VEC>(static_cast<C*>(O.cube) + o, a);
+      put4<VEC>(static_cast<C*>(O.cube) + o + N, b);
     }
   }
 }
 
 // Both passes over n_img images (at most 65535).
-template <int N, int OUT>
+template <int N, int OUT, bool VEC>
 int launch_irfft2(const DenseImages& I, int n_img, const float2* twn, const DenseOut& O,
                   cudaStream_t stream) {
   using Dg = DenseGeom<N>;
@@ -1127,7 +1135,7 @@ int launch_irfft2(const DenseImages& I, int n_img, const float2* twn, const Dens
   if (!attr) {
     if (cudaFuncSetAttribute(irfft2_cols_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem_c) != cudaSuccess ||
-        cudaFuncSetAttribute(irfft2_rows_kernel<N, OUT>,
+        cudaFuncSetAttribute(irfft2_rows_kernel<N, OUT, VEC>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_r) !=
             cudaSuccess)
       return DSB_E_CUDA;
@@ -1136,19 +1144,19 @@ int launch_irfft2(const DenseImages& I, int n_img, const float2* twn, const Dens
   const dim3 gc((Dg::NH + FFT_CW - 1) / FFT_CW, n_img);
   irfft2_cols_kernel<N><<<gc, Dg::COL_THREADS, smem_c, stream>>>(I, twn);
   const dim3 gr((N / 2 + Dg::ROW_GROUPS - 1) / Dg::ROW_GROUPS, n_img);
-  irfft2_rows_kernel<N, OUT><<<gr, Dg::ROW_THREADS, smem_r, stream>>>(I, twn, O);
+  irfft2_rows_kernel<N, OUT, VEC><<<gr, Dg::ROW_THREADS, smem_r, stream>>>(I, twn, O);
   return launch_status();
 }
 
-template <int OUT>
+template <int OUT, bool VEC>
 int launch_irfft2_n(int N, const DenseImages& I, int n_img, const float2* twn, const DenseOut& O,
                     cudaStream_t stream) {
   switch (N) {
-    case 32: return launch_irfft2<32, OUT>(I, n_img, twn, O, stream);
-    case 64: return launch_irfft2<64, OUT>(I, n_img, twn, O, stream);
-    case 128: return launch_irfft2<128, OUT>(I, n_img, twn, O, stream);
-    case 256: return launch_irfft2<256, OUT>(I, n_img, twn, O, stream);
-    case 512: return launch_irfft2<512, OUT>(I, n_img, twn, O, stream);
+    case 32: return launch_irfft2<32, OUT, VEC>(I, n_img, twn, O, stream);
+    case 64: return launch_irfft2<64, OUT, VEC>(I, n_img, twn, O, stream);
+    case 128: return launch_irfft2<128, OUT, VEC>(I, n_img, twn, O, stream);
+    case 256: return launch_irfft2<256, OUT, VEC>(I, n_img, twn, O, stream);
+    case 512: return launch_irfft2<512, OUT, VEC>(I, n_img, twn, O, stream);
     default: return DSB_E_UNSUPPORTED;
   }
 }
@@ -1185,8 +1193,10 @@ int dsb_irfft2(void* half, int n_img, int N, const void* twiddles, float* out,
     return DSB_E_ARG;
   const float2* tw = static_cast<const float2*>(twiddles);
   const DenseImages I{static_cast<float2*>(half), 0, n_img};
-  const DenseOut O{out, (reinterpret_cast<uintptr_t>(out) & 15) == 0, nullptr, nullptr, 0, 0, 0};
-  return launch_irfft2_n<DENSE_IMG>(N, I, n_img, tw, O, stream);
+  const DenseOut O{out, nullptr, nullptr, 0, 0, 0};
+  return (reinterpret_cast<uintptr_t>(out) & 15) == 0
+             ? launch_irfft2_n<DENSE_IMG, true>(N, I, n_img, tw, O, stream)
+             : launch_irfft2_n<DENSE_IMG, false>(N, I, n_img, tw, O, stream);
 }
 
 int dsb_irfft2_cube(void* half, long long f_stride, int n_f, int n_t, int N, const void* twiddles,
@@ -1195,14 +1205,20 @@ int dsb_irfft2_cube(void* half, long long f_stride, int n_f, int n_t, int N, con
   if (!half || !twiddles || !mask || !cube || n_f <= 0 || n_t <= 0 || f_stride < 0 ||
       cube_f0 < 0 || cube_f0 + n_f > cube_f_total || (long long)n_f * n_t > 65535)
     return DSB_E_ARG;
-  if ((reinterpret_cast<uintptr_t>(half) & 7) || (reinterpret_cast<uintptr_t>(mask) & 15) ||
-      (reinterpret_cast<uintptr_t>(cube) & (cube_f16 ? 7 : 15)))
+  const uintptr_t at = reinterpret_cast<uintptr_t>(cube), at_m = reinterpret_cast<uintptr_t>(mask);
+  if ((reinterpret_cast<uintptr_t>(half) & 7) || (at_m & 3) || (at & (cube_f16 ? 1 : 3)))
     return DSB_E_ARG;
   const float2* tw = static_cast<const float2*>(twiddles);
   const DenseImages I{static_cast<float2*>(half), f_stride, n_t};
-  const DenseOut O{nullptr, 0, cube, mask, mask_per_f, cube_f_total, cube_f0};
-  return cube_f16 ? launch_irfft2_n<DENSE_CUBE_F16>(N, I, n_f * n_t, tw, O, stream)
-                  : launch_irfft2_n<DENSE_CUBE_F32>(N, I, n_f * n_t, tw, O, stream);
+  const DenseOut O{nullptr, cube, mask, mask_per_f, cube_f_total, cube_f0};
+  const bool vec = (at & (cube_f16 ? 7 : 15)) == 0 && (at_m & 15) == 0;
+  auto go = [&](auto out, auto v) {
+    return launch_irfft2_n<decltype(out)::value, decltype(v)::value>(N, I, n_f * n_t, tw, O, stream);
+  };
+  using F32 = std::integral_constant<int, DENSE_CUBE_F32>;
+  using F16 = std::integral_constant<int, DENSE_CUBE_F16>;
+  if (vec) return cube_f16 ? go(F16{}, std::true_type{}) : go(F32{}, std::true_type{});
+  return cube_f16 ? go(F16{}, std::false_type{}) : go(F32{}, std::false_type{});
 }
 
 int dsb_image_fft(const void* D, int d_format, const long long* seg_base, const int* seg_depth,

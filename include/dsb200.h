@@ -365,8 +365,8 @@ int dsb_irfft2(void* half, int n_img, int N, const void* twiddles, float* out,
  * (f, t) of half (at half + f * f_stride + t * N * (N/2+1), complex64, used
  * as the work buffer) times mask (N x N, or mask_per_f: n_f x N x N) to
  * cube[t][cube_f0 + f][N][N] (float16 or float32, cube_f_total fine DMs).
- * mask 16-byte aligned, cube 16-byte (float16: 8-byte) aligned; n_f * n_t at
- * most 65535.  Replaces the transform, mask and cube write of
+ * n_f * n_t at most 65535 (four pixels per access where mask and cube start
+ * on that boundary).  Replaces the transform, mask and cube write of
  * GpuImager.process_cube (src/dsart/image/imager_gpu.py:590-650). */
 int dsb_irfft2_cube(void* half, long long f_stride, int n_f, int n_t, int N, const void* twiddles,
                     const float* mask, int mask_per_f, void* cube, int cube_f16, int cube_f_total,
