@@ -481,6 +481,8 @@ class GpuImager:
         256^2, against 1103 us one fine DM at a time)."""
         cfg = self.config
         N, nh = cfg.n_grid, cfg.n_grid // 2 + 1
+        if cfg.n_fdm == 0:
+            return
         cap = min(buf.numel() // (N * nh), 65535)
         nf_c = min(cfg.n_fdm, cap)
         nt_c = min(cfg.t_det, cap // nf_c)
@@ -523,6 +525,8 @@ class GpuImager:
                              "calibration needs the dense combine")
         if t_stream < cfg.t_det:
             raise ValueError(f"compact_t_stream={t_stream} < T_det={cfg.t_det}")
+        if cfg.n_fdm == 0:
+            raise ValueError("compact combine needs at least one fine DM")
 
         def combine(csr, st):
             for f0, n_f, t0, nt, work in self._chunks(t_lo, full):

@@ -1,6 +1,6 @@
 """GpuImager.process_cube on a cube and masks of the caller's own: views that
 start off the 16-byte boundaries of the kernels' wide accesses give the same
-pixels."""
+pixels, and a configuration without fine DMs gives an empty cube."""
 
 import pytest
 import torch
@@ -38,3 +38,16 @@ def test_cube_and_mask_at_any_offset(cube_off, mask_off, N, dt, per_f):
     if per_f:
         im.edge_mask_per_fdm = _off(im.edge_mask_per_fdm, mask_off)
     assert torch.equal(im.process_cube(**kw), ims[0].process_cube(**kw))
+
+
+def test_no_fine_dms():
+    from dsb200.search import GpuImager, GpuImagerConfig
+    dev = torch.device("cuda", 0)
+    im = GpuImager.build(GpuImagerConfig(n_grid=32, t_det=5, n_fdm=0, n_chgroup=3, device=dev))
+    sh = torch.zeros(0, 3, dtype=torch.int32, device=dev)
+    st = torch.zeros(3, 9, 2, 32, 32, dtype=torch.int8, device=dev)
+    assert im.process_cube(streams_cint8=st, time_shifts_gpu=sh).shape == (5, 0, 32, 32)
+    with pytest.raises((RuntimeError, ValueError)):     # the compact combine never took it
+        im.process_cube(streams_cint8=torch.zeros(3, 4, 9, 2, dtype=torch.int8, device=dev),
+                        time_shifts_gpu=sh, compact_t_stream=9,
+                        compact_inv_lut=torch.full((3, 1024), -1, dtype=torch.int64, device=dev))
