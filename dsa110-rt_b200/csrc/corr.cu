@@ -155,15 +155,17 @@ constexpr int TC_THREADS = 256;
 constexpr int TC_TMEM_COLS = 512;   // two accumulators of <= 256 columns
 constexpr int TC_SMEM_BUDGET = 224 * 1024;
 constexpr int TC_PRE = 4;          // 16-byte raw loads per thread per item (nant <= 128)
-// gridding rows of one (chgroup, subband) whose offsets are kept in smem: a
-// baseline meets about two cells over a chgroup's subbands, so four rows per
-// baseline, at most 12288 (24 KB).  Groups beyond it read their tables in
-// place, which costs a chain of global loads per row: with 4096 rows, too few
-// for some of the 512^2 patterns of 96 antennas, the gridding took 37 us of
-// every unit and set the kernel's time.
-__host__ __device__ constexpr int tc_cap_rows(int nant) {
+// Gridding rows of one (chgroup, subband) whose offsets are kept in shared
+// memory, at least: a baseline meets about two cells over a chgroup's
+// subbands, so four rows per baseline, between 4096 (wide chgroups: 2404 rows
+// at 32 antennas, two chgroups over the band, 512^2) and 12288.  What the
+// operand stages leave free holds more (tc_fit_rows).  Groups beyond it read
+// their tables in place, which costs a chain of global loads per row: 37 us of
+// every unit of some 512^2 patterns of 96 antennas where it was 4096 rows, and
+// 261 -> 177 us for those 32 antennas (2 x 512 packets), which 2112 left out.
+__host__ __device__ constexpr int tc_min_rows(int nant) {
   const int n = 2 * nant * (nant + 1);
-  return n < 1024 ? 1024 : n > 12288 ? 12288 : n;
+  return n < 4096 ? 4096 : n > 12288 ? 12288 : n;
 }
 // Every CTA requests more than half an SM's shared memory so that exactly
 // one CTA (and one 512-column tensor-memory allocation) lives on each SM.
@@ -186,6 +188,7 @@ struct TcArgs {
   const int* ycnt;    // (n_chgroup*ceff) rows in the group
   const int* row_off; // (n_rows + 1) CSR over rows: baselines gridded into each row
   const int* row_bls; // baseline index of each CSR entry
+  int cap_rows;       // rows of one group whose offsets fit shared memory
   float2* yout;
   long long y_t_stride;
   long long t_base;
@@ -387,7 +390,7 @@ DSB_DEV void tc_fill(const TcArgs& A, uint8_t* st, int g, int f, int s, int q) {
 struct TcTab {
   int* cached;      // group index whose tables are loaded (-1 none)
   uint16_t* bls;    // (nbase) baseline of each entry
-  uint16_t* roff;   // (tc_cap_rows + 1) row offsets relative to the group's first entry
+  uint16_t* roff;   // (TcArgs.cap_rows + 1) row offsets relative to the group's first entry
 };
 
 // NT threads (warps 0 .. NT / 32 - 1 of the CTA) take part; sync is their
@@ -471,7 +474,7 @@ DSB_DEV void tc_epilogue(const TcArgs& A, uint32_t acc, int g, int f, int s, int
     const int cnt = A.ycnt[gs];
     const int e0 = A.row_off[row0];
     const int ne = A.row_off[row0 + cnt] - e0;
-    const bool use_tab = cnt <= tc_cap_rows(A.nant) && ne <= A.nant * (A.nant + 1) / 2;
+    const bool use_tab = cnt <= A.cap_rows && ne <= A.nant * (A.nant + 1) / 2;
     const bool reload = use_tab && *tab.cached != gs;
     if (reload) {
       for (int k = threadIdx.x; k <= cnt; k += NT) tab.roff[k] = (uint16_t)(A.row_off[row0 + k] - e0);
@@ -1552,7 +1555,14 @@ int launch_status() {
 int tc_extra_bytes(const TcArgs& A, int mode) {
   if (mode != 1) return A.q_pitch * TC_QF * 8;
   const int nbase = A.nant * (A.nant + 1) / 2;
-  return nbase * 8 + 16 + nbase * 2 + (tc_cap_rows(A.nant) + 1) * 2 + 16;
+  return nbase * 8 + 16 + nbase * 2 + (A.cap_rows + 1) * 2 + 16;
+}
+
+// Offsets of more rows in `room` bytes that the stages leave free (no more
+// than the subbands can give: one row per baseline and subband).
+void tc_fit_rows(TcArgs& A, int room) {
+  const long long most = (long long)A.nant * (A.nant + 1) / 2 * A.ceff;
+  A.cap_rows = (int)std::max<long long>(A.cap_rows, std::min<long long>(most, A.cap_rows + room / 2));
 }
 
 // Fill the derived geometry; returns DSB_OK or an error code.
@@ -1572,12 +1582,13 @@ int tc_plan(TcArgs& A, int mode) {
   A.nkblk = (2 * A.kc + 127) / 128;
   A.stage_bytes = A.nkblk * A.rows * 128;
   A.n_mma = 2 * A.kc / 32;
-  const int extra = tc_extra_bytes(A, mode);
-  const int budget = TC_SMEM_BUDGET - extra - 1024 - 256;
-  A.nstage = std::min(4, budget / A.stage_bytes);
-  if (A.nstage < 2) return DSB_E_UNSUPPORTED;
   A.tma = 0;
   A.q_pitch = 0;
+  A.cap_rows = tc_min_rows(A.nant);
+  const int budget = TC_SMEM_BUDGET - tc_extra_bytes(A, mode) - 1024 - 256;
+  A.nstage = std::min(4, budget / A.stage_bytes);
+  if (A.nstage < 2) return DSB_E_UNSUPPORTED;
+  tc_fit_rows(A, budget - A.nstage * A.stage_bytes);
   return DSB_OK;
 }
 
@@ -1591,6 +1602,7 @@ bool ws_plan(TcArgs& A, int mode, int kc, int q_pitch) {
       ((kc / 4) % A.csf))
     return false;
   TcArgs P = A;
+  P.cap_rows = tc_min_rows(P.nant);
   P.kc = kc;
   P.n_chunks = kprime / kc;
   P.nkblk = (2 * kc + 127) / 128;
@@ -1610,6 +1622,7 @@ bool ws_plan(TcArgs& A, int mode, int kc, int q_pitch) {
                      tc_extra_bytes(P, mode) - 1024 - 256;
     const int ns = std::min(4, (room - P.nraw * P.raw_stage) / P.stage_bytes);
     if (ns < 2) continue;
+    tc_fit_rows(P, room - P.nraw * P.raw_stage - ns * P.stage_bytes);
     P.tma = 1;
     P.ws_nstage = ns;
     A = P;
