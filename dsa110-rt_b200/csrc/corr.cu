@@ -412,33 +412,42 @@ DSB_DEV void tc_epilogue(const TcArgs& A, uint32_t acc, int g, int f, int s, int
       tmem_ld16(lane_base + (uint32_t)(nant + c0), vi);
       tmem_ld_wait();
       if (b < nant) {
+        auto each = [&](auto emit) {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const int a = c0 + j;
-          if (a < b || a >= nant) continue;
-          const int bls = upper_bls(a, b);
-          const int re = (int)vr[j], im = (int)vi[j];
-          if constexpr (MODE == 0) {
-            if (A.q_pitch) {
-              vbuf[((A.unit_order ? s : f) & (TC_QF - 1)) * A.q_pitch + bls] = make_int2(re, im);
-              continue;
-            }
-            A.out[(size_t)g * A.o_g + (size_t)f * A.o_f + (size_t)bls * A.o_b + (size_t)s * A.o_s] =
-                make_float2((float)re, (float)im);
-          } else if (A.gains) {
-            // calibrated: V' = g_a conj(g_b) V (V = conj(E_b) E_a), every
-            // product and sum rounded on its own (no contraction)
-            const float2* gs = A.gains + ((size_t)g * A.ceff + s) * nant;
-            const float2 ga = gs[a], gb = gs[b];
+          for (int j = 0; j < 16; ++j) {
+            const int a = c0 + j;
+            if (a < b || a >= nant) continue;
+            emit(a, upper_bls(a, b), (int)vr[j], (int)vi[j]);
+          }
+        };
+        if constexpr (MODE == 0) {
+          // (a loop of its own per form: the test per output cost the direct
+          // one up to a tenth, 34.6 -> 38 us per 2 x 128 packets of 48 antennas)
+          if (A.q_pitch) {
+            int2* v = vbuf + ((A.unit_order ? s : f) & (TC_QF - 1)) * A.q_pitch;
+            each([&](int, int bls, int re, int im) { v[bls] = make_int2(re, im); });
+          } else {
+            float2* o = A.out + (size_t)g * A.o_g + (size_t)f * A.o_f + (size_t)s * A.o_s;
+            each([&](int, int bls, int re, int im) {
+              o[(size_t)bls * A.o_b] = make_float2((float)re, (float)im);
+            });
+          }
+        } else if (A.gains) {
+          // calibrated: V' = g_a conj(g_b) V (V = conj(E_b) E_a), every
+          // product and sum rounded on its own (no contraction)
+          const float2* gs = A.gains + ((size_t)g * A.ceff + s) * nant;
+          const float2 gb = gs[b];
+          each([&](int a, int bls, int re, int im) {
+            const float2 ga = gs[a];
             const float pr = __fadd_rn(__fmul_rn(ga.x, gb.x), __fmul_rn(ga.y, gb.y));
             const float pi = __fsub_rn(__fmul_rn(ga.y, gb.x), __fmul_rn(ga.x, gb.y));
             const float fr = (float)re, fi = (float)im;
             reinterpret_cast<float2*>(vbuf)[bls] =
                 make_float2(__fsub_rn(__fmul_rn(fr, pr), __fmul_rn(fi, pi)),
                             __fadd_rn(__fmul_rn(fr, pi), __fmul_rn(fi, pr)));
-          } else {
-            vbuf[bls] = make_int2(re, im);
-          }
+          });
+        } else {
+          each([&](int, int bls, int re, int im) { vbuf[bls] = make_int2(re, im); });
         }
       }
     }
