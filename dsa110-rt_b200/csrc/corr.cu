@@ -1642,14 +1642,20 @@ bool ws_plan(TcArgs& A, int mode, int kc, int q_pitch) {
 
 // The TMA form's plan, if it has one: mode 0 with outputs of adjacent units
 // staged where they are adjacent in memory (with 96 antennas that takes
-// chunks of 64 samples instead of 128).
-void ws_choose(TcArgs& A, int mode) {
+// chunks of 64 samples instead of 128) and the CTAs have TC_QF units or more
+// each to write together: 269 -> 116 us for 3072 units of 96 antennas at the
+// 262-us cadence, but 10.2 -> 12.7 us for 24 (equal near 600, four per CTA).
+void ws_choose(TcArgs& A, int mode, int n_units, int max_ctas) {
   const int nbase = A.nant * (A.nant + 1) / 2;
   // pitch = 4 mod 16 eight-byte words: four units' reads in different banks
   const int pitch = (nbase + 15) / 16 * 16 + 4;
+  TcArgs P = A;
   if (mode == 0 && (A.unit_order ? A.o_s : A.o_f) == 1 &&
-      (ws_plan(A, mode, A.kc, pitch) || ws_plan(A, mode, 64, pitch)))
+      (ws_plan(P, mode, P.kc, pitch) || ws_plan(P, mode, 64, pitch)) &&
+      n_units > (TC_QF - 1) * (max_ctas > 0 ? max_ctas : P.ctas * num_sms())) {
+    A = P;
     return;
+  }
   ws_plan(A, mode, A.kc, 0);
 }
 
@@ -1697,7 +1703,7 @@ int tc_launch(TcArgs& A, int n_units, int max_ctas, cudaStream_t stream) {
   CUtensorMap tmap;
   memset(&tmap, 0, sizeof(tmap));
   const TcArgs plain = A;
-  ws_choose(A, MODE);
+  ws_choose(A, MODE, n_units, max_ctas);
   if (A.tma && !tc_raw_tmap(A, &tmap)) A = plain;
   if (A.tma) {
     A.nstage = A.ws_nstage;
