@@ -258,8 +258,8 @@ class FastCorrKernel:
     nbada_pol: int = BADA_NPOL
     accum_dtype: torch.dtype = torch.float32
     _nbase: int = field(init=False)
-    # (stream, zeroed status words, how many are taken), see _status_word
-    _words: Optional[tuple] = field(default=None, init=False, repr=False, compare=False)
+    # per stream: zeroed status words, the indices not taken yet (_status_word)
+    _words: dict = field(default_factory=dict, init=False, repr=False, compare=False)
     _last: Optional[tuple] = field(default=None, init=False, repr=False, compare=False)
 
     def __post_init__(self) -> None:
@@ -288,22 +288,32 @@ class FastCorrKernel:
         if st is not None:
             _lib.check_status(st, "FastCorrKernel")
 
-    _N_WORDS = 256
+    _N_WORDS, _N_STREAMS = 256, 16
+
+    def __getstate__(self) -> dict:
+        """Without the status words: a copy's launches take words of its own."""
+        return {**self.__dict__, "_words": {}}
 
     def _status_word(self, stream: int) -> Tuple[torch.Tensor, int]:
         """A zeroed device status word of this launch's own, (words, index).
         Zeroing one per launch cost it an allocation and a fill kernel (20.9
-        -> 14.3 us per call at 16 antennas x 64 packets); 256 are zeroed at a time, on the stream that uses them, and none is
-        used twice.  A captured launch gets its own, which every replay
-        zeroes.  (The held tuple is read once: calls from two threads may
-        share a word, never run past the last.)"""
+        -> 14.3 us per call at 16 antennas x 64 packets); 256 are zeroed at a
+        time, on the stream that uses them, and no index is handed out twice
+        (list.pop, one step for other threads too).  Words are held for the
+        last few streams only.  A captured launch gets its own, which every
+        replay zeroes."""
         if torch.cuda.is_current_stream_capturing():
             return _lib.status_word(self.device), 0
-        held = self._words
-        if held is None or held[0] != stream or held[2] >= self._N_WORDS:
-            held = (stream, torch.zeros(self._N_WORDS, dtype=torch.int32, device=self.device), 0)
-        self._words = (stream, held[1], held[2] + 1)
-        return held[1], held[2]
+        try:
+            words, free = self._words[stream]
+            return words, free.pop()
+        except (KeyError, IndexError):
+            words = torch.zeros(self._N_WORDS, dtype=torch.int32, device=self.device)
+            free = list(range(self._N_WORDS))
+            i = free.pop()
+            held = {k: v for k, v in list(self._words.items()) if k != stream}
+            self._words = {**dict(list(held.items())[1 - self._N_STREAMS:]), stream: (words, free)}
+            return words, i
 
     def compute_split(self, real_v: torch.Tensor, imag_v: torch.Tensor, *,
                       n_fv_chunk: Optional[int] = None, fuse_stokes_i: bool = False,
