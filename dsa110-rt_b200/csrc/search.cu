@@ -399,24 +399,49 @@ __global__ void mask_to_cube_kernel(const float* __restrict__ img, const float* 
 // fftshift; int32 sums, so exact; fp16 pairs or complex64.  Only active
 // cells are written.
 //
-// A CTA takes 32 consecutive active cells and a tile of CS_T output times for
-// every fine DM.  Each stream row (cell k or mirror km of one stream) is
-// staged once in shared memory, the tile's times plus the spread of all
-// shifts, zero outside [0, t_rows); a lane then owns a cell and sums 8 times
-// at a time, two samples per word (re and im bytes offset to unsigned in 16-bit
-// lanes), and a warp's stores go to consecutive active cells.  One CTA per
-// cell, each thread one (fine DM, time) with 2-byte gathers and 8-byte stores
-// a whole spectrum apart, took 353 us for 16 fine DMs x 64 times of 33k half
-// cells (270 MB written); this takes 226 us.
-// Cells whose rows do not fit at 32 run in groups of 16, 8, ... 1; a window
-// too wide even for one cell is read in place.
+// Two forms.  A cell at a time (sparse_cell): the cell's entries in shared
+// memory, a thread per (fine DM, time) with 2-byte gathers along the time.
+//
+// Staged (combine_sparse_kernel): a CTA takes 32 or 16 consecutive active
+// cells and a tile of CS_T output times for every fine DM.  Each stream row
+// (cell k or mirror km of one stream) is staged once in shared memory, the
+// tile's times plus the spread of all shifts, zero outside [0, t_rows); a lane
+// then owns a cell and sums 8 times at a time, two samples per word (re and im
+// bytes offset to unsigned in 16-bit lanes), and a warp's stores go to
+// consecutive active cells.  16 fine DMs x 64 times of 28.6k half cells: 380 us
+// a cell at a time, 228 us with 32 cells per CTA, 196 us with 16.
+// Cells whose rows do not fit together run in groups of 16, 8, ... 1.
+//
+// The staged form's set-up (shift range, row lists, window) and its few CTAs
+// pay only where many outputs share them: 381 cells x 8 fine DMs x 64 times
+// take 5.2 us a cell at a time and 6.4 us staged (30 us with 32 cells per
+// CTA), 1581 cells 10 and 12 us, 10.2k cells x 4 x 32 times 20 and 14 us; so
+// calls of less than CS_STAGED_MIN outputs go a cell at a time.  So does a
+// CTA whose windows hold more words than twice the outputs per row (only the
+// device knows the shifts), on cells a grid apart, so that those that run
+// together write the same sectors: 484 us for 16 fine DMs with shifts spread
+// over 3000 times, staged 787 (combine_cell_kernel's fuller SMs take 359).
 // ===========================================================================
 constexpr int CS_T = 64;
 constexpr int CS_MAXE = 64;
 constexpr int CS_CELLS = 32;
 constexpr int CS_THREADS = 128;
-constexpr int CS_WORDS = 10240;                 // staged words (two samples each)
+constexpr int CS_WORDS = 10240;                 // staged words (two samples each) of 32 cells
 constexpr int CS_ROWS = CS_WORDS / (CS_T / 2);  // most rows of a group
+constexpr int CS_CELL_THREADS = 256;
+constexpr long long CS_STAGED_MIN = 1 << 20;
+
+struct SparseArgs {
+  const int16_t* dense;
+  const int *cell_uw, *cell_ptr, *ent_g, *ent_k, *ent_km, *shifts;
+  void* out;
+  int n_act, cpc, words;   // active cells; cells per CTA and staged words of the staged form
+  int n_sb, t_rows, t_pad, nfm, N, n_fdm, t_out_len, t_lo, fftshift, out_rows, out_row0;
+  int* status;
+};
+DSB_DEV bool sparse_entry_ok(const SparseArgs& A, int g, int k, int km) {
+  return g >= 0 && g < A.n_sb && k < A.nfm && km < A.nfm;
+}
 
 template <bool OUT_F16>
 DSB_DEV void sparse_put(void* out, long long o, float re, float im, bool flip) {
@@ -430,25 +455,81 @@ DSB_DEV void sparse_put(void* out, long long o, float re, float im, bool flip) {
     reinterpret_cast<float2*>(out)[o] = make_float2(re, im);
 }
 
+// Cell a at output times t0 .. t0 + nt - 1 for every fine DM, by the NT threads
+// of the CTA.  s_ent: 3 * CS_MAXE ints.
+template <bool OUT_F16, int NT>
+DSB_DEV void sparse_cell(const SparseArgs& A, int a, int t0, int nt, int* s_ent) {
+  const int e0 = A.cell_ptr[a], ne = A.cell_ptr[a + 1] - e0;
+  if (ne > CS_MAXE || ne < 0) {
+    if (threadIdx.x == 0) dsb_flag(A.status, DSB_E_CAPACITY);
+    return;
+  }
+  for (int e = threadIdx.x; e < ne; e += NT) {
+    const int g = A.ent_g[e0 + e], k = A.ent_k[e0 + e], km = A.ent_km[e0 + e];
+    const bool ok = sparse_entry_ok(A, g, k, km);
+    s_ent[3 * e] = ok ? g : -1;
+    s_ent[3 * e + 1] = k;
+    s_ent[3 * e + 2] = km;
+    if (!ok) dsb_flag(A.status, DSB_E_ARG);
+  }
+  __syncthreads();
+  const int nh = A.N / 2 + 1, uw = A.cell_uw[a];
+  const bool flip = A.fftshift && ((uw / nh + uw % nh) & 1);
+  for (int idx = threadIdx.x; idx < A.n_fdm * CS_T; idx += NT) {
+    const int f = idx / CS_T, tl = idx % CS_T;
+    if (tl >= nt) continue;
+    const int t = t0 + tl;
+    int re = 0, im = 0;
+    for (int e = 0; e < ne; ++e) {
+      const int g = s_ent[3 * e], k = s_ent[3 * e + 1], km = s_ent[3 * e + 2];
+      if (g < 0) continue;
+      const int ts = t + A.t_lo - A.shifts[f * A.n_sb + g];
+      if (ts < 0 || ts >= A.t_rows) continue;
+      const long long row = (long long)g * A.nfm;
+      if (k >= 0) {
+        const int16_t v = __ldg(A.dense + (row + k) * A.t_pad + ts);
+        re += (int)(int8_t)(v & 0xff);
+        im += (int)(int8_t)((v >> 8) & 0xff);
+      }
+      if (km >= 0) {
+        const int16_t v = __ldg(A.dense + (row + km) * A.t_pad + ts);
+        re += (int)(int8_t)(v & 0xff);
+        im -= (int)(int8_t)((v >> 8) & 0xff);
+      }
+    }
+    sparse_put<OUT_F16>(A.out, ((long long)f * A.out_rows + A.out_row0 + t) * A.N * nh + uw,
+                        0.5f * (float)re, 0.5f * (float)im, flip);
+  }
+}
+
 template <bool OUT_F16>
-__global__ void __launch_bounds__(CS_THREADS) combine_sparse_kernel(
-    const int16_t* __restrict__ dense, const int* __restrict__ cell_uw,
-    const int* __restrict__ cell_ptr, const int* __restrict__ ent_g,
-    const int* __restrict__ ent_k, const int* __restrict__ ent_km,
-    const int* __restrict__ shifts, void* __restrict__ out, int n_act, int n_sb, int t_rows,
-    int t_pad, int nfm, int N, int n_fdm, int t_out_len, int t_lo, int fftshift, int out_rows,
-    int out_row0, int* __restrict__ status) {
-  __shared__ uint32_t s_win[CS_WORDS];
+__global__ void __launch_bounds__(CS_CELL_THREADS) combine_cell_kernel(const SparseArgs A) {
+  __shared__ int s_ent[3 * CS_MAXE];
+  const int t0 = blockIdx.y * CS_T;
+  sparse_cell<OUT_F16, CS_CELL_THREADS>(A, blockIdx.x, t0, min(CS_T, A.t_out_len - t0), s_ent);
+}
+
+template <bool OUT_F16>
+__global__ void __launch_bounds__(CS_THREADS) combine_sparse_kernel(const SparseArgs A) {
+  extern __shared__ uint32_t s_win[];              // [A.words]
   __shared__ long long s_row[CS_ROWS];             // stream row of each staged row
   __shared__ int s_rowg[CS_ROWS];                  // its stream
   __shared__ int s_ptr[CS_CELLS], s_ne[CS_CELLS], s_r0[CS_CELLS + 1], s_rm[CS_CELLS];
   __shared__ int s_min, s_max, s_group;
+  const int16_t* dense = A.dense;
+  const int *cell_uw = A.cell_uw, *cell_ptr = A.cell_ptr, *ent_g = A.ent_g, *ent_k = A.ent_k,
+            *ent_km = A.ent_km, *shifts = A.shifts;
+  void* out = A.out;
+  const int n_sb = A.n_sb, t_rows = A.t_rows, t_pad = A.t_pad, nfm = A.nfm, N = A.N,
+            n_fdm = A.n_fdm, t_lo = A.t_lo, fftshift = A.fftshift, out_rows = A.out_rows,
+            out_row0 = A.out_row0;
+  int* status = A.status;
   // the streams as aligned words of two samples
   const int dense_off = (int)((reinterpret_cast<uintptr_t>(dense) >> 1) & 1);
   const uint32_t* dense2 = reinterpret_cast<const uint32_t*>(dense - dense_off);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int a0 = blockIdx.x * CS_CELLS, nc = min(CS_CELLS, n_act - a0);
-  const int t0 = blockIdx.y * CS_T, nt = min(CS_T, t_out_len - t0);
+  const int a0 = blockIdx.x * A.cpc, nc = min(A.cpc, A.n_act - a0);
+  const int t0 = blockIdx.y * CS_T, nt = min(CS_T, A.t_out_len - t0);
   const int nh = N / 2 + 1;
   if (tid == 0) {
     s_min = 0x7fffffff;
@@ -473,8 +554,9 @@ __global__ void __launch_bounds__(CS_THREADS) combine_sparse_kernel(
   // words of a row: the tile's times at every shift, one more for odd starts,
   // odd so that lanes on different rows spread over the banks
   const int pitch = spread > 2 * CS_WORDS ? 0 : (int)((CS_T + spread + 1) / 2 + 1) | 1;
-  const int cap = pitch ? min(CS_ROWS, CS_WORDS / pitch) : 0;
-  auto entry_ok = [&](int g, int k, int km) { return g >= 0 && g < n_sb && k < nfm && km < nfm; };
+  const int cap = pitch && pitch <= 2LL * n_fdm * nt
+                      ? min(CS_ROWS, A.words / pitch) : 0;
+  auto entry_ok = [&](int g, int k, int km) { return sparse_entry_ok(A, g, k, km); };
   if (warp == 0) {
     // this lane's cell: its entries and rows (k rows and km rows)
     int ptr = 0, ne = 0, rows = 0;
@@ -505,38 +587,23 @@ __global__ void __launch_bounds__(CS_THREADS) combine_sparse_kernel(
     int group = 0, sum = rows;
 #pragma unroll
     for (int g = 1; g <= 32; g *= 2) {
-      if ((int)__reduce_max_sync(0xffffffffu, sum) <= cap) group = g;
+      if (g <= A.cpc && (int)__reduce_max_sync(0xffffffffu, sum) <= cap) group = g;
       sum += __shfl_xor_sync(0xffffffffu, sum, g);
     }
     if (lane == 0) s_group = group;
   }
   __syncthreads();
+  // (the rule of a group is the CTA's own, that of the windows the whole
+  // grid's: only then may the cells be dealt out anew)
+  const bool wide = cap == 0;
   const int group = s_group;
   if (group == 0) {
-    for (long long i = tid; i < (long long)nc * n_fdm * nt; i += CS_THREADS) {
-      const int c = (int)(i % nc), tl = (int)(i / nc % nt), f = (int)(i / nc / nt);
-      if (s_ne[c] < 0) continue;
-      const int uw = cell_uw[a0 + c], u = uw / nh, w = uw % nh, t = t0 + tl;
-      int re = 0, im = 0;
-      for (int e = s_ptr[c]; e < s_ptr[c] + s_ne[c]; ++e) {
-        const int g = ent_g[e], k = ent_k[e], km = ent_km[e];
-        if (!entry_ok(g, k, km)) continue;
-        const int ts = t + t_lo - shifts[f * n_sb + g];
-        if (ts < 0 || ts >= t_rows) continue;
-        const long long row = (long long)g * nfm;
-        if (k >= 0) {
-          const int16_t v = __ldg(dense + (row + k) * t_pad + ts);
-          re += (int)(int8_t)(v & 0xff);
-          im += (int)(int8_t)((v >> 8) & 0xff);
-        }
-        if (km >= 0) {
-          const int16_t v = __ldg(dense + (row + km) * t_pad + ts);
-          re += (int)(int8_t)(v & 0xff);
-          im -= (int)(int8_t)((v >> 8) & 0xff);
-        }
-      }
-      sparse_put<OUT_F16>(out, ((long long)f * out_rows + out_row0 + t) * N * nh + uw,
-                          0.5f * (float)re, 0.5f * (float)im, fftshift && ((u + w) & 1));
+    int* s_ent = reinterpret_cast<int*>(s_win);
+    for (int i = 0; i < nc || (wide && i < A.cpc); ++i) {
+      const int a = wide ? (int)blockIdx.x + i * (int)gridDim.x : a0 + i;
+      if (a >= A.n_act) break;
+      sparse_cell<OUT_F16, CS_THREADS>(A, a, t0, nt, s_ent);
+      __syncthreads();   // the entries' places are the next cell's
     }
     return;
   }
@@ -1663,17 +1730,24 @@ int dsb_combine_sparse(const void* dense, const int* cell_uw, const int* cell_pt
     return DSB_E_ARG;
   if (n_act == 0 || t_out_len == 0) return DSB_OK;
   if ((t_out_len + CS_T - 1) / CS_T > 65535) return DSB_E_ARG;
-  const dim3 grid((n_act + CS_CELLS - 1) / CS_CELLS, (t_out_len + CS_T - 1) / CS_T);
-  if (out_f16)
-    combine_sparse_kernel<true><<<grid, CS_THREADS, 0, stream>>>(
-        static_cast<const int16_t*>(dense), cell_uw, cell_ptr, ent_g, ent_k, ent_km, shifts, out,
-        n_act, n_sb, t_rows, t_pad, n_filled_max, N, n_fdm, t_out_len, t_lo, fftshift, out_rows,
-        out_row0, status);
-  else
-    combine_sparse_kernel<false><<<grid, CS_THREADS, 0, stream>>>(
-        static_cast<const int16_t*>(dense), cell_uw, cell_ptr, ent_g, ent_k, ent_km, shifts, out,
-        n_act, n_sb, t_rows, t_pad, n_filled_max, N, n_fdm, t_out_len, t_lo, fftshift, out_rows,
-        out_row0, status);
+  SparseArgs A{static_cast<const int16_t*>(dense), cell_uw, cell_ptr, ent_g, ent_k, ent_km, shifts,
+               out, n_act, 1, 0, n_sb, t_rows, t_pad, n_filled_max, N, n_fdm, t_out_len, t_lo,
+               fftshift, out_rows, out_row0, status};
+  const int tiles = (t_out_len + CS_T - 1) / CS_T;
+  if ((long long)n_act * n_fdm * t_out_len < CS_STAGED_MIN) {
+    auto kern = out_f16 ? combine_cell_kernel<true> : combine_cell_kernel<false>;
+    kern<<<dim3(n_act, tiles), CS_CELL_THREADS, 0, stream>>>(A);
+    return launch_status();
+  }
+  // 32 cells per CTA (five CTAs per SM) where they fill whole rounds of the
+  // chip, else 16 (twice the CTAs), fewer while that leaves SMs idle
+  auto ctas = [&](int cpc) { return (long long)((n_act + cpc - 1) / cpc) * tiles; };
+  const long long round = 148 * 5, n32 = ctas(CS_CELLS);
+  A.cpc = n32 * 10 >= (n32 + round - 1) / round * round * 7 ? CS_CELLS : CS_CELLS / 2;
+  A.words = A.cpc == CS_CELLS ? CS_WORDS : CS_WORDS / 2;
+  while (A.cpc > 1 && ctas(A.cpc) < 2 * 148) A.cpc /= 2;
+  auto kern = out_f16 ? combine_sparse_kernel<true> : combine_sparse_kernel<false>;
+  kern<<<dim3((n_act + A.cpc - 1) / A.cpc, tiles), CS_THREADS, (size_t)A.words * 4, stream>>>(A);
   return launch_status();
 }
 
