@@ -330,11 +330,24 @@ __global__ void __launch_bounds__(CP_MAX_THREADS) combine_pair_kernel(
   }
 }
 
-// Whether combine_pair_kernel takes the streams: whole 4-byte words of cells
+// Whether combine_pair_kernel can take the streams: whole 4-byte words of cells
 // in every row (other shapes run one cell per thread above).
 bool combine_pair_ok(const void* streams, int N, int n_t) {
   return N % 4 == 0 && N <= 8192 && n_t <= 65535 &&
          (reinterpret_cast<uintptr_t>(streams) & 3) == 0;
+}
+
+// Whether it should, for one fine DM.  Its lists, shared sums and barriers cost
+// about what four chgroups' loads do, so that few chgroups are faster one cell
+// per thread, more of them where that kernel has a float chain to hide its
+// byte loads behind: 64 times of 256^2 uncalibrated 23.9 and 25.0 us at one
+// chgroup, 28.6 and 25.9 at two; calibrated 22.8 and 26.8 at two, 28.5 and
+// 27.1 at three; 16 times of 512^2 calibrated 25.2 and 27.5 at four, 38.3 and
+// 33.3 at six; and as many where its CTAs leave SMs idle (2 times of 64^2 at
+// three: 2.6 and 2.9).
+bool combine_pair_better(bool calib, int G, int N, int n_t) {
+  if ((long long)(N / 2 + 1) * n_t < 128) return G >= 5;
+  return G >= (!calib ? 2 : N <= 256 ? 3 : 5);
 }
 
 int launch_combine_pair(const int8_t* streams, const int* shifts, const float* scales,
@@ -1773,7 +1786,8 @@ int dsb_combine_dense(const void* streams, const int* shifts, const float* scale
   if (half && (N & 1)) return DSB_E_ARG;
   const bool calib = scales != nullptr;
   if (calib && (!off_re || !off_im)) return DSB_E_ARG;
-  if (half && combine_pair_ok(streams, N, t_det - t_lo))
+  if (half && combine_pair_ok(streams, N, t_det - t_lo) &&
+      combine_pair_better(calib, G, N, t_det - t_lo))
     return launch_combine_pair(static_cast<const int8_t*>(streams), shifts, scales, off_re, off_im,
                                per_t, out, out_f16, G, t_stream, N, 1, t_det - t_lo, t_lo,
                                fftshift, 1.f, stream);
