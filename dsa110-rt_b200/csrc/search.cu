@@ -779,14 +779,17 @@ __global__ void padded_cumsum_kernel(const T* __restrict__ x, int n, long long i
   for (int r = 0; r < pr; ++r) cs[(long long)(1 + pl + n + r) * inner + e] = last;
 }
 
-// A CTA walks BA_T consecutive outputs of V x 128 adjacent cells, V cells per
-// thread and access: the prefix rows of one output are the next ones' too, so
+// A CTA walks tt consecutive outputs (BA_T in calls that fill the chip) of
+// V x 128 adjacent cells, V cells per thread and access: the prefix rows of one output are the next ones' too, so
 // all but the first touch of a row come from L1, and what bounds the kernel
 // is the L1 rate of its 2 K loads per output (then memory: every prefix read
 // and 6 to 8 bytes written once).  One output per thread, with two 64-bit
 // divisions and 2 K 4-byte loads from L2 each, took 309 us for 128 outputs of
 // 4 x 256^2 cells at boxcars 1..16; this takes 95 us (tiles of 4, 16, 32 and 64
-// times: 100, 108, 123, 120).
+// times: 100, 108, 123, 120).  Small calls take shorter tiles, down to one
+// output, while there are fewer than eight CTAs per SM, and one cell per
+// thread below one: 16 outputs of 64^2 cells 2.4 us (6.6 in tiles of 8), 64 of
+// 100^2 4.4 (9.3).
 //
 // CHECK: every prefix row read must lie in [0, cs_rows); an output whose
 // widths / offsets would read outside gets S/N NaN and winner -1 instead
@@ -798,7 +801,7 @@ template <int V, bool OUT_F16, bool CHECK>
 __global__ void __launch_bounds__(BA_THREADS) multi_boxcar_argmax_kernel(
     const float* __restrict__ cs, long long inner, const int* __restrict__ widths,
     const int* __restrict__ offsets, const float* __restrict__ sinv, int K, int n_out, int t_base,
-    void* __restrict__ out_max, int16_t* __restrict__ out_win, long long cs_rows, int n_tt) {
+    void* __restrict__ out_max, int16_t* __restrict__ out_win, long long cs_rows, int n_tt, int tt) {
   // each width's first and last row relative to the output's, as offsets into
   // cs, and its scale
   __shared__ longlong2 s_off[BA_MAX_K];
@@ -812,7 +815,7 @@ __global__ void __launch_bounds__(BA_THREADS) multi_boxcar_argmax_kernel(
   __syncthreads();
   // time tiles fastest: the CTAs that run together share rows in L2
   const long long e = ((long long)(blockIdx.x / n_tt) * BA_THREADS + threadIdx.x) * V;
-  const int t0 = (int)(blockIdx.x % n_tt) * BA_T, t1 = min(n_out, t0 + BA_T);
+  const int t0 = (int)(blockIdx.x % n_tt) * tt, t1 = min(n_out, t0 + tt);
   if (e >= inner) return;
   using VT = typename std::conditional<V == 4, float4, float>::type;
   for (int t = t0; t < t1; ++t) {
@@ -883,16 +886,23 @@ template <bool CHECK>
 int launch_argmax(const float* cs, long long inner, const int* widths, const int* offsets,
                   const float* sinv, int K, int n_out, int t_base, void* out_max, int out_f16,
                   int16_t* out_win, long long cs_rows, cudaStream_t stream) {
-  const bool four = inner % 4 == 0 && (reinterpret_cast<uintptr_t>(cs) % 16) == 0 &&
+  const bool aligned = inner % 4 == 0 && (reinterpret_cast<uintptr_t>(cs) % 16) == 0 &&
                     (reinterpret_cast<uintptr_t>(out_max) % (out_f16 ? 8 : 16)) == 0 &&
                     (reinterpret_cast<uintptr_t>(out_win) % 8) == 0;
-  const int n_tt = (n_out + BA_T - 1) / BA_T;
-  const long long per = (long long)BA_THREADS * (four ? 4 : 1);
-  const long long blocks = (inner + per - 1) / per * n_tt;
+  // shorter time tiles, then one cell per thread, while the CTAs leave SMs idle
+  auto n_blocks = [&](int v, int tt) {
+    const long long per = (long long)BA_THREADS * v;
+    return (inner + per - 1) / per * ((n_out + tt - 1) / tt);
+  };
+  int tt = BA_T;
+  while (tt > 1 && n_blocks(aligned ? 4 : 1, tt) < 148 * 8) tt /= 2;
+  const bool four = aligned && n_blocks(4, tt) >= 148;
+  const int n_tt = (n_out + tt - 1) / tt;
+  const long long blocks = n_blocks(four ? 4 : 1, tt);
   if (blocks > 0x7fffffffLL) return DSB_E_ARG;
   auto go = [&](auto kern) {
     kern<<<(unsigned)blocks, BA_THREADS, 0, stream>>>(cs, inner, widths, offsets, sinv, K, n_out,
-                                                      t_base, out_max, out_win, cs_rows, n_tt);
+                                                      t_base, out_max, out_win, cs_rows, n_tt, tt);
     return cudaGetLastError() == cudaSuccess ? DSB_OK : DSB_E_CUDA;
   };
   if (four) return out_f16 ? go(multi_boxcar_argmax_kernel<4, true, CHECK>)
