@@ -1800,9 +1800,14 @@ int dsb_unpack_int4(const void* raw, int npkt, int nant, int nchan, int out_dtyp
     return DSB_E_ARG;
   const int rows = npkt * nant;
   const uint32_t* r = static_cast<const uint32_t*>(raw);
-  // four rows per store where every plane of rows starts on that boundary
+  // four rows per store where every plane of rows starts on that boundary, in
+  // calls of enough 128 x 32 tiles: with fewer the four times as many small
+  // tiles end sooner (32 tiles of float16 3.1 and 3.4 us, 48 3.6 and 3.4;
+  // float32, whose stores are 128 bytes either way, 384 tiles 9.0 and 9.5 us,
+  // 1152 33.9 and 30.4)
   const size_t esz = out_dtype == DSB_DT_INT8 ? 1 : out_dtype == DSB_DT_F16 ? 2 : 4;
-  const bool four = rows % 4 == 0 && (((uintptr_t)out_re | (uintptr_t)out_im) % (4 * esz)) == 0;
+  const long long tiles = (long long)((rows + 127) / 128) * ((nchan + 31) / 32);
+  const bool four = rows % 4 == 0 && tiles >= (esz == 4 ? 592 : 40) && (((uintptr_t)out_re | (uintptr_t)out_im) % (4 * esz)) == 0;
   auto go = [&](auto t) {
     using T = decltype(t);
     T *re = static_cast<T*>(out_re), *im = static_cast<T*>(out_im);
