@@ -471,8 +471,9 @@ constexpr int S1_THREADS = 256;
 constexpr int S1_MAX_C = 64;
 constexpr int S1_TT = 64;   // output times per tile
 constexpr int S1_DG = 32;   // largest DM group (coarse DMs per CTA)
-// CTAs per SM of the chunked form with 8 DMs (80 registers): the 312 CTAs of
-// the small configuration then run in one wave (two per SM: 245 us, not 190)
+// CTAs per SM of the chunked form with 8 DMs (80 registers, 56 bytes of them
+// spilled): the 312 CTAs of the small configuration then run in one wave (two
+// per SM, without spills: 245 us, not 190)
 constexpr int S1_CHUNK_CTAS8 = 3;
 
 __host__ __device__ inline size_t s1_smem_bytes(int ceff, int dg, int win_len) {
@@ -585,15 +586,17 @@ __global__ void __launch_bounds__(S1_THREADS, CHUNK && DG == 8 ? S1_CHUNK_CTAS8 
   if constexpr (CHUNK) {
     constexpr int KT = S1_TT / L;
     static_assert(KT <= 4, "a thread's sums stay in registers");
-    const int lane = tid & 31, warp = tid >> 5;
     const int n_ch = (ceff + A.sbc - 1) / A.sbc;
     const int n_items = (A.n_t + S1_TT - 1) / S1_TT * n_ch;   // (tile, subbands)
+    // four warps per subband's copies: with windows so long that a chunk is one
+    // subband, one warp issuing them all took 343 us where the whole windows
+    // take 278, four 271 (64 DMs in 16s, 6 subbands, shifts spread over 1000)
     auto load = [&](int item) {
       const int tt = item / n_ch * S1_TT, s0 = item % n_ch * A.sbc;
       const int w0 = (item & 1) * A.sbc;
-      for (int q = warp; q < min(A.sbc, ceff - s0); q += S1_THREADS / 32) {
+      for (int q = tid / 128; q < min(A.sbc, ceff - s0); q += S1_THREADS / 128) {
         const int sb = s0 + q;
-        for (int tau = lane; tau < s_len[sb]; tau += 32) {
+        for (int tau = tid % 128; tau < s_len[sb]; tau += 128) {
           const long long r2 = ((((A.t0 + tt + s_lo[sb] + tau) & A.y_mask) * A.y_rows) + ycol +
                                 (long long)sb * pitch) / 2;
           if (!DSB_INB(r2 + 1, (A.y_mask + 1) * A.y_rows / 2, A.status)) continue;
@@ -826,11 +829,15 @@ int dsb_stage1_rows(const void* Y, long long y_rows, long long y_mask, int n_blo
   A.sky_count = sky_count; A.sky_subtract = sky_subtract; A.status = status;
   // chunks where the whole windows leave room for one CTA per SM only (and
   // a DM group narrow enough to keep its sums in registers): as many subbands
-  // as two buffers in half an SM hold, at most one per warp
+  // as two buffers in half an SM hold, at most eight.  A grid that gives the
+  // SMs one CTA each keeps the whole windows: 111 us for 100 CTAs of 8 DMs
+  // (121 in chunks), 86 for 80 (91); 100 CTAs of 16 DMs 129 and 120.
   size_t bytes = smem;
   const size_t tables = s1_smem_bytes(ceff, dm_group, 0), per_sb = (size_t)2 * win_len * 32;
   const size_t room = 227 * 1024 / (dm_group == 8 ? S1_CHUNK_CTAS8 : 2) - 1024;
-  if (dm_group <= 16 && smem > 113 * 1024 && tables + per_sb <= room) {
+  const long long ctas = (long long)n_blocks * ((n_dm + dm_group - 1) / dm_group);
+  if (dm_group <= 16 && smem > 113 * 1024 && tables + per_sb <= room &&
+      ctas > (dm_group == 8 ? 148 : 74)) {
     A.sbc = (int)std::min<size_t>(S1_THREADS / 32, (room - tables) / per_sb);
     A.sbc = std::min(A.sbc, ceff);
     bytes = tables + (size_t)A.sbc * per_sb;
