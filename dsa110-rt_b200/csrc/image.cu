@@ -287,10 +287,13 @@ constexpr int IMG_MAX_G = 64;
 //    S arrays (int32 real and imaginary parts) take 192 KB of shared memory.
 //  * N = 256: FOLD 4, 256 threads, three CTAs per SM with 128 TMEM columns
 //    each, 16-bit entry metadata.
-//  * N = 64: the same with 64 threads and up to 16 CTAs per SM of 32 columns
-//    each.  An image is a chain of short steps (a few hundred S entries, 12
-//    barriers), so the images in flight decide the rate: with 256 threads and
-//    three CTAs per SM 16,896 images took 389 us, now 231.
+//  * N = 64: the same with 64 threads and up to 12 CTAs per SM of 32 columns
+//    each (80 registers; 16 CTAs at 64 registers spilled in the complex64
+//    form, 249 us against 239).  An image is a chain of short steps (a few
+//    hundred S entries, 12 barriers), so the images in flight decide the rate:
+//    with 256 threads and three CTAs per SM 16,896 images of 492 S entries
+//    took 412 us, now 239.  One image alone takes about as long (13.2 and 12.7
+//    us there, 11.1 and 12.1 with 238 entries).
 // TMEM: warps w, w + 4, w + 8, ... reach the same 32 lanes; each takes an
 // equal share of the CTA's columns, two 32-bit columns per complex S entry.
 template <int N>
@@ -303,7 +306,7 @@ struct ImgGeom {
   static constexpr int R1 = (N == 64) ? 8 : 16;   // threads per row transform
   static constexpr int R2 = N / R1;               // points per thread
   static constexpr int THREADS = (N == 512) ? 512 : (N == 256) ? 256 : 64;
-  static constexpr int CTAS = (N == 512) ? 1 : (N == 256) ? 3 : 16; // resident CTAs per SM
+  static constexpr int CTAS = (N == 512) ? 1 : (N == 256) ? 3 : 12; // resident CTAs per SM
   static constexpr int TMEM_COLS = (N == 512) ? 512 : (N == 256) ? 128 : 32;
   // columns per warp (warps 4 apart share lanes)
   static constexpr int WARP_COLS = TMEM_COLS / (THREADS > 128 ? THREADS / 128 : 1);
