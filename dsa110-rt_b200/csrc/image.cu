@@ -327,7 +327,8 @@ struct ImgGeom {
   // 32-bit form: the fold reads compact tables that follow gmeta in its
   // buffer (a nibble q | last << 3 per entry, [chunk][thread]; the first slot
   // of each thread; the slots' column-buffer offsets n' P + w' as uint16),
-  // copied per image into the part of buf the column buffer leaves free
+  // copied into the part of buf the column buffer leaves free, once per CTA
+  // where the combine's S arrays leave it free too, else once per image
   static constexpr int MAXC = MAXE / 8;                         // 8-entry chunks
   static constexpr size_t GM_BYTES = (size_t)(MAXE / 4) * THREADS * 16;
   static constexpr size_t FC_BYTES = (size_t)MAXC * THREADS * 4;
@@ -709,11 +710,13 @@ __global__ void __launch_bounds__(ImgGeom<N>::THREADS, ImgGeom<N>::CTAS)
               entry(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]), code & 7u, last, off);
             }
           } else {
+            static_assert(Gm::META32 || Gm::LAST_SH == 15,
+                          "the 16-bit entry's last bit is its top");
             constexpr unsigned LAST = 1u << Gm::LAST_SH;
 #pragma unroll
             for (int j = 0; j < 8; ++j)
               entry(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]),
-                    (m[j] >> Gm::Q_SH) & (FOLD - 1), (m[j] & LAST) != 0u && j < sn - 8 * c,
+                    (m[j] >> Gm::Q_SH) & (FOLD - 1), m[j] >= LAST && j < sn - 8 * c,
                     ((m[j] >> Gm::NP_SH) & (LC - 1)) * P + (m[j] & (NC - 1)));
           }
         };
