@@ -712,7 +712,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) corr_tc_kernel(const TcArgs A) 
 // products themselves, 0.6 us each per SM.  One role after the other between
 // CTA barriers, with the gridding's tables read in place, took 11.0 ms for 16
 // native pages gridded into 512^2 patterns and 445 us for one page; this takes
-// 4.1 ms and 288 us (2.7 ms and 175 us without the writing).
+// 3.3 ms and 286 us (175 us a page without the writing).
 //
 // Where two accumulators need fewer than 512 columns, the CTA takes only
 // those (a power of two) and several CTAs share an SM (TcArgs.ctas): a unit

@@ -105,9 +105,8 @@ __global__ void __launch_bounds__(DV_THREADS, 2)
   const int cell0 = (int)(blockIdx.x / n_tiles) * DV_CELLS;
   const int nc = min(DV_CELLS, n_filled - cell0);
 
-  // each subband's shift range over this CTA's DMs, and the window pitch:
-  // the longest window, made odd so that lanes on consecutive sources write
-  // different banks
+  // each subband's shift range over this CTA's DMs, and the widest of them:
+  // whether every source's window fits a buffer
   if (tid == 0) s_w = 0;
   __syncthreads();
   int w_max = 0;

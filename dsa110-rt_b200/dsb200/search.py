@@ -540,7 +540,7 @@ class GpuImager:
         full = getattr(self, "_uv_full", None)
         if full is None:
             # every image at once: the combine stages each stream row once for
-            # all fine DMs and 64 times (0.60 ms a cube of 16 x 64 images of
+            # all fine DMs and 64 times (0.57 ms a cube of 16 x 64 images of
             # 256^2, against 0.85 ms in chunks of 48 MB)
             full = self._uv_full = torch.empty((cfg.n_fdm * cfg.t_det, N, N // 2 + 1),
                                                dtype=torch.complex64, device=self.device)
