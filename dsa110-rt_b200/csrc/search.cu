@@ -428,9 +428,11 @@ __global__ void mask_to_cube_kernel(const float* __restrict__ img, const float* 
 // The staged form's set-up (shift range, row lists, window) and its few CTAs
 // pay only where many outputs share them: 381 cells x 8 fine DMs x 64 times
 // take 5.2 us a cell at a time and 6.4 us staged (30 us with 32 cells per
-// CTA), 1581 cells 10 and 12 us, 10.2k cells x 4 x 32 times 20 and 14 us; so
-// calls of less than CS_STAGED_MIN outputs go a cell at a time.  So does a
-// CTA whose windows hold more words than twice the outputs per row (only the
+// CTA), 1581 cells 10 and 12 us.  But a CTA per cell costs some 1.5 us per
+// thousand cells (16k cells x 4 x 16 times: 26 us, staged 17), so calls of at
+// most CS_CELL_MAX cells (times their time tiles) and CS_CELL_OUT outputs go a
+// cell at a time.  So does a CTA
+// whose windows hold more words than twice the outputs per row (only the
 // device knows the shifts), on cells a grid apart, so that those that run
 // together write the same sectors: 484 us for 16 fine DMs with shifts spread
 // over 3000 times, staged 787 (combine_cell_kernel's fuller SMs take 359).
@@ -442,7 +444,7 @@ constexpr int CS_THREADS = 128;
 constexpr int CS_WORDS = 10240;                 // staged words (two samples each) of 32 cells
 constexpr int CS_ROWS = CS_WORDS / (CS_T / 2);  // most rows of a group
 constexpr int CS_CELL_THREADS = 256;
-constexpr long long CS_STAGED_MIN = 1 << 20;
+constexpr long long CS_CELL_MAX = 2048, CS_CELL_OUT = 1 << 20;
 
 struct SparseArgs {
   const int16_t* dense;
@@ -1763,7 +1765,8 @@ int dsb_combine_sparse(const void* dense, const int* cell_uw, const int* cell_pt
                out, n_act, 1, 0, n_sb, t_rows, t_pad, n_filled_max, N, n_fdm, t_out_len, t_lo,
                fftshift, out_rows, out_row0, status};
   const int tiles = (t_out_len + CS_T - 1) / CS_T;
-  if ((long long)n_act * n_fdm * t_out_len < CS_STAGED_MIN) {
+  if ((long long)n_act * tiles <= CS_CELL_MAX &&
+      (long long)n_act * n_fdm * t_out_len < CS_CELL_OUT) {
     auto kern = out_f16 ? combine_cell_kernel<true> : combine_cell_kernel<false>;
     kern<<<dim3(n_act, tiles), CS_CELL_THREADS, 0, stream>>>(A);
     return launch_status();
