@@ -178,15 +178,15 @@ def combine_sparse_v4(dense: torch.Tensor, csr: SparseCellCsr, shifts: torch.Ten
     signature; this kernel needs neither."""
     st = _lib.status_word(out.device)
     _combine_sparse(dense, csr, shifts, t_rows=t_rows, t_out_len=t_out_len, t_lo=t_lo,
-                    fftshift=fftshift, out=out, out_row0=out_row0, status=st)
+                    fftshift=fftshift, out=out, out_row0=out_row0, status=st.data_ptr())
     _lib.check_status(st, "dsb_combine_sparse")
     return out
 
 
 def _combine_sparse(dense, csr, shifts, *, t_rows, t_out_len, t_lo, fftshift, out, out_row0,
-                    status) -> None:
-    """combine_sparse_v4's checks and launch; the device status is the
-    caller's to read."""
+                    status, stream=None) -> None:
+    """combine_sparse_v4's checks and launch; the device status word, by its
+    address, is the caller's to read."""
     n_sb, nfm, t_pad, two = dense.shape
     if two != 2 or n_sb != csr.n_sb:
         raise ValueError(f"dense {tuple(dense.shape)} does not match csr n_sb={csr.n_sb}")
@@ -218,11 +218,11 @@ def _combine_sparse(dense, csr, shifts, *, t_rows, t_out_len, t_lo, fftshift, ou
         _lib.require_cuda(x, nm)
     sh = shifts.to(torch.int32).contiguous()
     _lib.check(_lib.lib().dsb_combine_sparse(
-        _lib.ptr(dense), _lib.ptr(csr.cell_uw), _lib.ptr(csr.cell_ptr), _lib.ptr(csr.ent_g),
-        _lib.ptr(csr.ent_k), _lib.ptr(csr.ent_km), csr.n_cells, _lib.ptr(sh), _lib.ptr(out),
+        dense.data_ptr(), csr.cell_uw.data_ptr(), csr.cell_ptr.data_ptr(), csr.ent_g.data_ptr(),
+        csr.ent_k.data_ptr(), csr.ent_km.data_ptr(), csr.n_cells, sh.data_ptr(), out.data_ptr(),
         f16, n_sb, int(t_rows), int(t_pad), int(nfm), N, n_fdm, int(t_out_len), int(t_lo),
-        int(bool(fftshift)), out_rows, int(out_row0), _lib.ptr(status),
-        _lib.stream_of(out.device)), "dsb_combine_sparse")
+        int(bool(fftshift)), out_rows, int(out_row0), status,
+        _lib.stream_of(out.device) if stream is None else stream), "dsb_combine_sparse")
 
 
 # ---------------------------------------------------------------------------
@@ -309,8 +309,11 @@ _CUBE_DTYPES = (torch.float16, torch.float32)
 def _require_pixels(t: torch.Tensor, name: str, dtypes=_CUBE_DTYPES) -> None:
     """A contiguous CUDA tensor whose type the kernels know: they would read or
     write any other's pixels at the wrong width (bfloat16's past the end)."""
-    if isinstance(t, torch.Tensor) and t.dtype not in dtypes:
-        raise ValueError(f"{name} dtype {t.dtype} not in {dtypes}")
+    if isinstance(t, torch.Tensor):
+        if t.dtype not in dtypes:
+            raise ValueError(f"{name} dtype {t.dtype} not in {dtypes}")
+        if t.is_cuda and t.is_contiguous():
+            return
     _lib.require_cuda(t, name)
 
 
@@ -451,17 +454,17 @@ class GpuImager:
                     fftshift=True)
                 if cfg.imager_uv_prescale != 1.0:
                     uv.mul_(cfg.imager_uv_prescale)
-                self._transform_to_cube(uv, 1, n_t, cube, f, t_lo)
+                self._transform_to_cube(uv, 1, n_t, cube, f, t_lo, _lib.stream_of(self.device))
             return cube
+        stream = _lib.stream_of(self.device)
         for f0, n_f, t0, nt, work in self._chunks(t_lo, self.uv_slab):
             _lib.check(_lib.lib().dsb_combine_dense_fdm(
                 _lib.ptr(streams_cint8), _lib.ptr(shifts[f0:f0 + n_f]), n_f,
                 _lib.ptr(chgroup_scales if calib else None),
                 _lib.ptr(chgroup_offsets_re if calib else None),
                 _lib.ptr(chgroup_offsets_im if calib else None), int(per_t), _lib.ptr(work), G, T,
-                N, nt, t0, 1, float(cfg.imager_uv_prescale), _lib.stream_of(self.device)),
-                "dsb_combine_dense_fdm")
-            self._transform_to_cube(work, n_f, nt, cube, f0, t0)
+                N, nt, t0, 1, float(cfg.imager_uv_prescale), stream), "dsb_combine_dense_fdm")
+            self._transform_to_cube(work, n_f, nt, cube, f0, t0, stream)
         return cube
 
     # half spectra in flight between the dense combine, the column pass and the
@@ -493,19 +496,22 @@ class GpuImager:
                 n_f = min(nf_c, cfg.n_fdm - f0)
                 yield f0, n_f, t0, nt, buf[:n_f * nt * N * nh].view(n_f, nt, N, nh)
 
-    def _transform_to_cube(self, work, n_f: int, n_t: int, cube, f0: int, t0: int) -> None:
+    def _transform_to_cube(self, work, n_f: int, n_t: int, cube, f0: int, t0: int,
+                           stream) -> None:
         """Inverse real FFT of ``work`` [n_f, n_t, N, N/2+1] (overwritten) times
         the mask into ``cube[t0:t0 + n_t, f0:f0 + n_f]``."""
         N = self.config.n_grid
         per_f = self.edge_mask_per_fdm is not None
-        mask = self.edge_mask_per_fdm[f0:f0 + n_f] if per_f else self.edge_mask_real
+        mask = self.edge_mask_per_fdm if per_f else self.edge_mask_real
         _require_pixels(mask, "edge mask", (torch.float32,))
         _require_pixels(cube, "output cube")
+        f16, f_total = int(cube.dtype == torch.float16), int(cube.shape[1])
         _lib.check(_lib.lib().dsb_irfft2_cube(
-            _lib.ptr(work), n_t * N * (N // 2 + 1), n_f, n_t, N,
-            _lib.ptr(twiddles(N, self.device)), _lib.ptr(mask), int(per_f), _lib.ptr(cube[t0:]),
-            int(cube.dtype == torch.float16), int(cube.shape[1]), f0,
-            _lib.stream_of(self.device)), "dsb_irfft2_cube")
+            work.data_ptr(), n_t * N * (N // 2 + 1), n_f, n_t, N,
+            twiddles(N, self.device).data_ptr(),
+            mask.data_ptr() + (4 * N * N * f0 if per_f else 0), int(per_f),
+            cube.data_ptr() + (2 if f16 else 4) * N * N * f_total * t0, f16, f_total, f0, stream),
+            "dsb_irfft2_cube")
 
     def _process_compact(self, streams, shifts, inv_lut, t_stream, t_lo, cube, calib):
         """The compact path of process_cube (imager_gpu.py:300-330, 487-520):
@@ -529,13 +535,17 @@ class GpuImager:
             raise ValueError("compact combine needs at least one fine DM")
 
         def combine(csr, st):
+            stream = None
             for f0, n_f, t0, nt, work in self._chunks(t_lo, full):
                 work.zero_()
+                if stream is None:     # (looked up under the first fill)
+                    stream = _lib.stream_of(self.device)
                 _combine_sparse(streams, csr, shifts[f0:f0 + n_f], t_rows=t_stream, t_out_len=nt,
-                                t_lo=t0, fftshift=True, out=work, out_row0=0, status=st)
+                                t_lo=t0, fftshift=True, out=work, out_row0=0,
+                                status=st.data_ptr(), stream=stream)
                 if cfg.imager_uv_prescale != 1.0:
                     work.mul_(cfg.imager_uv_prescale)
-                self._transform_to_cube(work, n_f, nt, cube, f0, t0)
+                self._transform_to_cube(work, n_f, nt, cube, f0, t0, stream)
 
         full = getattr(self, "_uv_full", None)
         if full is None:
@@ -549,21 +559,22 @@ class GpuImager:
         # the images, and read with their status (no further wait): a table may
         # be rewritten in place, or another come to lie at its address.
         held = getattr(self, "_lut_csr", None)
-        if held is not None and inv_lut.is_cuda and \
-                (held[0].shape, held[0].dtype, held[0].device) == \
-                (inv_lut.shape, inv_lut.dtype, inv_lut.device):
-            st = torch.zeros(2, dtype=torch.int32, device=self.device)   # status, changed
+        if held is not None and held[0].device == inv_lut.device and \
+                held[0].shape == inv_lut.shape and held[0].dtype == inv_lut.dtype:
+            # one word to read: the combine's status, and above it the comparison
+            st = torch.zeros((), dtype=torch.int64, device=self.device)
             combine(held[1], st)
             lut = inv_lut.contiguous()
-            _lib.check(_lib.lib().dsb_tables_differ(
-                _lib.ptr(held[0]), _lib.ptr(lut), lut.numel() * lut.element_size(),
-                _lib.ptr(st[1:]), _lib.stream_of(self.device)), "dsb_tables_differ")
-            both = int(st.view(torch.int64).item())    # one word to read
+            _lib.check(_lib.lib().dsb_tables_differ(held[0].data_ptr(), lut.data_ptr(), held[2],
+                                                    st.data_ptr() + 4, _lib.stream_of(self.device)),
+                       "dsb_tables_differ")
+            both = int(st.item())
             if not both >> 32:
                 _lib.check_status_code(both, "dsb_combine_sparse")
                 return cube
-        lut = inv_lut.detach().clone(memory_format=torch.contiguous_format)
-        self._lut_csr = (lut, build_sparse_cell_csr(lut, n_grid=N))
+        lut = inv_lut.detach().to(self.device, copy=True).contiguous()
+        self._lut_csr = (lut, build_sparse_cell_csr(lut, n_grid=N),
+                         lut.numel() * lut.element_size())
         st = _lib.status_word(self.device)
         combine(self._lut_csr[1], st)
         _lib.check_status(st, "dsb_combine_sparse")
