@@ -216,7 +216,7 @@ def _combine_sparse(dense, csr, shifts, *, t_rows, t_out_len, t_lo, fftshift, ou
         raise ValueError(f"t_rows={t_rows} > t_pad={t_pad}")
     for x, nm in ((dense, "dense"), (shifts, "shifts"), (out, "out")):
         _lib.require_cuda(x, nm)
-    sh = shifts.to(torch.int32).contiguous()
+    sh = shifts if shifts.dtype == torch.int32 else shifts.to(torch.int32)
     _lib.check(_lib.lib().dsb_combine_sparse(
         dense.data_ptr(), csr.cell_uw.data_ptr(), csr.cell_ptr.data_ptr(), csr.ent_g.data_ptr(),
         csr.ent_k.data_ptr(), csr.ent_km.data_ptr(), csr.n_cells, sh.data_ptr(), out.data_ptr(),
@@ -269,7 +269,7 @@ _TWIDDLES: dict = {}
 
 def twiddles(n_grid: int, device) -> torch.Tensor:
     """(N,) complex64 exp(+2 pi i e / N) on ``device`` (cached)."""
-    key = (int(n_grid), str(device))
+    key = (int(n_grid), device)
     if key not in _TWIDDLES:
         e = np.arange(n_grid)
         _TWIDDLES[key] = torch.from_numpy(
@@ -540,7 +540,8 @@ class GpuImager:
                 work.zero_()
                 if stream is None:     # (looked up under the first fill)
                     stream = _lib.stream_of(self.device)
-                _combine_sparse(streams, csr, shifts[f0:f0 + n_f], t_rows=t_stream, t_out_len=nt,
+                sh = shifts if n_f == cfg.n_fdm else shifts[f0:f0 + n_f]
+                _combine_sparse(streams, csr, sh, t_rows=t_stream, t_out_len=nt,
                                 t_lo=t0, fftshift=True, out=work, out_row0=0,
                                 status=st.data_ptr(), stream=stream)
                 if cfg.imager_uv_prescale != 1.0:
